@@ -125,7 +125,7 @@ struct wrk_scene {
     uint32_t envW = 0, envH = 0;
     bool finalized = false;
     DevBuf dEnvMap;
-    DevBuf dVtx, dNrm, dUv, dIdx, dTriMat, dMats, dTexels, dTexInfo, dEmissive, dCdf, dLights, dErr;
+    DevBuf dVtx, dNrm, dUv, dIdx, dTriMat, dMats, dTexels, dTexInfo, dEmissive, dCdf, dLights, dErr, dPairs;
     uint4* nodes = nullptr;
     float4* tris = nullptr;
     std::vector<uint32_t> emissive;
@@ -617,8 +617,9 @@ int wrk_scene_finalize(wrk_scene* s) {
     s->nodes = br.nodes;
     s->tris = br.tris;
     // the shade bucket of each record's material, so the trace kernel sorts a hit
-    // with one load from the record it just tested
-    launch_leaf_buckets(br.tris, nt, s->dMats.as<wrk_material>(), (uint32_t)s->mats.size(), 0);
+    // with one load from its record, and the two-triangle records traversal tests
+    if ((rc = s->dPairs.alloc(5 * sizeof(float4) * (size_t)nt))) return rc;
+    launch_leaf_records(br.tris, nt, s->dMats.as<wrk_material>(), (uint32_t)s->mats.size(), s->dPairs.as<float4>(), 0);
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(0));
     s->info.numTriangles = nt;
@@ -647,6 +648,7 @@ int wrk_scene_finalize(wrk_scene* s) {
     for (int k = 0; k < 3; ++k) v.env[k] = s->env[k];
     v.nodes = s->nodes;
     v.tris = s->tris;
+    v.pairs = s->dPairs.as<float4>();
     v.numNodes = br.numNodes;
     if (!s->envMap.empty()) {
         if ((rc = upload(s->dEnvMap, s->envMap))) return rc;

@@ -207,19 +207,34 @@ __global__ void k_tonemap(const float* __restrict__ rgb, uint32_t nfloat, uint8_
     for (uint32_t i = n4 * 4 + blockIdx.x * blockDim.x + threadIdx.x; i < nfloat; i += stride) out[i] = aces_byte(rgb[i]);
 }
 
-__global__ void k_leaf_buckets(float4* tris, uint32_t nt, const wrk_material* __restrict__ mats, uint32_t numMats) {
+// One thread per leaf position: the shade bucket into its record's e2.w, and its pair
+// record (this position's triangle and the next one's; the last position pairs with
+// itself, which the traversal never selects).  v0 is stored negated, so the test's
+// o - v0 is one packed add.
+__global__ void k_leaf_records(float4* tris, uint32_t nt, const wrk_material* __restrict__ mats, uint32_t numMats,
+                               float4* __restrict__ pairs) {
     for (uint32_t l = blockIdx.x * blockDim.x + threadIdx.x; l < nt; l += gridDim.x * blockDim.x) {
-        const uint32_t mat = __float_as_uint(tris[3 * (size_t)l + 1].w);
-        const uint32_t b = mat < numMats ? bucket_of_material(mats[mat]) : (uint32_t)kBucketOther;
-        tris[3 * (size_t)l + 2].w = __uint_as_float(b);
+        const float4* r = tris + 3 * (size_t)l;
+        const float4* n = l + 1 < nt ? r + 3 : r;
+        const float4 a = r[0], b = r[1], a1 = n[0], b1 = n[1];
+        const float4 c = r[2], c1 = n[2];
+        const uint32_t mat = __float_as_uint(b.w);
+        tris[3 * (size_t)l + 2].w =
+            __uint_as_float(mat < numMats ? bucket_of_material(mats[mat]) : (uint32_t)kBucketOther);
+        float4* p = pairs + 5 * (size_t)l;
+        p[0] = make_float4(-a.x, -a1.x, -a.y, -a1.y);
+        p[1] = make_float4(-a.z, -a1.z, b.x, b1.x);
+        p[2] = make_float4(b.y, b1.y, b.z, b1.z);
+        p[3] = make_float4(c.x, c1.x, c.y, c1.y);
+        p[4] = make_float4(c.z, c1.z, 0.0f, 0.0f);
     }
 }
 
-void launch_leaf_buckets(float4* tris, uint32_t numTris, const wrk_material* mats, uint32_t numMats,
+void launch_leaf_records(float4* tris, uint32_t numTris, const wrk_material* mats, uint32_t numMats, float4* pairs,
                          cudaStream_t st) {
     if (!numTris) return;
     const uint32_t grid = (uint32_t)std::min<uint64_t>(((uint64_t)numTris + 255) / 256, 148u * 16u);
-    k_leaf_buckets<<<grid, 256, 0, st>>>(tris, numTris, mats, numMats);
+    k_leaf_records<<<grid, 256, 0, st>>>(tris, numTris, mats, numMats, pairs);
 }
 
 void launch_cdf(const float* cdf, uint32_t ncdf, const float* u, uint32_t n, uint32_t* out, cudaStream_t st) {

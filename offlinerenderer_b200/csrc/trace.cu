@@ -4,7 +4,7 @@
 // there are no RT cores on B200, so traversal is SIMT integer/FP32 work.
 //
 // Per node: five 16-byte loads (__ldg, read-only path), eight quantized slab tests
-// decoded with one byte permute and one directed-rounding FMA per plane.
+// decoded with one byte permute per plane and one packed FMA per near / far plane pair.
 // Internal-child hits go into an 8-bit mask permuted by the ray octant so the
 // lowest set bit is the child nearest the ray's entry corner; leaf-child hits set
 // bits of a triangle mask.  Pending node groups
@@ -12,9 +12,10 @@
 // shared memory, spilling to a bounded local array; overflow raises an error bit
 // and ends the ray instead of corrupting memory.
 //
-// The triangle test is Moller-Trumbore written with _rn / fmaf intrinsics so the
-// FP32 result is the same sequence of correctly rounded operations as the CPU
-// oracle's.
+// The triangle test is Moller-Trumbore in packed FP32 pairs (two triangles a test), on
+// each half the same sequence of correctly rounded operations as the CPU oracle's.
+#include <algorithm>
+
 #include "wrk_internal.h"
 #include "wrk_shading.cuh"
 #include "wrk_tri.cuh"
@@ -22,46 +23,61 @@
 namespace wrk {
 
 constexpr int kTraceBlock = 128;
-#ifndef WRK_STACK_SMEM
-#define WRK_STACK_SMEM 12
-#endif
-constexpr int kStackSmem = WRK_STACK_SMEM;
+// Stack entries per lane in shared memory (the rest, rarely used, in local memory).
+constexpr int kStackSmem = 8;
 constexpr int kStackLocal = 48 - kStackSmem;
 constexpr uint32_t kMaxVisits = 1u << 16;
+// A warp fetches new rays when fewer lanes than this still have one in flight.  The
+// wavefront kernels fetch through one counter, whose cost grows with the number of
+// fetches (showcase extension stage 32.8 ms at 16, 33.6 at 18, 38.6 at 24); the query
+// kernel's chunks are static, so it refills earlier (1M closest + occlusion queries of a
+// 676k-triangle scene 739 us at 16, 703 at 20).
+constexpr int kRefillAt = 16, kRefillQuery = 20;
+// Resident blocks per SM of the persistent kernels; each grid is that many blocks per SM.
+// The kernels wait on L1 / L2 for about a third of their cycles, so blocks pay until the
+// registers (65536 / (128 x blocks)) spill: extension traversal of the showcase 32.8 ms
+// with 8 blocks (64 registers, no spills), 35.4 with 9 (56, 148 B of spills), 35.4 with
+// 7.  A multi-scene lane also carries its scene's pointers.
+constexpr int kBlocksExtension = 8, kBlocksShadow = 8, kBlocksMulti = 7, kBlocksQuery = 8;
 
 // Byte k of w as the float 2^15 + b, exactly, without an int->float conversion:
 // one byte permute builds the bits 0x4700bb00 (exponent 2^15, b in mantissa bits
 // 8-15).  The 2^15 bias is folded into the per-node plane offset (see
-// intersect_node), so a plane costs one permute and one FMA.
+// intersect_node).
 __device__ __forceinline__ float qbias(uint32_t w, uint32_t k) {
     return __uint_as_float(__byte_perm(w, 0x47000000u, 0x7504u | (k << 4)));
 }
 
 // Intersects the 8 children of a node; returns internal hits (permuted by octant)
 // and the triangle mask relative to triBase.
-__device__ __forceinline__ void intersect_node(const uint4* __restrict__ nodes, uint32_t idx, const Ray& r,
-                                               float ix, float iy, float iz, uint32_t oct_inv, float tfar_max,
-                                               uint32_t& childBase, uint32_t& triBase, uint32_t& hits,
-                                               uint32_t& imask, uint32_t& tmask) {
+//
+// The node test is issue- and ALU-bound (byte permutes and min / max run at half
+// rate), so an axis' near and far planes share one packed FMA, and a child's outcome
+// is the sign of one FMA shifted into the hit mask.  With the refill below, 1M rays
+// against a 676k-triangle scene (closest hit + occlusion): 803 -> 753 us.
+__device__ __forceinline__ void intersect_node(const uint4* __restrict__ nodes, uint32_t idx, float ox, float oy,
+                                               float oz, float ix, float iy, float iz, uint32_t oct_inv, float tmin,
+                                               float tfar_max, uint32_t& childBase, uint32_t& triBase,
+                                               uint32_t& hits, uint32_t& imask, uint32_t& tmask) {
     const uint4* n = nodes + 5 * (size_t)idx;
     uint4 n0 = __ldg(n), n1 = __ldg(n + 1), n2 = __ldg(n + 2), n3 = __ldg(n + 3), n4 = __ldg(n + 4);
     float px = __uint_as_float(n0.x), py = __uint_as_float(n0.y), pz = __uint_as_float(n0.z);
     float sx = __uint_as_float((n0.w & 0xffu) << 23) * ix;
     float sy = __uint_as_float(((n0.w >> 8) & 0xffu) << 23) * iy;
     float sz = __uint_as_float(((n0.w >> 16) & 0xffu) << 23) * iz;
-    float ax = (px - r.ox) * ix, ay = (py - r.oy) * iy, az = (pz - r.oz) * iz;
+    float ax = (px - ox) * ix, ay = (py - oy) * iy, az = (pz - oz) * iz;
     // plane t = q*s + a = (2^15 + q)*s + (a - 2^15*s).  The biased offsets are
-    // rounded down for near planes and up for far planes, and the plane FMAs round
-    // the same way, so the slab only grows (by at most ~1/256 of a quantization
-    // step): a child box the ray crosses is never rejected.
-    const float axl = __fmaf_rd(-32768.0f, sx, ax), axh = __fmaf_ru(-32768.0f, sx, ax);
-    const float ayl = __fmaf_rd(-32768.0f, sy, ay), ayh = __fmaf_ru(-32768.0f, sy, ay);
-    const float azl = __fmaf_rd(-32768.0f, sz, az), azh = __fmaf_ru(-32768.0f, sz, az);
+    // rounded down for near planes and up for far planes, so their rounding only
+    // grows the slab (by at most ~1/256 of a quantization step); the plane FMAs
+    // round to nearest (2^-24 of t), which the 2^-22 slack of the test below covers:
+    // a child box the ray crosses is never rejected.
+    const f32x2 sx2 = pack2(sx, sx), sy2 = pack2(sy, sy), sz2 = pack2(sz, sz);
+    const f32x2 ax2 = pack2(__fmaf_rd(-32768.0f, sx, ax), __fmaf_ru(-32768.0f, sx, ax));
+    const f32x2 ay2 = pack2(__fmaf_rd(-32768.0f, sy, ay), __fmaf_ru(-32768.0f, sy, ay));
+    const f32x2 az2 = pack2(__fmaf_rd(-32768.0f, sz, az), __fmaf_ru(-32768.0f, sz, az));
     imask = n0.w >> 24;
     childBase = n1.x;
     triBase = n1.y;
-    hits = 0;
-    tmask = 0;
     // near/far plane words per axis: dir >= 0 -> near = lo, far = hi
     uint32_t xn0 = ix >= 0.0f ? n2.x : n3.z, xn1 = ix >= 0.0f ? n2.y : n3.w;
     uint32_t xf0 = ix >= 0.0f ? n3.z : n2.x, xf1 = ix >= 0.0f ? n3.w : n2.y;
@@ -72,27 +88,26 @@ __device__ __forceinline__ void intersect_node(const uint4* __restrict__ nodes, 
     const float tfar_lim = tfar_max * 1.00000024f;
     uint32_t hm = 0;  // children whose slab the ray crosses, by slot
 #pragma unroll
-    for (int s = 0; s < 8; ++s) {
+    for (int s = 7; s >= 0; --s) {
         const uint32_t k = s & 3;
         uint32_t xn = s < 4 ? xn0 : xn1, xf = s < 4 ? xf0 : xf1;
         uint32_t yn = s < 4 ? yn0 : yn1, yf = s < 4 ? yf0 : yf1;
         uint32_t zn = s < 4 ? zn0 : zn1, zf = s < 4 ? zf0 : zf1;
-        float t0x = __fmaf_rd(qbias(xn, k), sx, axl);
-        float t1x = __fmaf_ru(qbias(xf, k), sx, axh);
-        float t0y = __fmaf_rd(qbias(yn, k), sy, ayl);
-        float t1y = __fmaf_ru(qbias(yf, k), sy, ayh);
-        float t0z = __fmaf_rd(qbias(zn, k), sz, azl);
-        float t1z = __fmaf_ru(qbias(zf, k), sz, azh);
+        float t0x, t1x, t0y, t1y, t0z, t1z;
+        unpack2(fma2(pack2(qbias(xn, k), qbias(xf, k)), sx2, ax2), t0x, t1x);
+        unpack2(fma2(pack2(qbias(yn, k), qbias(yf, k)), sy2, ay2), t0y, t1y);
+        unpack2(fma2(pack2(qbias(zn, k), qbias(zf, k)), sz2, az2), t0z, t1z);
         // Three-input integer max / min on the float bit patterns.  Non-negative
         // floats order like their bit patterns; negative ones order reversed, which
         // only moves tn down and tf up (a larger slab, never a smaller one), and a
-        // negative tf still fails against tn >= tmin >= 0.  No plane distance is
-        // NaN: the inverse directions are finite (trav_init).
+        // negative tf still fails against tn >= tmin >= 0.
         float tn = __int_as_float(__vimax3_s32(__float_as_int(t0x), __float_as_int(t0y),
-                                               max(__float_as_int(t0z), __float_as_int(r.tmin))));
+                                               max(__float_as_int(t0z), __float_as_int(tmin))));
         float tf = __int_as_float(__vimin3_s32(__float_as_int(t1x), __float_as_int(t1y),
                                                min(__float_as_int(t1z), __float_as_int(tfar_lim))));
-        hm |= (tn <= tf * 1.00000024f) ? (1u << s) : 0u;
+        // crossed when tn - tf * (1 + 2^-22) <= 0: the sign of one FMA (rounded down, so
+        // that an exact zero is -0; a NaN, from a NaN ray, has its sign clear: missed)
+        hm = __funnelshift_l(__float_as_uint(__fmaf_rd(tf, -1.00000024f, tn)), hm, 1);
     }
     // internal hits, moved from slot s to bit s ^ oct_inv by three conditional swaps
     uint32_t ih = hm & imask;
@@ -102,6 +117,7 @@ __device__ __forceinline__ void intersect_node(const uint4* __restrict__ nodes, 
     hits = ih;
     // leaf hits: each adds its run of cnt triangles starting at bit off
     uint32_t lh = hm & ~imask;
+    tmask = 0;
     while (lh) {
         const uint32_t j = __ffs(lh) - 1;
         lh &= lh - 1;
@@ -111,23 +127,23 @@ __device__ __forceinline__ void intersect_node(const uint4* __restrict__ nodes, 
     }
 }
 
-// The four scene fields traversal needs (a DevScene has them too).
+// The scene fields traversal needs (a DevScene has them too).
 struct TraceGeom {
     const uint4* nodes;
     const float4* tris;
+    const float4* pairs;
     uint32_t numNodes, numTris;
 };
 
-// Per-lane traversal state, kept in registers across the persistent loop's rounds.
+// Per-lane traversal state, kept in registers across the persistent loop's rounds: every
+// word of it counts (an extension kernel that spills runs several percent slower).
+constexpr uint32_t kOctShift = 8, kVisitShift = 11;
 struct Trav {
-    Ray r;
+    float ox, oy, oz;
     float ix, iy, iz;
-    uint32_t octInv;
     uint32_t gBase;
     uint32_t gBits;  // node group: child hit bits (bits 0-7, octant order) | internal-child mask << 8
-    uint32_t tBase, tMask;
-    int sp;
-    uint32_t visits;
+    uint32_t state;  // stack entries (bits 0-7) | ray octant, inverted (8-10) | nodes visited << 11
     float tBest;
     // Leaf position (index into the BVH triangle records) of the best hit, kNoHit
     // while there is none; the hit's primitive and material are read from that
@@ -142,8 +158,11 @@ __device__ __forceinline__ uint32_t record_material(const float4* tris, uint32_t
     return l == kNoHit ? 0u : __float_as_uint(__ldg(tris + 3 * (size_t)l + 1).w);
 }
 
-__device__ __forceinline__ void trav_init(Trav& t, const Ray& r) {
-    t.r = r;
+__device__ __forceinline__ void trav_init(Trav& t, float4* sdir, const Ray& r) {
+    t.ox = r.ox;
+    t.oy = r.oy;
+    t.oz = r.oz;
+    sdir[threadIdx.x] = make_float4(r.dx, r.dy, r.dz, r.tmin);
     // Direction components below 2^-80 in magnitude are replaced by +-2^-80 for
     // the slab tests only (the triangle test uses the true direction), so inverse
     // directions and plane distances stay finite and never NaN.
@@ -152,14 +171,11 @@ __device__ __forceinline__ void trav_init(Trav& t, const Ray& r) {
     t.iy = 1.0f / (fabsf(r.dy) < ooeps ? copysignf(ooeps, r.dy) : r.dy);
     t.iz = 1.0f / (fabsf(r.dz) < ooeps ? copysignf(ooeps, r.dz) : r.dz);
     uint32_t oct = (r.dx < 0.0f ? 1u : 0u) | (r.dy < 0.0f ? 2u : 0u) | (r.dz < 0.0f ? 4u : 0u);
-    t.octInv = oct ^ 7u;  // slot of the child nearest the entry corner -> bit 0
+    const uint32_t octInv = oct ^ 7u;  // slot of the child nearest the entry corner -> bit 0
+    t.state = octInv << kOctShift;
     // the root is a one-child node group
     t.gBase = 0;
-    t.gBits = (1u << t.octInv) | (1u << 8);
-    t.tBase = 0;
-    t.tMask = 0;
-    t.sp = 0;
-    t.visits = 0;
+    t.gBits = (1u << octInv) | (1u << 8);
     t.tBest = r.tmax;
     t.lBest = kNoHit;
 }
@@ -168,84 +184,106 @@ __device__ __forceinline__ void trav_init(Trav& t, const Ray& r) {
 // (pushing the group's remainder), test the triangles that node exposes, and pop
 // when the group is used up.  Returns true when the ray is finished.  Closest hit
 // keeps ties in t with the lower primitive index; any hit stops at the first hit.
-template <bool kAnyHit, class Geom>
-__device__ __forceinline__ bool trav_step(const Geom& s, Trav& t, uint2* sstack, uint2* lstack,
+// kTmin0: every ray's tmin is at least 0, so the node test clamps at 0 (the triangle
+// test always applies the ray's own); otherwise at the ray's tmin.
+template <bool kAnyHit, bool kTmin0, class Geom>
+__device__ __forceinline__ bool trav_step(const Geom& s, Trav& t, const float4* sdir, uint2* sstack, uint2* lstack,
                                           uint32_t* errFlag) {
     const int tid = threadIdx.x;
-    if (++t.visits > kMaxVisits) {  // a malformed tree must not spin forever
+    t.state += 1u << kVisitShift;
+    if (t.state >> kVisitShift > kMaxVisits) {  // a malformed tree must not spin forever
         atomicOr(errFlag, kErrBadIndex);
         return true;
     }
+    uint32_t tBase = 0, tMask = 0;  // the triangles the node exposes
     if (t.gBits & 0xffu) {
+        const uint32_t octInv = (t.state >> kOctShift) & 7u;
         uint32_t pos = __ffs(t.gBits) - 1;  // the lowest set bit is a hit bit
         t.gBits &= t.gBits - 1;
-        uint32_t slot = pos ^ t.octInv;
+        uint32_t slot = pos ^ octInv;
         uint32_t child = t.gBase + __popc(t.gBits & (((1u << slot) - 1u) << 8));
         if (t.gBits & 0xffu) {
             uint2 e = make_uint2(t.gBase, t.gBits);
-            if (t.sp < kStackSmem) sstack[t.sp * kTraceBlock + tid] = e;
-            else if (t.sp < kStackSmem + kStackLocal) lstack[t.sp - kStackSmem] = e;
+            const int sp = t.state & 0xffu;
+            if (sp < kStackSmem) sstack[sp * kTraceBlock + tid] = e;
+            else if (sp < kStackSmem + kStackLocal) lstack[sp - kStackSmem] = e;
             else {
                 atomicOr(errFlag, kErrStackOverflow);
                 return true;
             }
-            ++t.sp;
+            ++t.state;
         }
         if (child >= s.numNodes) {
             atomicOr(errFlag, kErrBadIndex);
             return true;
         }
         uint32_t hits, imask;
-        intersect_node(s.nodes, child, t.r, t.ix, t.iy, t.iz, t.octInv, t.tBest, t.gBase, t.tBase, hits, imask,
-                       t.tMask);
+        intersect_node(s.nodes, child, t.ox, t.oy, t.oz, t.ix, t.iy, t.iz, octInv, kTmin0 ? 0.0f : sdir[tid].w, t.tBest,
+                       t.gBase, tBase, hits, imask, tMask);
         t.gBits = hits | (imask << 8);
-        if (t.tMask && t.tBase + (31u - __clz(t.tMask)) >= s.numTris) {
+        if (tMask && tBase + (31u - __clz(tMask)) >= s.numTris) {
             atomicOr(errFlag, kErrBadIndex);
             return true;
         }
     }
-    while (t.tMask) {
-        uint32_t j = __ffs(t.tMask) - 1;
-        t.tMask &= t.tMask - 1;
-        const float4* tp = s.tris + 3 * (size_t)(t.tBase + j);
-        float4 a = __ldg(tp), b = __ldg(tp + 1), c = __ldg(tp + 2);
-        float th;
-        // closest hit: tBest <= tmax, so the update test below implies th <= tmax;
-        // any hit: tBest is tmax until the first hit, which ends the ray
-        if (mt_rn(t.r, a, b, c, th) && th >= t.r.tmin && (!kAnyHit || th <= t.tBest)) {
-            if (kAnyHit) {
-                t.tBest = th;
-                t.lBest = t.tBase + j;
-                return true;
+    // A leaf's triangles occupy a handful of lanes while the others wait, so two are
+    // tested at a time (mt_pair), and the ray's direction, which only this part reads,
+    // stays in shared memory: 64 registers without spills, where one triangle at a time
+    // and the direction in registers took 58.  Showcase extension stage 34.0 -> 32.8 ms,
+    // 1M-ray queries 753 -> 704 us.
+    if (tMask) {
+        const float4 dt = sdir[tid];
+        const Ray r{t.ox, t.oy, t.oz, dt.x, dt.y, dt.z, dt.w, 0.0f};
+        while (tMask) {
+            // the lowest pending triangle and, when it is pending too, the next one, in one
+            // packed test
+            const uint32_t j = __ffs(tMask) - 1;
+            const bool two = (tMask >> j) & 2u;
+            tMask &= ~(3u << j);
+            uint32_t l = tBase + j;
+            float2 num, det;
+            bool in0, in1;
+            mt_pair(r, s.pairs + kPairWords * (size_t)l, num, det, in0, in1);
+            in1 = in1 && two;
+            if (!in0) {
+                if (!in1) continue;
+                ++l;
             }
-            if (th < t.tBest || (th == t.tBest && __float_as_uint(a.w) < record_prim(s.tris, t.lBest))) {
-                t.tBest = th;
-                t.lBest = t.tBase + j;
+            // both inside (a shared edge, coincident triangles): the first, then the second
+            bool again = in0 && in1;
+            float n = in0 ? num.x : num.y, d = in0 ? det.x : det.y;
+            while (true) {
+                const float th = __fdiv_rn(n, d);
+                // closest hit: tBest <= tmax, so the update test below implies th <= tmax;
+                // any hit: tBest is tmax until the first hit, which ends the ray
+                if (th >= r.tmin && (!kAnyHit || th <= t.tBest)) {
+                    if (kAnyHit) {
+                        t.tBest = th;
+                        t.lBest = l;
+                        return true;
+                    }
+                    if (th < t.tBest || (th == t.tBest && record_prim(s.tris, l) < record_prim(s.tris, t.lBest))) {
+                        t.tBest = th;
+                        t.lBest = l;
+                    }
+                }
+                if (!again) break;
+                again = false;
+                ++l;
+                n = num.y;
+                d = det.y;
             }
         }
     }
     if (!(t.gBits & 0xffu)) {
-        if (t.sp == 0) return true;
-        --t.sp;
-        uint2 e = t.sp < kStackSmem ? sstack[t.sp * kTraceBlock + tid] : lstack[t.sp - kStackSmem];
+        const int sp = (int)(t.state & 0xffu) - 1;
+        if (sp < 0) return true;
+        --t.state;
+        uint2 e = sp < kStackSmem ? sstack[sp * kTraceBlock + tid] : lstack[sp - kStackSmem];
         t.gBase = e.x;
         t.gBits = e.y;
     }
     return false;
-}
-
-template <bool kAnyHit>
-__device__ __forceinline__ bool traverse(const DevScene& s, const Ray& r, float& tBest, uint32_t& pBest,
-                                         uint32_t& mBest, uint2* sstack, uint32_t* errFlag) {
-    uint2 lstack[kStackLocal];
-    Trav t;
-    trav_init(t, r);
-    while (!trav_step<kAnyHit>(s, t, sstack, lstack, errFlag)) {
-    }
-    tBest = t.tBest;
-    pBest = record_prim(s.tris, t.lBest);
-    mBest = record_material(s.tris, t.lBest);
-    return t.lBest != kNoHit;
 }
 
 __device__ __forceinline__ Ray load_ray8(const float* p) {
@@ -254,39 +292,76 @@ __device__ __forceinline__ Ray load_ray8(const float* p) {
     return Ray{a.x, a.y, a.z, b.x, b.y, b.z, a.w, b.w};
 }
 
-__global__ void __launch_bounds__(kTraceBlock) k_closest_query(DevScene s, const float* __restrict__ rays, uint32_t n,
-                                                               float* tOut, uint32_t* pOut, uint32_t* err) {
+// Ray queries: persistent warps, each taking every gridDim-th chunk of 32 rays and
+// refilling idle lanes from its chunks (below kRefillQuery busy lanes), so a warp does not
+// wait for its slowest ray (one thread per ray ran at 8 of 32 lanes per instruction:
+// 1M closest + occlusion queries of a 676k-triangle scene 1022 us, 803 with the refill).
+// The chunks are assigned statically: no state is shared between calls.
+template <bool kAnyHit>
+__global__ void __launch_bounds__(kTraceBlock, kBlocksQuery)
+    k_query(DevScene s, const float* __restrict__ rays, uint32_t n, float* tOut, uint32_t* pOut, uint32_t* err) {
     __shared__ uint2 sstack[kStackSmem * kTraceBlock];
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    Ray r = load_ray8(rays + 8 * (size_t)i);
-    float t;
-    uint32_t p, m;
-    bool hit = traverse<false>(s, r, t, p, m, sstack, err);
-    tOut[i] = hit ? t : __int_as_float(0x7f800000);
-    pOut[i] = hit ? p : kNoHit;
+    __shared__ float4 sdir[kTraceBlock];  // the lanes' ray directions | tmin (read by triangle tests only)
+    uint2 lstack[kStackLocal];
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint64_t stride = (uint64_t)gridDim.x * kTraceBlock;
+    uint64_t next = (uint64_t)blockIdx.x * kTraceBlock + (threadIdx.x & ~31u);
+    uint32_t used = 0;  // rays of the chunk at `next` already taken
+    const TraceGeom geo{s.nodes, s.tris, s.pairs, s.numNodes, s.numTris};
+    Trav t;
+    uint32_t idx = 0;
+    bool active = false;
+    while (true) {
+        uint32_t idle;
+        while (next < n && (idle = __ballot_sync(0xffffffffu, !active)) != 0) {
+            const uint32_t avail = (uint32_t)min((unsigned long long)32u, (unsigned long long)(n - next)) - used;
+            const uint32_t rank = __popc(idle & ((1u << lane) - 1u));
+            if (!active && rank < avail) {
+                idx = (uint32_t)next + used + rank;
+                trav_init(t, sdir, load_ray8(rays + 8 * (size_t)idx));
+                active = true;
+            }
+            used += min(avail, (uint32_t)__popc(idle));
+            if (used >= 32u || next + used >= n) {
+                next += stride;
+                used = 0;
+            }
+        }
+        if (!__any_sync(0xffffffffu, active)) break;
+        const int refillAt = next < n ? kRefillQuery : 1;
+        bool fin = false;
+        do {
+            if (active && !fin) fin = trav_step<kAnyHit, false>(geo, t, sdir, sstack, lstack, err);
+        } while (__popc(__ballot_sync(0xffffffffu, active && !fin)) >= refillAt);
+        if (active && fin) {
+            const bool hit = t.lBest != kNoHit;
+            if (kAnyHit) {
+                pOut[idx] = hit ? 1u : 0u;
+            } else {
+                tOut[idx] = hit ? t.tBest : __int_as_float(0x7f800000);
+                pOut[idx] = record_prim(s.tris, t.lBest);
+            }
+            active = false;
+        }
+    }
 }
 
-__global__ void __launch_bounds__(kTraceBlock) k_occluded_query(DevScene s, const float* __restrict__ rays,
-                                                                uint32_t n, uint32_t* out, uint32_t* err) {
-    __shared__ uint2 sstack[kStackSmem * kTraceBlock];
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    Ray r = load_ray8(rays + 8 * (size_t)i);
-    float t;
-    uint32_t p, m;
-    out[i] = traverse<true>(s, r, t, p, m, sstack, err) ? 1u : 0u;
+static int query_grid(uint32_t n) {
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return (int)std::min<uint64_t>(((uint64_t)n + kTraceBlock - 1) / kTraceBlock, (uint64_t)sms * kBlocksQuery);
 }
 
 void launch_closest_query(const DevScene& s, const float* rays, uint32_t n, float* t, uint32_t* prim, uint32_t* err,
                           cudaStream_t st) {
     if (!n) return;
-    k_closest_query<<<(n + kTraceBlock - 1) / kTraceBlock, kTraceBlock, 0, st>>>(s, rays, n, t, prim, err);
+    k_query<false><<<query_grid(n), kTraceBlock, 0, st>>>(s, rays, n, t, prim, err);
 }
 void launch_occluded_query(const DevScene& s, const float* rays, uint32_t n, uint32_t* occ, uint32_t* err,
                            cudaStream_t st) {
     if (!n) return;
-    k_occluded_query<<<(n + kTraceBlock - 1) / kTraceBlock, kTraceBlock, 0, st>>>(s, rays, n, occ, err);
+    k_query<true><<<query_grid(n), kTraceBlock, 0, st>>>(s, rays, n, nullptr, occ, err);
 }
 
 // ---------------------------------------------------------------------------
@@ -297,22 +372,6 @@ void launch_occluded_query(const DevScene& s, const float* rays, uint32_t n, uin
 // lanes of a warp write consecutive entries.  Queue entries are read and written
 // once per pass, so they go through the cache with the streaming (evict-first)
 // policy (__ldcs / __stcs) and leave L1 to the BVH nodes and triangle records.
-__device__ __forceinline__ uint32_t warp_append_pos(uint32_t* counter, bool pred, uint32_t cap, uint32_t* err) {
-    uint32_t b = __ballot_sync(0xffffffffu, pred);
-    if (!b) return kInvalidSlot;
-    uint32_t lane = threadIdx.x & 31u;
-    uint32_t leader = __ffs(b) - 1;
-    uint32_t base = 0;
-    if (lane == leader) base = atomicAdd(counter, (uint32_t)__popc(b));
-    base = __shfl_sync(0xffffffffu, base, leader);
-    uint32_t pos = base + __popc(b & ((1u << lane) - 1u));
-    if (pred && pos >= cap) {
-        atomicOr(err, kErrQueueOverflow);
-        return kInvalidSlot;
-    }
-    return pred ? pos : kInvalidSlot;
-}
-
 __device__ __forceinline__ PathQ pick_bucket(const Queues& q, uint32_t b) {
     switch (b) {
         case kBucketLambert: return q.bucket[kBucketLambert];
@@ -327,21 +386,9 @@ __device__ __forceinline__ PathQ pick_bucket(const Queues& q, uint32_t b) {
 // fewer than kRefillAt lanes still have a ray in flight, instead of waiting for
 // the slowest ray of a fixed batch (Aila & Laine 2009, "Understanding the
 // efficiency of ray traversal on GPUs").
-#ifndef WRK_REFILL_AT
-#define WRK_REFILL_AT 16
-#endif
-// Resident blocks per SM of each persistent trace kernel (its register budget is
-// 65536 / (128 x blocks)); the grid is that many blocks per SM.
-#ifndef WRK_TRACE_EXT_BLOCKS
-#define WRK_TRACE_EXT_BLOCKS 9
-#endif
-#ifndef WRK_TRACE_SHADOW_BLOCKS
-#define WRK_TRACE_SHADOW_BLOCKS 8
-#endif
-constexpr int kRefillAt = WRK_REFILL_AT;
 template <bool kAnyHit, bool kMulti>
 struct TraceBlocks {
-    static constexpr int value = kMulti ? 8 : (kAnyHit ? WRK_TRACE_SHADOW_BLOCKS : WRK_TRACE_EXT_BLOCKS);
+    static constexpr int value = kMulti ? kBlocksMulti : (kAnyHit ? kBlocksShadow : kBlocksExtension);
 };
 
 // Adds a miss's environment term and accumulates the path into its request's sums
@@ -368,6 +415,7 @@ template <bool kAnyHit, bool kMulti>
 __global__ void __launch_bounds__(kTraceBlock, (TraceBlocks<kAnyHit, kMulti>::value))
     k_trace_persistent(DevScene s0, Queues q) {
     __shared__ uint2 sstack[kStackSmem * kTraceBlock];
+    __shared__ float4 sdir[kTraceBlock];  // the lanes' ray directions | tmin (read by triangle tests only)
     uint2 lstack[kStackLocal];
     Counters* c = q.ctr;
     const uint32_t cur = c->cur;
@@ -377,43 +425,47 @@ __global__ void __launch_bounds__(kTraceBlock, (TraceBlocks<kAnyHit, kMulti>::va
     const uint32_t lane = threadIdx.x & 31u;
     // the shadow stage continues every Lambert path it traces (statistics slot)
     if (kAnyHit && blockIdx.x == 0 && threadIdx.x == 0) c->bucket[kBucketLambertResume].v = n;
+    // A warp's first 32 rays are the ones at its position in the grid: a queue of at
+    // most 32 rays per warp never touches the fetch counter (which every warp of the
+    // grid, idle ones too, would otherwise visit).  Later rays come from the counter,
+    // as many as there are idle lanes: larger grains per warp measured slower.
+    const uint32_t gridRays = gridDim.x * kTraceBlock;
+    uint32_t base = blockIdx.x * kTraceBlock + (threadIdx.x & ~31u);
+    bool exhausted = base >= n;
     Trav t;
-    TraceGeom geo{s0.nodes, s0.tris, s0.numNodes, s0.numTris};
-    uint32_t sceneIdx = 0;
+    TraceGeom geo{s0.nodes, s0.tris, s0.pairs, s0.numNodes, s0.numTris};
     uint32_t idx = 0;
-    bool active = false, exhausted = false;
+    bool active = false;
     while (true) {
-        uint32_t idle = __ballot_sync(0xffffffffu, !active && !exhausted);
+        const uint32_t idle = exhausted ? 0u : __ballot_sync(0xffffffffu, !active);
         if (idle) {
-            uint32_t leader = __ffs(idle) - 1, base = 0;
-            if (lane == leader) base = atomicAdd(fetch, (uint32_t)__popc(idle));
-            base = __shfl_sync(0xffffffffu, base, leader);
-            if (!active && !exhausted) {
-                idx = base + __popc(idle & ((1u << lane) - 1u));
-                if (idx < n) {
-                    float4 o = kAnyHit ? __ldcs(in.sh_o + idx) : __ldcs(in.ray_o + idx);
-                    float4 d = kAnyHit ? __ldcs(in.sh_d + idx) : __ldcs(in.ray_d + idx);
+            if (base == kInvalidSlot) {
+                if (lane == 0) base = atomicAdd(fetch, (uint32_t)__popc(idle)) + gridRays;
+                base = __shfl_sync(0xffffffffu, base, 0);
+            }
+            idx = active ? idx : base + __popc(idle & ((1u << lane) - 1u));
+            if (!active && idx < n) {
+                float4 o = kAnyHit ? __ldcs(in.sh_o + idx) : __ldcs(in.ray_o + idx);
+                float4 d = kAnyHit ? __ldcs(in.sh_d + idx) : __ldcs(in.ray_d + idx);
+                if constexpr (kMulti) {
                     // a shadow entry keeps its request slot where tmin would be
                     const uint32_t slot = kAnyHit ? __float_as_uint(o.w) : slot_of(__ldcs(&in.st[idx].w));
-                    if (kAnyHit) o.w = kShadowTmin;
-                    if constexpr (kMulti) {
-                        sceneIdx = q.req[slot].scene;
-                        const DevScene& sc = q.scenes[sceneIdx];
-                        geo = TraceGeom{sc.nodes, sc.tris, sc.numNodes, sc.numTris};
-                    }
-                    trav_init(t, Ray{o.x, o.y, o.z, d.x, d.y, d.z, o.w, d.w});
-                    active = true;
-                } else {
-                    exhausted = true;
+                    const DevScene& sc = q.scenes[q.req[slot].scene];
+                    geo = TraceGeom{sc.nodes, sc.tris, sc.pairs, sc.numNodes, sc.numTris};
                 }
+                if (kAnyHit) o.w = kShadowTmin;
+                trav_init(t, sdir, Ray{o.x, o.y, o.z, d.x, d.y, d.z, o.w, d.w});
+                active = true;
             }
+            exhausted = n <= gridRays || base + __popc(idle) >= n;
+            base = kInvalidSlot;
         }
-        if (__all_sync(0xffffffffu, exhausted && !active)) break;
+        if (!__any_sync(0xffffffffu, active)) break;
         // once the queue is drained nothing can refill a lane: run to completion
-        const int refillAt = __any_sync(0xffffffffu, exhausted) ? 1 : kRefillAt;
+        const int refillAt = exhausted ? 1 : kRefillAt;
         bool fin = false;
         do {
-            if (active && !fin) fin = trav_step<kAnyHit>(geo, t, sstack, lstack, &c->error);
+            if (active && !fin) fin = trav_step<kAnyHit, true>(geo, t, sdir, sstack, lstack, &c->error);
         } while (__popc(__ballot_sync(0xffffffffu, active && !fin)) >= refillAt);
         const bool done = active && fin;
         if (kAnyHit) {
@@ -460,9 +512,11 @@ __global__ void __launch_bounds__(kTraceBlock, (TraceBlocks<kAnyHit, kMulti>::va
                 pBest = record_prim(geo.tris, t.lBest);
                 mBest = record_material(geo.tris, t.lBest);
                 const Frame& f = q.req[slot_of(st.w)];
+                const float4 dt = sdir[threadIdx.x];
+                const float3 dir = make_float3(dt.x, dt.y, dt.z);
                 if (pBest != kNoHit) bucket = __float_as_uint(__ldg(geo.tris + 3 * (size_t)t.lBest + 2).w);
-                else if constexpr (kMulti) miss_accumulate(q.scenes[sceneIdx], f, th, rd, make_float3(t.r.dx, t.r.dy, t.r.dz));
-                else miss_accumulate(s0, f, th, rd, make_float3(t.r.dx, t.r.dy, t.r.dz));
+                else if constexpr (kMulti) miss_accumulate(q.scenes[f.scene], f, th, rd, dir);
+                else miss_accumulate(s0, f, th, rd, dir);
                 missed = pBest == kNoHit;
             }
             count_ended_t(q.ctl, missed, slot_of(st.w));
@@ -470,19 +524,30 @@ __global__ void __launch_bounds__(kTraceBlock, (TraceBlocks<kAnyHit, kMulti>::va
             const bool texL = bucket == (kBucketLambert | kRecTextured);
             if (bucket != kNumBuckets) bucket = texL ? (uint32_t)kBucketLambert : min(bucket, (uint32_t)kBucketOther);
             uint32_t pos = kInvalidSlot;
-#pragma unroll
-            for (uint32_t b = 0; b < kBucketLambertResume; ++b) {
-                uint32_t pb = warp_append_pos(&c->bucket[b].v, bucket == b && !texL, q.capacity, &c->error);
-                if (bucket == b && !texL) pos = pb;
-            }
-            {
-                const uint32_t pt = warp_append_pos(&c->lambertTex.v, texL, q.capacity, &c->error);
-                if (texL && pt != kInvalidSlot) pos = q.capacity - 1u - pt;
+            // the five appends' atomics are issued together, one by each of lanes 0-4
+            const uint32_t dest = texL ? 4u : bucket;
+            const uint32_t m0 = __ballot_sync(0xffffffffu, dest == 0u), m1 = __ballot_sync(0xffffffffu, dest == 1u),
+                           m2 = __ballot_sync(0xffffffffu, dest == 2u), m3 = __ballot_sync(0xffffffffu, dest == 3u),
+                           m4 = __ballot_sync(0xffffffffu, dest == 4u && texL);
+            const uint32_t mine = lane == 0 ? m0 : lane == 1 ? m1 : lane == 2 ? m2 : lane == 3 ? m3 : lane == 4 ? m4 : 0u;
+            uint32_t base = 0;
+            if (mine) base = atomicAdd(lane == 4 ? &c->lambertTex.v : &c->bucket[lane].v, (uint32_t)__popc(mine));
+            base = __shfl_sync(0xffffffffu, base, dest & 7u);
+            if (bucket != kNumBuckets) {
+                const uint32_t peers = dest == 0u ? m0 : dest == 1u ? m1 : dest == 2u ? m2 : dest == 3u ? m3 : m4;
+                pos = base + __popc(peers & ((1u << lane) - 1u));
+                if (pos >= q.capacity) {
+                    atomicOr(&c->error, kErrQueueOverflow);
+                    pos = kInvalidSlot;
+                } else if (texL) {
+                    pos = q.capacity - 1u - pos;
+                }
             }
             if (pos != kInvalidSlot) {
                 const PathQ o = pick_bucket(q, bucket);
-                __stcs(o.ray_o + pos, make_float4(t.r.ox, t.r.oy, t.r.oz, t.r.tmin));
-                __stcs(o.ray_d + pos, make_float4(t.r.dx, t.r.dy, t.r.dz, t.tBest));
+                const float4 dt = sdir[threadIdx.x];
+                __stcs(o.ray_o + pos, make_float4(t.ox, t.oy, t.oz, dt.w));
+                __stcs(o.ray_d + pos, make_float4(dt.x, dt.y, dt.z, t.tBest));
                 o.hit[pos] = make_float4(t.tBest, __uint_as_float(pBest), __uint_as_float(mBest),
                                          __uint_as_float(t.lBest));
                 __stcs(o.thr + pos, th);

@@ -117,6 +117,9 @@ struct DevScene {
     // BVH triangle records in leaf order, 3 float4 each: v0 | prim, v1 - v0 |
     // material, v2 - v0 | bucket (the material's shade bucket, set at finalize)
     const float4* tris;
+    // Per leaf position the triangle there and the next one, component by component
+    // (5 float4: -v0, v1 - v0, v2 - v0), for the traversal's packed two-triangle test
+    const float4* pairs;
     uint32_t numNodes;
     const float4* envMap;  // lat-long RGBA f32 map (null = none); used with WRK_FLAG_ENV_MAP
     uint32_t envW, envH;
@@ -257,9 +260,9 @@ int build_bvh8(const float* d_vtx, const uint32_t* d_idx, const uint32_t* d_triM
 // Sets the per-thread message returned by wrk_last_error(); returns `code`.
 int report_error(int code, const char* msg);
 
-// Writes the shade bucket of each BVH triangle record's material into its e2.w
-// (kernels_misc.cu).
-void launch_leaf_buckets(float4* tris, uint32_t numTris, const wrk_material* mats, uint32_t numMats,
+// Completes the leaf data (kernels_misc.cu): writes the shade bucket of each BVH
+// triangle record's material into its e2.w, and the pair records (5 float4 per leaf position, see DevScene::pairs).
+void launch_leaf_records(float4* tris, uint32_t numTris, const wrk_material* mats, uint32_t numMats, float4* pairs,
                          cudaStream_t st);
 
 // standalone ray queries (trace.cu)

@@ -33,6 +33,68 @@ __device__ __forceinline__ bool mt_rn(const Ray& r, float4 a, float4 b, float4 c
     return true;
 }
 
+// Packed FP32 pairs (sm_100's two-wide FMA pipe instructions): one issue slot for two
+// independent, correctly rounded operations.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float a, float b) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+// mt_rn for the two triangles of a pair record (kPairWords float4: the triangles at
+// one leaf position and the next, component by component), the same operations on
+// each half.  num / det: t's numerator and denominator where inside.
+constexpr uint32_t kPairWords = 5;
+__device__ __forceinline__ void mt_pair(const Ray& r, const float4* __restrict__ p, float2& num, float2& det, bool& in0,
+                                        bool& in1) {
+    const float4 p0 = __ldg(p), p1 = __ldg(p + 1), p2 = __ldg(p + 2), p3 = __ldg(p + 3), p4 = __ldg(p + 4);
+    const f32x2 ax = pack2(p0.x, p0.y), ay = pack2(p0.z, p0.w), az = pack2(p1.x, p1.y), bx = pack2(p1.z, p1.w),
+                by = pack2(p2.x, p2.y), bz = pack2(p2.z, p2.w), cx = pack2(p3.x, p3.y), cy = pack2(p3.z, p3.w),
+                cz = pack2(p4.x, p4.y);
+    const f32x2 dx = pack2(r.dx, r.dx), dy = pack2(r.dy, r.dy), dz = pack2(r.dz, r.dz);
+    const f32x2 nx = pack2(-r.dx, -r.dx), ny = pack2(-r.dy, -r.dy), nz = pack2(-r.dz, -r.dz);
+    // -(a * b) is exactly (-a) * b: the products below are the negated ones of mt_rn
+    const f32x2 px = fma2(dy, cz, mul2(nz, cy)), py = fma2(dz, cx, mul2(nx, cz)), pz = fma2(dx, cy, mul2(ny, cx));
+    const f32x2 d = fma2(bx, px, fma2(by, py, mul2(bz, pz)));
+    // s = o - a; the records hold -v0
+    const f32x2 sx = add2(pack2(r.ox, r.ox), ax), sy = add2(pack2(r.oy, r.oy), ay), sz = add2(pack2(r.oz, r.oz), az);
+    const f32x2 un = fma2(sx, px, fma2(sy, py, mul2(sz, pz)));
+    const f32x2 mone = pack2(-1.0f, -1.0f);
+    const f32x2 tx = mul2(sx, mone), ty = mul2(sy, mone), tz = mul2(sz, mone);
+    const f32x2 qx = fma2(sy, bz, mul2(tz, by)), qy = fma2(sz, bx, mul2(tx, bz)), qz = fma2(sx, by, mul2(ty, bx));
+    const f32x2 vn = fma2(dx, qx, fma2(dy, qy, mul2(dz, qz)));
+    const f32x2 uv = add2(un, vn);
+    const f32x2 tn = fma2(cx, qx, fma2(cy, qy, mul2(cz, qz)));
+    float u0, u1, v0, v1, w0, w1;
+    unpack2(un, u0, u1);
+    unpack2(vn, v0, v1);
+    unpack2(uv, w0, w1);
+    unpack2(d, det.x, det.y);
+    unpack2(tn, num.x, num.y);
+    auto inside = [](float dt, float u, float v, float w) {
+        return dt > 0.0f ? (u >= 0.0f && v >= 0.0f && w <= dt) : (dt < 0.0f && u <= 0.0f && v <= 0.0f && w >= dt);
+    };
+    in0 = inside(det.x, u0, v0, w0);
+    in1 = inside(det.y, u1, v1, w1);
+}
+
 // Does the ray hit the light triangle of light record `lr` (v0, v1, v2 in its first
 // three float4s) within [tmin, tmax]?  The triangle is rebuilt as the BVH builder
 // writes it (v0, v1 - v0, v2 - v0 with correctly rounded subtractions), so the
