@@ -5,17 +5,12 @@
 // Layout: activations NHWC bf16, dense channels (C a multiple of 16); weights
 // [Cout][3*3][Cin] bf16 (K-major: k = tap*Cin + ci, tap = dy*3 + dx).
 //
-// k_conv_fwd  -- implicit GEMM, M = 128 output pixels (a 16 x 8 pixel tile),
-//                N = Cout (padded to 16, <= 256), K = 9 taps x Cin.  Every K step is
-//                one TMA load of the input tile shifted by the tap (zero fill at the
-//                image border comes from the TMA out-of-bounds fill) plus one TMA load
-//                of the weight slice, both K-major in 32/64/128-byte swizzled rows.
-//                Persistent CTAs walk the tiles; one thread issues tcgen05.mma into a
-//                double-buffered TMEM accumulator while four warps run the previous
-//                tile's epilogue (bias, ReLU, optional ReLU-derivative mask of another
-//                tensor, bf16 or f32 store at a channel offset of a wider buffer).
-//                Used for the forward pass and, with flipped / transposed weights, for
-//                the data gradient.
+// k_conv_fwd  -- implicit GEMM, M = 128 output pixels (an 8 x 16 pixel tile), N = output
+//                channels (a multiple of 16, <= 256), K = 9 taps x Cin, from one halo of
+//                the input per tile.  Used for the forward pass and, with flipped /
+//                transposed weights, for the data gradient.  The epilogue also makes the
+//                2x2 average pool, the nearest 2x upsample (four stores) or the network's
+//                output image, so those take no passes of their own.
 // k_conv_wgrad -- weight gradient dW[co][tap][ci] = sum_p G[p][co] X[p+tap][ci]:
 //                M = 128 output channels, N = input channels, K = pixels; both
 //                operands are loaded channel-contiguous (MN-major) so the tap shift
@@ -43,109 +38,203 @@ constexpr uint32_t kTileW = 16, kTileH = 8, kTileP = 128;
 
 __host__ __device__ inline uint32_t round_up(uint32_t x, uint32_t a) { return (x + a - 1) / a * a; }
 
-// ---------------------------------------------------------------------------
-// Epilogue of one 128-pixel tile: thread (warp w, lane l) owns TMEM lane / tile
-// row 32w + l and its N accumulator columns starting at `col`.
-__device__ __forceinline__ void fwd_epilogue(const FwdShape& sh, const Epilogue& ep, uint32_t tmem, uint32_t col,
-                                             uint32_t warp, uint32_t lane, uint32_t b, uint32_t h0, uint32_t w0,
-                                             uint32_t tileW = kTileW) {
-    const uint32_t row = warp * 32 + lane;
-    const uint32_t h = h0 + row / tileW, w = w0 + row % tileW;
-    const size_t pix = ((size_t)b * sh.H + h) * sh.W + w;
-    for (uint32_t c0 = 0; c0 < sh.N; c0 += 16) {
-        float v[16];
-        tmem_ld16(tmem + ((warp * 32u) << 16) + col + c0, v);
-        if (c0 >= ep.coutValid) continue;
-        const uint32_t nv = min(16u, ep.coutValid - c0);
-#pragma unroll
-        for (uint32_t j = 0; j < 16; ++j) {
-            float x = v[j];
-            if (ep.bias && c0 + j < ep.nBias) x += ep.bias[c0 + j];
-            if (ep.relu) x = fmaxf(x, 0.0f);
-            v[j] = x;
-        }
-        if (ep.mask) {
-            const __nv_bfloat16* m = ep.mask + pix * ep.maskStride + ep.maskOffset + c0;
-#pragma unroll
-            for (uint32_t j = 0; j < 16; ++j)
-                if (j < nv && !(__bfloat162float(m[j]) > 0.0f)) v[j] = 0.0f;
-        }
-        if (ep.outF32) {
-            float* o = (float*)ep.out + pix * ep.outStride + ep.outOffset + c0;
-            if (nv == 16 && ((uintptr_t)o & 15u) == 0) {
-#pragma unroll
-                for (uint32_t j = 0; j < 16; j += 4) {
-                    float4 x = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-                    if (ep.accumulate) {
-                        float4 y = *(float4*)(o + j);
-                        x.x += y.x;
-                        x.y += y.y;
-                        x.z += y.z;
-                        x.w += y.w;
-                    }
-                    *(float4*)(o + j) = x;
-                }
-            } else {
-                for (uint32_t j = 0; j < nv; ++j) o[j] = ep.accumulate ? o[j] + v[j] : v[j];
-            }
-        } else {
-            __nv_bfloat16* o = (__nv_bfloat16*)ep.out + pix * ep.outStride + ep.outOffset + c0;
-            if (nv == 16 && ((uintptr_t)o & 15u) == 0) {
-                uint32_t p[8];
-#pragma unroll
-                for (uint32_t j = 0; j < 8; ++j) {
-                    __nv_bfloat162 t = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
-                    p[j] = *(uint32_t*)&t;
-                }
-                *(uint4*)o = make_uint4(p[0], p[1], p[2], p[3]);
-                *(uint4*)(o + 8) = make_uint4(p[4], p[5], p[6], p[7]);
-            } else {
-                for (uint32_t j = 0; j < nv; ++j) o[j] = __float2bfloat16_rn(v[j]);
-            }
-        }
-    }
-}
-
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
-// Persistent: each CTA walks tiles blockIdx.x, += gridDim.x.  Warps 0-3 run the
-// epilogue, warp 4 the TMA producer, warp 5 the MMA issuer.  The stage ring runs
-// across tile boundaries, and the accumulator is double-buffered in TMEM (columns
-// [0, N) and [N, 2N)), so the epilogue of one tile overlaps the next tile's loads
-// and MMAs.
-template <int CHUNK>
-__global__ void __launch_bounds__(192, 1)
-    k_conv_fwd(const __grid_constant__ CUtensorMap mx, const __grid_constant__ CUtensorMap mw, FwdShape sh, Epilogue ep,
-               uint32_t* err) {
+// ---------------------------------------------------------------------------
+// Forward convolution (also the data gradient, with flipped / transposed weights).
+//
+// A work item is one 8 x 16 pixel tile (M = 128) and one slice of N output channels.
+// Its input is the tile's 10 x 18 pixel halo, one TMA load per channel chunk (64, 32 or
+// 16 channels; zero padding from the out-of-bounds fill), stored K-major with one
+// 128 / 64 / 32-byte swizzled row per pixel: the 128 pixels shifted by tap (dy, dx) start
+// dy*10 + dx rows in, with the tile's 8-pixel rows (the M core-matrix groups) 10 rows
+// apart, so all nine taps are descriptors into the same halo and the input crosses
+// L2 -> shared memory once instead of nine times.  The halo chunks form a ring that runs
+// across work items, so the next item's input loads while this one computes.
+//
+// Weights: kResident keeps the layer's whole weight tensor in shared memory; otherwise
+// (tap, chunk) slices stream through a second ring.
+//
+// Warps: epilogue (four or eight), input loads, MMA, weight loads.  The accumulator is
+// double-buffered in TMEM (columns [0, N) and [N, 2N)), so the epilogue of one item
+// overlaps the next one's MMAs.  K runs tap-major, then by channel, whatever the plan:
+// every output sums in the same order.
+//
+// What bounds it, on a 1920 x 1088 frame (device time per layer, before -> now, with the
+// pools and upsamples that were passes of their own, 66 + 178 us, now in it): an M128 K16
+// MMA takes 50-60 cycles up to 64 output channels, whatever their number (its 4 KB input
+// operand), so 96 -> 32 channels at full resolution takes 287 -> 193 us, the MMAs alone
+// 184; the other full-resolution layers waited on their epilogue's 16-byte stores at
+// 64-byte strides (32 -> 32 124 us, 65 without the stores) and now leave through shared
+// memory and TMA stores (75 us); the layers whose weights do not fit waited on L2 ->
+// shared memory traffic, nine copies of the input among it (192 -> 64 202 -> 164 us,
+// 384 -> 128 125 -> 96 us) and now wait on their weight slices' MMA steps (315 cycles for
+// 200 of MMAs at 64 channels).  The whole frame: 1940 -> 1125 us.
+constexpr uint32_t kHaloW = 10, kHaloH = 18, kHaloPix = kHaloW * kHaloH, kHTileW = 8, kHTileH = 16;
+// Epilogue warps: four per accumulator buffer for resident layers (one group of four
+// alternating between the buffers could not keep up with 9-36 MMAs a tile), four in all
+// for streaming ones.
+__host__ __device__ constexpr uint32_t fwd_epilogue_warps(bool resident) { return resident ? 8 : 4; }
+__host__ __device__ constexpr uint32_t fwd_threads(bool resident) { return (fwd_epilogue_warps(resident) + 3) * 32; }
+// Bytes of one channel chunk's halo, padded so that every chunk starts on a swizzle
+// pattern boundary.
+__host__ __device__ constexpr uint32_t halo_block_bytes(uint32_t chunk) {
+    return (kHaloPix * chunk * 2 + 1023) / 1024 * 1024;
+}
+
+// ---- epilogue ----
+// 16-byte unit u of row r in a staging tile of rowBytes-wide rows, swizzled as the TMA
+// store expects it (SWIZZLE_128B / 64B / 32B).
+__device__ __forceinline__ uint32_t staged_unit(uint32_t r, uint32_t u, uint32_t rowBytes) {
+    const uint32_t x = rowBytes == 128 ? (r & 7u) : rowBytes == 64 ? ((r >> 1) & 3u) : ((r >> 2) & 1u);
+    return r * rowBytes + ((u ^ x) << 4);
+}
+__device__ __forceinline__ void st_shared16(uint32_t a, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
+    asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
+}
+__device__ __forceinline__ uint4 ld_shared16(uint32_t a) {
+    uint4 v;
+    asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ uint32_t bf2(float a, float b) {
+    const __nv_bfloat162 t = __floats2bfloat162_rn(a, b);
+    return *(const uint32_t*)&t;
+}
+
+// 16 accumulator columns from channel c0 on (channels of this launch's output): bias,
+// ReLU, ReLU-derivative mask.
+__device__ __forceinline__ void finish16(const Epilogue& ep, const float* bias, uint32_t c0, size_t pix, bool inside,
+                                         float (&v)[16]) {
+    if (ep.bias) {
+#pragma unroll
+        for (uint32_t j = 0; j < 16; j += 4) {
+            const float4 x = *(const float4*)(bias + c0 + j);
+            v[j] += x.x;
+            v[j + 1] += x.y;
+            v[j + 2] += x.z;
+            v[j + 3] += x.w;
+        }
+    }
+    if (ep.relu) {
+#pragma unroll
+        for (uint32_t j = 0; j < 16; ++j) v[j] = fmaxf(v[j], 0.0f);
+    }
+    if (ep.mask && inside) {
+        const __nv_bfloat16* m = ep.mask + pix * ep.maskStride + ep.maskOffset + c0;
+        const uint4 a = *(const uint4*)m, b = *(const uint4*)(m + 8);
+        const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+        for (uint32_t j = 0; j < 8; ++j) {
+            const float2 f = __bfloat1622float2(*(const __nv_bfloat162*)&w[j]);
+            if (!(f.x > 0.0f)) v[2 * j] = 0.0f;
+            if (!(f.y > 0.0f)) v[2 * j + 1] = 0.0f;
+        }
+    }
+}
+
+// 16 finished channels, from channel c of the staged slice on, into a staged row
+// (rowAddr: the row's first byte; x: its swizzle, already times 16)
+__device__ __forceinline__ void stage16(uint32_t rowAddr, uint32_t x, uint32_t c, uint32_t f32, const float (&v)[16]) {
+    if (f32) {
+#pragma unroll
+        for (uint32_t j = 0; j < 4; ++j)
+            st_shared16(rowAddr + ((c * 4 + 16 * j) ^ x), __float_as_uint(v[4 * j]), __float_as_uint(v[4 * j + 1]),
+                        __float_as_uint(v[4 * j + 2]), __float_as_uint(v[4 * j + 3]));
+    } else {
+#pragma unroll
+        for (uint32_t j = 0; j < 2; ++j)
+            st_shared16(rowAddr + ((c * 2 + 16 * j) ^ x), bf2(v[8 * j], v[8 * j + 1]), bf2(v[8 * j + 2], v[8 * j + 3]),
+                        bf2(v[8 * j + 4], v[8 * j + 5]), bf2(v[8 * j + 6], v[8 * j + 7]));
+    }
+}
+
+// 32 accumulator columns: bias, bf16, ReLU (on the rounded pair: rounding keeps the sign),
+// into a staged row.
+__device__ __forceinline__ void stage32(uint32_t rowAddr, uint32_t x, uint32_t c, const float* bias, uint32_t relu,
+                                        const uint32_t (&r)[32]) {
+#pragma unroll
+    for (uint32_t u = 0; u < 4; ++u) {
+        const float4 p = *(const float4*)(bias + 8 * u), q = *(const float4*)(bias + 8 * u + 4);
+        uint32_t w[4] = {bf2(__uint_as_float(r[8 * u]) + p.x, __uint_as_float(r[8 * u + 1]) + p.y),
+                         bf2(__uint_as_float(r[8 * u + 2]) + p.z, __uint_as_float(r[8 * u + 3]) + p.w),
+                         bf2(__uint_as_float(r[8 * u + 4]) + q.x, __uint_as_float(r[8 * u + 5]) + q.y),
+                         bf2(__uint_as_float(r[8 * u + 6]) + q.z, __uint_as_float(r[8 * u + 7]) + q.w)};
+        if (relu) {
+#pragma unroll
+            for (uint32_t j = 0; j < 4; ++j) asm("max.bf16x2 %0, %1, %2;" : "=r"(w[j]) : "r"(w[j]), "r"(0u));
+        }
+        st_shared16(rowAddr + ((c * 2 + 16 * u) ^ x), w[0], w[1], w[2], w[3]);
+    }
+}
+
+// n / d with inv ~ 1 / d: an estimate and its correction (three integer divisions per
+// tile were a fifth of the small layers' epilogue).
+__device__ __forceinline__ uint32_t quotient(uint32_t n, uint32_t d, float inv) {
+    uint32_t q = __float2uint_rz(__uint2float_rz(n) * inv);
+    while ((uint64_t)q * d > n) --q;
+    while ((uint64_t)(q + 1) * d <= n) ++q;
+    return q;
+}
+// Image, first row and first column of a work item's tile, and its first output channel.
+struct TileAt {
+    uint32_t b, h0, w0, n0;
+};
+__device__ __forceinline__ TileAt tile_at(const FwdShape& sh, uint32_t perImg, float invImg, float invX, uint32_t item) {
+    const uint32_t tile = sh.nSplit == 1 ? item : item / sh.nSplit;
+    TileAt t;
+    t.n0 = (item - tile * sh.nSplit) * sh.N;
+    t.b = quotient(tile, perImg, invImg);
+    const uint32_t rem = tile - t.b * perImg, ty = quotient(rem, sh.tilesX, invX);
+    t.h0 = ty * kHTileH;
+    t.w0 = (rem - ty * sh.tilesX) * kHTileW;
+    return t;
+}
+
+// log1p of the clamped radiance: the network's input scale (and its output's base).
+__device__ __forceinline__ float log_radiance(float x) { return log1pf(fmaxf(x, 0.0f)); }
+
+// BLOCKS > 0: the channel chunks of a resident layer, so that the MMA issue is straight
+// code with constant descriptor offsets (0 = sh.Cin / CHUNK at run time).
+template <int CHUNK, bool kResident, int BLOCKS>
+__global__ void __launch_bounds__(fwd_threads(kResident), kResident && BLOCKS != 3 ? 2 : 1)
+    k_conv_fwd(const __grid_constant__ CUtensorMap mx, const __grid_constant__ CUtensorMap mw,
+               const __grid_constant__ OutMaps mo, FwdShape sh, Epilogue ep, uint32_t* err) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    constexpr uint32_t kRow = CHUNK * 2;  // bytes per pixel row / weight row in a stage
-    constexpr uint32_t kABytes = kTileP * kRow;
-    const uint32_t bBytes = round_up(sh.N * kRow, 1024);
-    const uint32_t stageBytes = kABytes + bBytes;
-    const uint32_t S = sh.stages;
-    uint64_t* bars = (uint64_t*)(smem + S * stageBytes);
-    // bars: full[S] empty[S] accFull[2] accEmpty[2] drain
-    uint32_t* tmemSlot = (uint32_t*)(bars + 2 * S + 5);
-    volatile uint32_t* abortFlag = tmemSlot + 1;
+    constexpr uint32_t kRow = CHUNK * 2;  // bytes of a pixel's row of one chunk
+    constexpr uint32_t kEpiWarps = fwd_epilogue_warps(kResident);
+    constexpr uint32_t kBlock = halo_block_bytes(CHUNK);
+    const uint32_t G = BLOCKS > 0 ? BLOCKS : sh.Cin / CHUNK;  // channel chunks
+    const uint32_t wSlice = sh.N * kRow;  // bytes of one (tap, chunk) weight slice
+    const uint32_t RA = sh.stagesA, RB = sh.stagesB;
+    const uint32_t steps = 9 * G;
+    // layout: halo ring | weights (resident or ring) | staging | bias | barriers
     const uint32_t base = smem_u32(smem);
-    auto full = [&](uint32_t s) { return smem_u32(bars + s); };
-    auto empty = [&](uint32_t s) { return smem_u32(bars + S + s); };
-    auto accFull = [&](uint32_t b) { return smem_u32(bars + 2 * S + b); };
-    auto accEmpty = [&](uint32_t b) { return smem_u32(bars + 2 * S + 2 + b); };
-    const uint32_t drain = smem_u32(bars + 2 * S + 4);
+    const uint32_t wBase = base + RA * kBlock;
+    const uint32_t sBase = wBase + round_up((kResident ? steps : RB) * wSlice, 1024);
+    uint8_t* tail = smem + (sBase - base) + sh.stagingBytes * (kEpiWarps / 4);
+    float* biasS = (float*)tail;
+    uint64_t* bars = (uint64_t*)(tail + 1024);
+    // bars: fullA[RA] emptyA[RA] fullB[RB] emptyB[RB] accFull[2] accEmpty[2] drain
+    uint32_t* tmemSlot = (uint32_t*)(bars + 2 * RA + 2 * RB + 5);
+    volatile uint32_t* abortFlag = tmemSlot + 1;
+    auto fullA = [&](uint32_t s) { return smem_u32(bars + s); };
+    auto emptyA = [&](uint32_t s) { return smem_u32(bars + RA + s); };
+    auto fullB = [&](uint32_t s) { return smem_u32(bars + 2 * RA + s); };
+    auto emptyB = [&](uint32_t s) { return smem_u32(bars + 2 * RA + RB + s); };
+    auto accFull = [&](uint32_t b) { return smem_u32(bars + 2 * RA + 2 * RB + b); };
+    auto accEmpty = [&](uint32_t b) { return smem_u32(bars + 2 * RA + 2 * RB + 2 + b); };
+    const uint32_t drain = smem_u32(bars + 2 * RA + 2 * RB + 4);
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
 
     if (threadIdx.x == 0) {
-        for (uint32_t s = 0; s < S; ++s) {
-            mbar_init(full(s), 1);
-            mbar_init(empty(s), 1);
-        }
+        for (uint32_t s = 0; s < 2 * RA + 2 * RB; ++s) mbar_init(smem_u32(bars + s), 1);
         for (uint32_t b = 0; b < 2; ++b) {
             mbar_init(accFull(b), 1);
-            mbar_init(accEmpty(b), 128);
+            mbar_init(accEmpty(b), 4);  // one arrival per epilogue warp
         }
         mbar_init(drain, 1);
         *abortFlag = 0;
@@ -153,6 +242,8 @@ __global__ void __launch_bounds__(192, 1)
         prefetch_map(&mx);
         prefetch_map(&mw);
     }
+    if (ep.bias)
+        for (uint32_t c = threadIdx.x; c < 256; c += blockDim.x) biasS[c] = c < ep.nBias ? ep.bias[c] : 0.0f;
     if (warp == 0) {
         tmem_alloc(smem_u32(tmemSlot), sh.tmemCols);
         tmem_relinquish();
@@ -163,250 +254,284 @@ __global__ void __launch_bounds__(192, 1)
     const uint32_t tmem = *tmemSlot;
 
     const uint32_t perImg = sh.tilesX * sh.tilesY;
-    const uint32_t numTiles = sh.B * perImg;
-    const uint32_t nChunk = sh.Cin / CHUNK;
-    const uint32_t kSteps = 9 * nChunk;
+    const uint32_t items = sh.B * perImg * sh.nSplit;
+    const float invImg = 1.0f / (float)perImg, invX = 1.0f / (float)sh.tilesX;
 
-    if (warp == 4) {
-        if (lane == 0) {  // TMA producer
-            uint32_t kg = 0, issued = 0;
-            for (uint32_t tile = blockIdx.x; tile < numTiles && !*abortFlag; tile += gridDim.x) {
-                const uint32_t b = tile / perImg, rem = tile % perImg;
-                const int h0 = (int)((rem / sh.tilesX) * kTileH), w0 = (int)((rem % sh.tilesX) * kTileW);
-                for (uint32_t k = 0; k < kSteps; ++k, ++kg) {
-                    const uint32_t s = kg % S, round = kg / S;
-                    if (*abortFlag || !mbar_wait(empty(s), (round & 1u) ^ 1u)) {
-                        *abortFlag = 1;
-                        break;
-                    }
-                    const uint32_t tap = k / nChunk, cc = k % nChunk;
-                    const int dy = (int)(tap / 3) - 1, dx = (int)(tap % 3) - 1;
-                    mbar_expect_tx(full(s), kABytes + sh.N * kRow);
-                    tma_load_4d(base + s * stageBytes, &mx, full(s), (int)(cc * CHUNK), w0 + dx, h0 + dy, (int)b);
-                    tma_load_2d(base + s * stageBytes + kABytes, &mw, full(s), (int)(tap * sh.Cin + cc * CHUNK),
-                                (int)sh.wRow0);
-                    ++issued;
-                }
-            }
-            if (*abortFlag) {  // let the copies in flight land before the block exits (bounded)
-                for (uint32_t k = issued > S ? issued - S : 0; k < issued; ++k) mbar_wait(full(k % S), (k / S) & 1u);
-            }
-        }
-    } else if (warp == 5) {
-        if (lane == 0) {  // MMA issuer
-            const uint32_t idesc = idesc_bf16(sh.N, false, false);
-            const uint32_t layout = layout_for_row_bytes(kRow);
-            uint32_t kg = 0, it = 0;
-            for (uint32_t tile = blockIdx.x; tile < numTiles && !*abortFlag; tile += gridDim.x, ++it) {
-                const uint32_t buf = it & 1u, use = it >> 1;
-                if (!mbar_wait(accEmpty(buf), (use & 1u) ^ 1u)) {
-                    *abortFlag = 1;
+    if (warp == kEpiWarps) {
+        // input: one halo chunk per ring slot (the whole warp runs the loop, one lane issues)
+        const bool leader = elect_one();
+        uint32_t s = 0, ph = 1, issued = 0;
+        bool ok = true;
+        for (uint32_t item = blockIdx.x; ok && item < items; item += gridDim.x) {
+            const TileAt at = tile_at(sh, perImg, invImg, invX, item);
+            for (uint32_t g = 0; g < G; ++g) {
+                if (*abortFlag || !warp_wait(emptyA(s), ph)) {
+                    ok = false;
                     break;
                 }
-                tc_fence_after();
-                const uint32_t acc = tmem + buf * sh.N;
-                for (uint32_t k = 0; k < kSteps; ++k, ++kg) {
-                    const uint32_t s = kg % S, round = kg / S;
-                    if (*abortFlag || !mbar_wait(full(s), round & 1u)) {
-                        *abortFlag = 1;
-                        break;
-                    }
-                    tc_fence_after();
-                    const uint32_t a0 = base + s * stageBytes, b0 = a0 + kABytes;
-#pragma unroll
-                    for (uint32_t kk = 0; kk < CHUNK / 16; ++kk) {
-                        const uint64_t ad = sdesc(a0 + kk * 32, 16, 8 * kRow, layout);
-                        const uint64_t bd = sdesc(b0 + kk * 32, 16, 8 * kRow, layout);
-                        umma_bf16(acc, ad, bd, idesc, (k | kk) ? 1u : 0u);
-                    }
-                    umma_commit(empty(s));
+                if (leader) {
+                    mbar_expect_tx(fullA(s), kHaloPix * kRow);
+                    tma_load_4d(base + s * kBlock, &mx, fullA(s), (int)(g * CHUNK), (int)at.w0 - 1, (int)at.h0 - 1,
+                                (int)at.b);
                 }
-                umma_commit(accFull(buf));
-            }
-            // every MMA this thread issued has completed before TMEM is released
-            umma_commit(drain);
-            mbar_wait(drain, 0);
-        }
-    } else {
-        // epilogue warps 0-3
-        uint32_t it = 0;
-        for (uint32_t tile = blockIdx.x; tile < numTiles; tile += gridDim.x, ++it) {
-            const uint32_t buf = it & 1u, use = it >> 1;
-            const bool ready = mbar_wait(accFull(buf), use & 1u);
-            // warp-uniform decision: tcgen05.ld below is .sync.aligned
-            const bool go = __all_sync(0xffffffffu, ready && !*abortFlag);
-            tc_fence_after();
-            if (!go) {
-                *abortFlag = 1;
-                break;
-            }
-            const uint32_t b = tile / perImg, rem = tile % perImg;
-            fwd_epilogue(sh, ep, tmem, buf * sh.N, warp, lane, b, (rem / sh.tilesX) * kTileH,
-                         (rem % sh.tilesX) * kTileW);
-            tc_fence_before();
-            mbar_arrive(accEmpty(buf));
-        }
-    }
-    __syncwarp();
-    tc_fence_before();
-    __syncthreads();
-    if (threadIdx.x == 0 && *abortFlag) atomicOr(err, 1u);
-    if (warp == 0) tmem_dealloc(tmem, sh.tmemCols);
-}
-
-// ---------------------------------------------------------------------------
-// Small-N variant (N <= 128, 9*Cin*N bf16 weights <= 72 KB): the whole weight tensor
-// stays in shared memory for the CTA's life, and each 8 x 16 pixel tile needs one
-// TMA load per 8-channel group of its 10 x 18 pixel halo.  Operands use the
-// non-swizzled K-major layout (8 x 16-byte core matrices): the halo is stored
-// [channel group][pixel][8 channels], so the view of the 128 output pixels shifted
-// by tap (dy, dx) starts (dy*10 + dx) * 16 bytes in, with core matrices (8
-// consecutive pixels of one row) 160 bytes apart along M and 2944 bytes (one
-// 2880-byte channel group, padded to 128 bytes) apart along K: all nine taps are descriptors into the same halo, and the input crosses
-// L2 -> shared memory once instead of nine times.
-constexpr uint32_t kHaloW = 10, kHaloH = 18, kHaloPix = kHaloW * kHaloH, kHTileW = 8, kHTileH = 16;
-// one channel group of a halo: 180 pixels x 16 bytes = 2880, padded so every TMA
-// destination stays 128-byte aligned
-constexpr uint32_t kHaloGroupBytes = 2944;
-
-// CIN > 0: the input channel count is a compile-time constant, so the MMA issuer's
-// 9 x CIN/16 descriptors are fixed offsets from one base descriptor per tile
-// (0 = read sh.Cin at run time).
-template <int CIN>
-__global__ void __launch_bounds__(192, 1)
-    k_conv_fwd_halo(const __grid_constant__ CUtensorMap mh, const __nv_bfloat16* __restrict__ wgt, FwdShape sh,
-                    Epilogue ep, uint32_t* err) {
-    if (CIN > 0) sh.Cin = CIN;
-    extern __shared__ uint8_t smem_raw[];
-    uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    const uint32_t G = sh.Cin / 8;                      // channel groups
-    const uint32_t haloBytes = G * kHaloPix * 16;       // bytes one stage's TMA loads deliver
-    const uint32_t stageBytes = round_up(G * kHaloGroupBytes, 1024);
-    const uint32_t wBytes = round_up(9 * sh.Cin * sh.N * 2, 1024);
-    const uint32_t S = sh.stages;
-    uint8_t* wsm = smem + S * stageBytes;
-    uint64_t* bars = (uint64_t*)(wsm + wBytes);
-    uint32_t* tmemSlot = (uint32_t*)(bars + 2 * S + 5);
-    volatile uint32_t* abortFlag = tmemSlot + 1;
-    const uint32_t base = smem_u32(smem), wbase = smem_u32(wsm);
-    auto full = [&](uint32_t s) { return smem_u32(bars + s); };
-    auto empty = [&](uint32_t s) { return smem_u32(bars + S + s); };
-    auto accFull = [&](uint32_t b) { return smem_u32(bars + 2 * S + b); };
-    auto accEmpty = [&](uint32_t b) { return smem_u32(bars + 2 * S + 2 + b); };
-    const uint32_t drain = smem_u32(bars + 2 * S + 4);
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-
-    // weights -> shared memory, [k group][n][8 channels] (k = tap * Cin + ci)
-    {
-        const uint32_t K = 9 * sh.Cin, units = K / 8 * sh.N;
-        for (uint32_t u = threadIdx.x; u < units; u += blockDim.x) {
-            const uint32_t kg = u / sh.N, n = u % sh.N;
-            const uint4 v = *reinterpret_cast<const uint4*>(wgt + (size_t)(n + sh.wRow0) * K + kg * 8);
-            *reinterpret_cast<uint4*>(wsm + ((size_t)kg * sh.N + n) * 16) = v;
-        }
-        fence_proxy_async();
-    }
-    if (threadIdx.x == 0) {
-        for (uint32_t s = 0; s < S; ++s) {
-            mbar_init(full(s), 1);
-            mbar_init(empty(s), 1);
-        }
-        for (uint32_t b = 0; b < 2; ++b) {
-            mbar_init(accFull(b), 1);
-            mbar_init(accEmpty(b), 128);
-        }
-        mbar_init(drain, 1);
-        *abortFlag = 0;
-        fence_mbar_init();
-        prefetch_map(&mh);
-    }
-    if (warp == 0) {
-        tmem_alloc(smem_u32(tmemSlot), sh.tmemCols);
-        tmem_relinquish();
-    }
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    const uint32_t tmem = *tmemSlot;
-
-    const uint32_t perImg = sh.tilesX * sh.tilesY;  // 8 x 16 tiles
-    const uint32_t numTiles = sh.B * perImg;
-
-    if (warp == 4) {
-        if (lane == 0) {  // TMA producer: one halo per tile
-            uint32_t it = 0, issued = 0;
-            for (uint32_t tile = blockIdx.x; tile < numTiles && !*abortFlag; tile += gridDim.x, ++it) {
-                const uint32_t s = it % S, round = it / S;
-                if (!mbar_wait(empty(s), (round & 1u) ^ 1u)) {
-                    *abortFlag = 1;
-                    break;
-                }
-                const uint32_t b = tile / perImg, rem = tile % perImg;
-                const int h0 = (int)((rem / sh.tilesX) * kHTileH), w0 = (int)((rem % sh.tilesX) * kHTileW);
-                mbar_expect_tx(full(s), haloBytes);
-                for (uint32_t g = 0; g < G; ++g)
-                    tma_load_4d(base + s * stageBytes + g * kHaloGroupBytes, &mh, full(s), (int)(g * 8), w0 - 1,
-                                h0 - 1, (int)b);
                 ++issued;
-            }
-            if (*abortFlag) {
-                for (uint32_t k = issued > S ? issued - S : 0; k < issued; ++k) mbar_wait(full(k % S), (k / S) & 1u);
+                if (++s == RA) {
+                    s = 0;
+                    ph ^= 1u;
+                }
             }
         }
-    } else if (warp == 5) {
-        if (lane == 0) {  // MMA issuer
-            const uint32_t idesc = idesc_bf16(sh.N, false, false);
-            const uint32_t lboA = kHaloGroupBytes, sboA = kHaloW * 16;  // K step of 8 channels, M step of 8 pixels
-            const uint32_t lboB = sh.N * 16, sboB = 8 * 16;
-            uint32_t it = 0;
-            for (uint32_t tile = blockIdx.x; tile < numTiles && !*abortFlag; tile += gridDim.x, ++it) {
-                const uint32_t buf = it & 1u, use = it >> 1;
-                const uint32_t s = it % S, round = it / S;
-                if (!mbar_wait(accEmpty(buf), (use & 1u) ^ 1u) || !mbar_wait(full(s), round & 1u)) {
-                    *abortFlag = 1;
-                    break;
-                }
-                tc_fence_after();
-                const uint32_t acc = tmem + buf * sh.N;
-                // descriptors advance by (byte offset >> 4) in their low 14-bit address field
-                const uint64_t a0 = sdesc(base + s * stageBytes, lboA, sboA, 0);
-                const uint64_t b0 = sdesc(wbase, lboB, sboB, 0);
-                const uint32_t nUnits = sh.N;  // lboB >> 4
-                constexpr uint32_t kKC = CIN > 0 ? CIN / 16 : 8;
-#pragma unroll
-                for (uint32_t tap = 0; tap < 9; ++tap) {
-                    const uint32_t shift = ((tap / 3) * kHaloW + (tap % 3));  // 16-byte units
-#pragma unroll
-                    for (uint32_t kk = 0; kk < kKC; ++kk) {
-                        if (CIN == 0 && kk >= sh.Cin / 16) break;
-                        const uint64_t ad = a0 + (2 * kk * (kHaloGroupBytes >> 4) + shift);
-                        const uint64_t bd = b0 + ((tap * sh.Cin + 16 * kk) / 8) * nUnits;
-                        umma_bf16(acc, ad, bd, idesc, (tap | kk) ? 1u : 0u);
+        if (!ok) {  // let the copies in flight land before the block exits (bounded)
+            *abortFlag = 1;
+            for (uint32_t j = issued > RA ? issued - RA : 0; j < issued; ++j) mbar_wait(fullA(j % RA), (j / RA) & 1u);
+        }
+    } else if (warp == kEpiWarps + 2) {
+        // weights
+        const bool leader = elect_one();
+        if (kResident) {
+            if (leader) {
+                mbar_expect_tx(fullB(0), steps * wSlice);
+                for (uint32_t k = 0; k < steps; ++k) tma_load_2d(wBase + k * wSlice, &mw, fullB(0), (int)(k * CHUNK), 0);
+            }
+            __syncwarp();
+            if (!warp_wait(fullB(0), 0)) *abortFlag = 1;
+        } else {
+            if (leader) {
+                uint32_t s = 0, ph = 1, issued = 0;
+                bool ok = true;
+                for (uint32_t item = blockIdx.x; ok && item < items; item += gridDim.x) {
+                    const int row = (int)((item % sh.nSplit) * sh.N);
+                    for (uint32_t j = 0; j < steps; ++j) {
+                        if (!mbar_wait(emptyB(s), ph)) {
+                            ok = false;
+                            break;
+                        }
+                        mbar_expect_tx(fullB(s), wSlice);
+                        tma_load_2d(wBase + s * wSlice, &mw, fullB(s), (int)(j * CHUNK), row);
+                        ++issued;
+                        if (++s == RB) {
+                            s = 0;
+                            ph ^= 1u;
+                        }
                     }
+                    ok = ok && !*abortFlag;
                 }
-                umma_commit(empty(s));
-                umma_commit(accFull(buf));
+                if (!ok) {
+                    *abortFlag = 1;
+                    for (uint32_t j = issued > RB ? issued - RB : 0; j < issued; ++j) mbar_wait(fullB(j % RB), (j / RB) & 1u);
+                }
             }
-            umma_commit(drain);
-            mbar_wait(drain, 0);
         }
-    } else {
-        uint32_t it = 0;
-        for (uint32_t tile = blockIdx.x; tile < numTiles; tile += gridDim.x, ++it) {
+    } else if (warp == kEpiWarps + 1) {
+        // MMA issuer: the whole warp runs the loop (uniform control flow and operands), one
+        // elected lane issues
+        const uint32_t leader = elect_one();
+        const uint32_t idesc = idesc_bf16(sh.N, false, false);
+        const uint32_t layout = layout_for_row_bytes(kRow);
+        // descriptors advance by (byte offset >> 4) in their low 14-bit address field
+        const uint64_t a0 = sdesc(base, 16, kHaloW * kRow, layout);
+        const uint64_t b0 = sdesc(wBase, 16, 8 * kRow, layout);
+        uint32_t sa0 = 0, phA = 0, sb = 0, phB = 0, it = 0;  // ring positions and their phases
+        bool ok = true;
+        if (kResident) ok = warp_wait(fullB(0), 0);
+        for (uint32_t item = blockIdx.x; ok && item < items; item += gridDim.x, ++it) {
             const uint32_t buf = it & 1u, use = it >> 1;
-            const bool ready = mbar_wait(accFull(buf), use & 1u);
-            const bool go = __all_sync(0xffffffffu, ready && !*abortFlag);
+            if (!(ok = warp_wait(accEmpty(buf), (use & 1u) ^ 1u))) break;
+            // orders the MMAs after the epilogue's TMEM loads; the operands come from TMA and
+            // need only their barriers
             tc_fence_after();
-            if (!go) {
+            const uint32_t acc = tmem + buf * sh.N;
+            if constexpr (kResident && BLOCKS > 0) {
+                uint64_t ad[BLOCKS];
+#pragma unroll
+                for (uint32_t g = 0; g < BLOCKS; ++g) {
+                    const bool wrap = sa0 + g >= RA;
+                    const uint32_t sa = wrap ? sa0 + g - RA : sa0 + g;
+                    if (ok) ok = warp_wait(fullA(sa), phA ^ (wrap ? 1u : 0u));
+                    ad[g] = a0 + sa * (kBlock >> 4);
+                }
+                if (!ok) break;
+                const uint32_t ws = wSlice >> 4;
+                if (leader) {
+#pragma unroll
+                    for (uint32_t tap = 0; tap < 9; ++tap) {
+                        const uint32_t shift = ((tap / 3) * kHaloW + (tap % 3)) * (kRow >> 4);  // 16-byte units
+#pragma unroll
+                        for (uint32_t g = 0; g < BLOCKS; ++g) {
+                            const uint64_t bd = b0 + (tap * BLOCKS + g) * ws;
+#pragma unroll
+                            for (uint32_t kk = 0; kk < CHUNK / 16; ++kk)
+                                umma_bf16(acc, ad[g] + (shift + 2 * kk), bd + 2 * kk, idesc, (tap | g | kk) ? 1u : 0u);
+                        }
+                    }
+#pragma unroll
+                    for (uint32_t g = 0; g < BLOCKS; ++g) umma_commit(emptyA(sa0 + g >= RA ? sa0 + g - RA : sa0 + g));
+                    umma_commit(accFull(buf));
+                }
+                __syncwarp();
+            } else {
+                for (uint32_t g = 0; g < G && ok; ++g) {
+                    const bool wrap = sa0 + g >= RA;
+                    ok = warp_wait(fullA(wrap ? sa0 + g - RA : sa0 + g), phA ^ (wrap ? 1u : 0u));
+                }
+                if (!ok) break;
+                // one lane runs the item's steps (a branch per step cost more than its MMAs)
+                if (leader) {
+#pragma unroll
+                    for (uint32_t tap = 0; tap < 9; ++tap) {
+                        const uint32_t shift = ((tap / 3) * kHaloW + (tap % 3)) * (kRow >> 4);
+                        uint32_t sa = sa0;
+                        for (uint32_t g = 0; g < G; ++g) {
+                            // (a wait that gave up leaves garbage sums and the error flag)
+                            if (!kResident && !mbar_wait(fullB(sb), phB)) *abortFlag = 1;
+                            const uint64_t ad = a0 + (sa * (kBlock >> 4) + shift);
+                            const uint64_t bd = b0 + (kResident ? tap * G + g : sb) * (wSlice >> 4);
+#pragma unroll
+                            for (uint32_t kk = 0; kk < CHUNK / 16; ++kk)
+                                umma_bf16(acc, ad + 2 * kk, bd + 2 * kk, idesc, (tap | g | kk) ? 1u : 0u);
+                            if (!kResident) {
+                                umma_commit(emptyB(sb));
+                                if (++sb == RB) {
+                                    sb = 0;
+                                    phB ^= 1u;
+                                }
+                            }
+                            if (tap == 8) umma_commit(emptyA(sa));
+                            if (++sa == RA) sa = 0;
+                        }
+                    }
+                    umma_commit(accFull(buf));
+                }
+                __syncwarp();
+                ok = !*abortFlag;
+            }
+            sa0 += G;
+            if (sa0 >= RA) {
+                sa0 -= RA;
+                phA ^= 1u;
+            }
+        }
+        if (!ok) *abortFlag = 1;
+        // every MMA has completed before TMEM is released
+        if (leader) umma_commit(drain);
+        __syncwarp();
+        mbar_wait(drain, 0);
+    } else {
+        // Epilogue: lane l of a group's warp w owns tile row (pixel) 32w + l.  A warp's 32 rows
+        // are four whole image rows of the tile, so it stages, pools and stores them by
+        // itself: no barrier joins the warps.
+        const uint32_t quad = warp & 3u, px = lane % kHTileW, py = lane / kHTileW;
+        const uint32_t rowBytes = sh.stagingBytes / 128, sliceC = ep.outF32 ? rowBytes / 4 : rowBytes / 2;
+        const uint32_t stg = sBase + warp * 32 * rowBytes;
+        const uint32_t rowAddr = stg + lane * rowBytes, rowSwz = staged_unit(lane, 0, rowBytes) - lane * rowBytes;
+        const bool plain = ep.bias && !ep.mask && !ep.outF32;  // bias, ReLU, bf16: the network's layers
+        uint32_t it = 0;
+        for (uint32_t item = blockIdx.x; item < items; item += gridDim.x, ++it) {
+            const uint32_t buf = it & 1u, use = it >> 1;
+            if (kEpiWarps == 8 && (warp >> 2) != buf) continue;  // the other group's buffer
+            const TileAt ta = tile_at(sh, perImg, invImg, invX, item);
+            const uint32_t n0 = ta.n0, b = ta.b, w0 = ta.w0, h0 = ta.h0 + quad * 4;  // the warp's rows
+            const uint32_t h = h0 + py, w = w0 + px;
+            const bool inside = h < sh.H;
+            const size_t pix = ((size_t)b * sh.H + h) * sh.W + w;
+            const size_t headAt = ((size_t)b * ep.headH + h) * ep.headW + w;
+            float rgb[3] = {0.0f, 0.0f, 0.0f};  // (fetched ahead of the wait)
+            if (ep.headDst && h < ep.headH && w < ep.headW)
+                for (uint32_t j = 0; j < 3; ++j) rgb[j] = ep.headRgb[3 * headAt + j];
+            if (*abortFlag || !warp_wait(accFull(buf), use & 1u)) {
                 *abortFlag = 1;
                 break;
             }
-            const uint32_t b = tile / perImg, rem = tile % perImg;
-            fwd_epilogue(sh, ep, tmem, buf * sh.N, warp, lane, b, (rem / sh.tilesX) * kHTileH,
-                         (rem % sh.tilesX) * kHTileW, kHTileW);
+            __syncwarp();
+            tc_fence_after();
+            const uint32_t tAcc = tmem + ((quad * 32u) << 16) + buf * sh.N;
+            if (ep.nOut) {
+                for (uint32_t c0 = 0; c0 < sh.N; c0 += sliceC) {
+                    if (lane == 0) bulk_wait_read<0>();  // the last store from this buffer has read it
+                    __syncwarp();
+                    if (sliceC % 32 == 0) {
+                        for (uint32_t c = 0; c < sliceC; c += 32) {
+                            uint32_t r[32];
+                            tmem_ld32_async(tAcc + c0 + c, r);
+                            tmem_ld_wait();
+                            if (plain) {
+                                stage32(rowAddr, rowSwz, c, biasS + n0 + c0 + c, ep.relu, r);
+                                continue;
+                            }
+#pragma unroll
+                            for (uint32_t q = 0; q < 2; ++q) {
+                                float v[16];
+#pragma unroll
+                                for (uint32_t j = 0; j < 16; ++j) v[j] = __uint_as_float(r[16 * q + j]);
+                                finish16(ep, biasS, n0 + c0 + c + 16 * q, pix, inside, v);
+                                stage16(rowAddr, rowSwz, c + 16 * q, ep.outF32, v);
+                            }
+                        }
+                    } else {
+                        float v[16];  // sliceC == 16
+                        tmem_ld16(tAcc + c0, v);
+                        finish16(ep, biasS, n0 + c0, pix, inside, v);
+                        stage16(rowAddr, rowSwz, 0, ep.outF32, v);
+                    }
+                    fence_proxy_async();
+                    __syncwarp();
+                    if (lane == 0 && h0 < sh.H) {
+                        for (uint32_t o = 0; o < ep.nOut; ++o)
+                            tma_store_4d(&mo.m[o], stg, (int)(n0 + c0), (int)w0, (int)h0, (int)b);
+                        bulk_commit();
+                    }
+                    if (ep.pool && h0 < sh.H) {
+                        // 2x2 averages of the stored (bf16) values: one 8-channel group of one
+                        // of the warp's 8 pooled pixels per step
+                        const uint32_t lg = sliceC == 64 ? 3u : sliceC == 32 ? 2u : 1u;  // log2(sliceC / 8)
+                        for (uint32_t k = lane; k < (8u << lg); k += 32) {
+                            const uint32_t g8 = k & ((1u << lg) - 1u), q = k >> lg, qy = q / 4, qx = q % 4;
+                            float s8[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll
+                            for (uint32_t d = 0; d < 4; ++d) {
+                                const uint32_t r = (2 * qy + (d >> 1)) * kHTileW + 2 * qx + (d & 1u);
+                                const uint4 u = ld_shared16(stg + staged_unit(r, g8, rowBytes));
+                                const uint32_t ww[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+                                for (uint32_t j = 0; j < 4; ++j) {
+                                    const float2 f = __bfloat1622float2(*(const __nv_bfloat162*)&ww[j]);
+                                    s8[2 * j] += f.x;
+                                    s8[2 * j + 1] += f.y;
+                                }
+                            }
+                            const size_t pp = ((size_t)b * (sh.H / 2) + h0 / 2 + qy) * (sh.W / 2) + w0 / 2 + qx;
+                            *(uint4*)(ep.pool + pp * ep.poolStride + n0 + c0 + g8 * 8) =
+                                make_uint4(bf2(s8[0] * 0.25f, s8[1] * 0.25f), bf2(s8[2] * 0.25f, s8[3] * 0.25f),
+                                           bf2(s8[4] * 0.25f, s8[5] * 0.25f), bf2(s8[6] * 0.25f, s8[7] * 0.25f));
+                        }
+                    }
+                }
+            } else {
+                for (uint32_t c0 = 0; c0 < sh.N; c0 += 16) {
+                    float v[16];
+                    tmem_ld16(tAcc + c0, v);
+                    if (n0 + c0 >= ep.coutValid || !inside) continue;
+                    finish16(ep, biasS, n0 + c0, pix, inside, v);
+                    if (ep.headDst) {
+                        // the network's last layer: radiance = expm1(log1p(rgb) + residual), cropped
+                        if (h < ep.headH && w < ep.headW)
+                            for (uint32_t j = 0; j < 3; ++j)
+                                ep.headDst[3 * headAt + j] = fmaxf(expm1f(log_radiance(rgb[j]) + v[j]), 0.0f);
+                        continue;
+                    }
+                    const uint32_t nv = min(16u, ep.coutValid - n0 - c0);
+                    const size_t at = pix * ep.outStride + ep.outOffset + n0 + c0;
+                    for (uint32_t j = 0; j < nv; ++j) {
+                        if (ep.outF32) ((float*)ep.out)[at + j] = v[j];
+                        else ((__nv_bfloat16*)ep.out)[at + j] = __float2bfloat16_rn(v[j]);
+                    }
+                }
+            }
             tc_fence_before();
-            mbar_arrive(accEmpty(buf));
+            __syncwarp();
+            if (lane == 0) mbar_arrive(accEmpty(buf));
         }
+        if (lane == 0) bulk_wait_all();
     }
     __syncwarp();
     tc_fence_before();
@@ -582,20 +707,6 @@ int make_act_map(CUtensorMap* m, const void* base, uint32_t C, uint32_t W, uint3
     return r == CUDA_SUCCESS ? 0 : 3;
 }
 
-int make_weight_map(CUtensorMap* m, const void* base, uint32_t K, uint32_t rows, uint32_t boxK, uint32_t boxRows) {
-    EncodeTiledFn enc = encode_fn();
-    if (!enc) return 1;
-    if (((uintptr_t)base & 15u) || (K * 2) % 16 || boxRows > 256) return 2;
-    cuuint64_t dims[2] = {K, rows};
-    cuuint64_t strides[1] = {(cuuint64_t)K * 2};
-    cuuint32_t box[2] = {boxK, boxRows};
-    cuuint32_t es[2] = {1, 1};
-    CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, es,
-                     CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle_for(boxK * 2), CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return r == CUDA_SUCCESS ? 0 : 3;
-}
-
 static uint32_t pow2_cols(uint32_t n) {
     uint32_t c = 32;
     while (c < n) c <<= 1;
@@ -614,61 +725,116 @@ static uint32_t smem_for(uint32_t need, uint32_t tmemCols) {
 
 int chunk_for(uint32_t c) { return c % 64 == 0 ? 64 : c % 32 == 0 ? 32 : 16; }
 
-int plan_fwd(uint32_t B, uint32_t H, uint32_t W, uint32_t Cin, uint32_t N, uint32_t numSMs, FwdPlan* p) {
-    if (Cin == 0 || Cin % 16 || N == 0 || N % 16 || N > 256 || W % kTileW || H % kTileH || B == 0) return 1;
+// Work split and rings of a forward launch.  Weights stay resident when they take at most
+// 72 KB (two blocks then share an SM where their rings fit); otherwise they stream, and
+// where an image has fewer tiles than the GPU has SMs the output channels are split over
+// blocks (a tile of 256 -> 256 channels takes a block 15 us per 128 output channels).
+int plan_fwd(uint32_t B, uint32_t H, uint32_t W, uint32_t Cin, uint32_t N, bool outF32, uint32_t numSMs, FwdPlan* p) {
+    if (Cin == 0 || Cin % 16 || N == 0 || N % 16 || W % 8 || H % 8 || B == 0) return 1;
     FwdShape& sh = p->shape;
     sh.B = B;
     sh.H = H;
     sh.W = W;
     sh.Cin = Cin;
-    sh.N = N;
-    sh.tilesX = W / kTileW;
-    sh.tilesY = H / kTileH;
-    sh.tmemCols = pow2_cols(2 * N);  // double-buffered accumulator
-    sh.wRow0 = 0;
+    sh.tilesX = W / kHTileW;
+    sh.tilesY = (H + kHTileH - 1) / kHTileH;
     p->chunk = chunk_for(Cin);
-    const uint32_t row = p->chunk * 2;
-    const uint32_t stage = kTileP * row + round_up(N * row, 1024);
-    uint32_t S = std::max(2u, std::min(8u, (100u * 1024u) / stage));
-    if (S * stage > 200u * 1024u) S = std::max(2u, (200u * 1024u) / stage);
-    sh.stages = S;
-    p->smem = smem_for(S * stage + (2 * S + 5) * 8 + 16 + 1024, sh.tmemCols);
-    p->halo = false;
-    const uint32_t wBytes = round_up(9 * Cin * N * 2, 1024);
-    if (N <= 128 && wBytes <= 72u * 1024u && H % kHTileH == 0 && W % kHTileW == 0) {
-        // small N: weights resident, one halo per 8 x 16 tile
-        p->halo = true;
-        sh.tilesX = W / kHTileW;
-        sh.tilesY = H / kHTileH;
-        const uint32_t hs = round_up(Cin / 8 * kHaloGroupBytes, 1024);
-        uint32_t Sh = std::max(2u, std::min(4u, (200u * 1024u - wBytes) / hs));
-        sh.stages = Sh;
-        p->smem = smem_for(Sh * hs + wBytes + (2 * Sh + 5) * 8 + 16 + 1024, sh.tmemCols);
-    }
+    const uint32_t kRow = p->chunk * 2, G = Cin / p->chunk, block = halo_block_bytes(p->chunk);
     const uint32_t tiles = B * sh.tilesX * sh.tilesY;
+    sh.nSplit = 1;
+    p->resident = N <= 128 && 9 * Cin * N * 2 <= 72u * 1024u;
+    if (!p->resident) {
+        // at most 192 channels an item, so that the weight ring holds several slices
+        while (N / sh.nSplit > 192 || N % sh.nSplit || (N / sh.nSplit) % 16)
+            if (++sh.nSplit > N / 16) return 1;
+        while (tiles * sh.nSplit * 2 <= numSMs && (N / sh.nSplit) % 64 == 0) sh.nSplit *= 2;
+    }
+    sh.N = N / sh.nSplit;
+    sh.tmemCols = pow2_cols(2 * sh.N);  // double-buffered accumulator
+    const uint32_t wSlice = sh.N * kRow, sliceC = outF32 ? (sh.N % 32 ? 16u : 32u) : (sh.N % 64 == 0 ? 64u : sh.N % 32 == 0 ? 32u : 16u);
+    p->sliceC = sliceC;
+    sh.stagingBytes = 128 * sliceC * (outF32 ? 4 : 2);
+    const uint32_t staging = sh.stagingBytes * (fwd_epilogue_warps(p->resident) / 4);
+    const uint32_t fixed = staging + 1024 /* bias */ + 1024 /* alignment */ + 1024 /* barriers */;
+    auto need = [&](uint32_t ra, uint32_t rb) {
+        return ra * block + round_up((p->resident ? 9 * G : rb) * wSlice, 1024) + fixed;
+    };
+    const uint32_t limit = 227u * 1024u, smPool = 228u * 1024u;
+    if (p->resident) {
+        // two blocks per SM where that leaves each three items' halos in flight
+        sh.stagesB = 1;
+        sh.stagesA = G;
+        for (uint32_t blocks = std::min(2u, 512u / sh.tmemCols); blocks >= 1; --blocks) {
+            const uint32_t room = std::min(limit, smPool / blocks - 1024u);
+            uint32_t ra = 8 * G;
+            while (ra > G && need(ra, 1) > room) --ra;
+            if (blocks == 1 || (need(ra, 1) <= room && ra >= 3 * G)) {
+                sh.stagesA = ra;
+                break;
+            }
+        }
+    } else {
+        // halos of one item at least and of two if that leaves six weight slices (a slice is
+        // 200-400 cycles of MMAs and takes ~2000 to be released and arrive)
+        sh.stagesA = 2 * G;
+        while (sh.stagesA > G && need(sh.stagesA, 6) > limit) --sh.stagesA;
+        sh.stagesB = 16;
+        while (sh.stagesB > 2 && need(sh.stagesA, sh.stagesB) > limit) --sh.stagesB;
+    }
+    if (need(sh.stagesA, sh.stagesB) > limit) return 1;
+    p->smem = smem_for(need(sh.stagesA, sh.stagesB), sh.tmemCols);
     const uint32_t perSM = std::max(1u, std::min(228u * 1024u / (p->smem + 1024u), 512u / sh.tmemCols));
-    p->grid = std::min(tiles, perSM * numSMs);
+    p->grid = std::min(tiles * sh.nSplit, perSM * numSMs);
     return 0;
 }
 
-static int make_halo_map(CUtensorMap* m, const void* base, uint32_t C, uint32_t W, uint32_t H, uint32_t B) {
+static int encode4(CUtensorMap* m, CUtensorMapDataType type, const void* base, const cuuint64_t (&dims)[4],
+                   const cuuint64_t (&strides)[3], const cuuint32_t (&box)[4], uint32_t rowBytes) {
     EncodeTiledFn enc = encode_fn();
     if (!enc) return 1;
-    if (((uintptr_t)base & 15u) || (C * 2) % 16) return 2;
-    cuuint64_t dims[4] = {C, W, H, B};
-    cuuint64_t strides[3] = {(cuuint64_t)C * 2, (cuuint64_t)W * C * 2, (cuuint64_t)H * W * C * 2};
-    cuuint32_t box[4] = {8, kHaloW, kHaloH, 1};
-    cuuint32_t es[4] = {1, 1, 1, 1};
-    CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, es,
-                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (((uintptr_t)base & 15u) || strides[0] % 16 || strides[1] % 16 || strides[2] % 16) return 2;
+    const cuuint32_t es[4] = {1, 1, 1, 1};
+    CUresult r = enc(m, type, 4, const_cast<void*>(base), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                     swizzle_for(rowBytes), CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? 0 : 3;
 }
 
 int make_input_map(const FwdPlan& p, const void* x, CUtensorMap* mx) {
     const FwdShape& sh = p.shape;
-    if (p.halo) return make_halo_map(mx, x, sh.Cin, sh.W, sh.H, sh.B);
-    return make_act_map(mx, x, sh.Cin, sh.W, sh.H, sh.B, p.chunk);
+    const cuuint64_t px = (cuuint64_t)sh.Cin * 2;
+    return encode4(mx, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, x, {sh.Cin, sh.W, sh.H, sh.B}, {px, px * sh.W, px * sh.W * sh.H},
+                   {(cuuint32_t)p.chunk, kHaloW, kHaloH, 1}, p.chunk * 2);
+}
+
+int make_weight_map(const FwdPlan& p, const void* w, CUtensorMap* mw) {
+    EncodeTiledFn enc = encode_fn();
+    if (!enc) return 1;
+    const FwdShape& sh = p.shape;
+    if ((uintptr_t)w & 15u) return 2;
+    const cuuint64_t dims[2] = {9ull * sh.Cin, (cuuint64_t)sh.N * sh.nSplit};
+    const cuuint64_t strides[1] = {18ull * sh.Cin};
+    const cuuint32_t box[2] = {(cuuint32_t)p.chunk, sh.N};
+    const cuuint32_t es[2] = {1, 1};
+    CUresult r = enc(mw, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(w), dims, strides, box, es,
+                     CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle_for(p.chunk * 2), CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? 0 : 3;
+}
+
+int make_out_maps(const FwdPlan& p, void* out, uint32_t stride, uint32_t offset, bool f32, bool up, OutMaps* mo) {
+    const FwdShape& sh = p.shape;
+    const size_t es = f32 ? 4 : 2;
+    const uint32_t C = sh.N * sh.nSplit, f = up ? 2 : 1;
+    memset(mo, 0, sizeof(*mo));
+    for (uint32_t o = 0; o < (up ? 4u : 1u); ++o) {
+        const size_t px = stride * es, row = px * sh.W * f;
+        uint8_t* base = (uint8_t*)out + offset * es + (o >> 1) * row + (o & 1u) * px;
+        const int rc = encode4(&mo->m[o], f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, base,
+                               {C, sh.W, sh.H, sh.B}, {px * f, row * f, row * f * sh.H},
+                               {p.sliceC, kHTileW, 4, 1}, (uint32_t)(p.sliceC * es));
+        if (rc) return rc;
+    }
+    return 0;
 }
 
 int plan_wgrad(uint32_t B, uint32_t H, uint32_t W, uint32_t Cin, uint32_t Cout, uint32_t numSMs, WgradPlan* p) {
@@ -709,43 +875,27 @@ static cudaError_t set_smem(K kern, uint32_t bytes) {
     return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
-cudaError_t launch_fwd(const FwdPlan& p, const CUtensorMap& mx, const CUtensorMap& mw, const void* w,
+cudaError_t launch_fwd(const FwdPlan& p, const CUtensorMap& mx, const CUtensorMap& mw, const OutMaps& mo,
                        const Epilogue& ep, uint32_t* err, cudaStream_t st) {
-    cudaError_t e = cudaSuccess;
-    if (p.halo) {
-        const __nv_bfloat16* wb = (const __nv_bfloat16*)w;
-#define WRK_HALO_CASE(C)                                                                       \
-    case C:                                                                                    \
-        e = set_smem(k_conv_fwd_halo<C>, p.smem);                                             \
-        if (e == cudaSuccess) k_conv_fwd_halo<C><<<p.grid, 192, p.smem, st>>>(mx, wb, p.shape, ep, err); \
-        break;
-        switch (p.shape.Cin) {
-            WRK_HALO_CASE(16)
-            WRK_HALO_CASE(32)
-            WRK_HALO_CASE(64)
-            WRK_HALO_CASE(96)
-            default:
-                e = set_smem(k_conv_fwd_halo<0>, p.smem);
-                if (e == cudaSuccess) k_conv_fwd_halo<0><<<p.grid, 192, p.smem, st>>>(mx, wb, p.shape, ep, err);
-                break;
-        }
-#undef WRK_HALO_CASE
-        return e != cudaSuccess ? e : cudaGetLastError();
+    cudaError_t e = cudaErrorInvalidValue;
+#define WRK_FWD_CASE(CHUNK, RES, BLOCKS)                                                                  \
+    if (p.chunk == CHUNK && p.resident == RES && (BLOCKS == 0 || p.shape.Cin == CHUNK * BLOCKS)) {        \
+        e = set_smem(k_conv_fwd<CHUNK, RES, BLOCKS>, p.smem);                                             \
+        if (e == cudaSuccess)                                                                             \
+            k_conv_fwd<CHUNK, RES, BLOCKS><<<p.grid, fwd_threads(RES), p.smem, st>>>(mx, mw, mo, p.shape, ep, err); \
+        return e != cudaSuccess ? e : cudaGetLastError();                                                 \
     }
-    switch (p.chunk) {
-        case 64:
-            e = set_smem(k_conv_fwd<64>, p.smem);
-            if (e == cudaSuccess) k_conv_fwd<64><<<p.grid, 192, p.smem, st>>>(mx, mw, p.shape, ep, err);
-            break;
-        case 32:
-            e = set_smem(k_conv_fwd<32>, p.smem);
-            if (e == cudaSuccess) k_conv_fwd<32><<<p.grid, 192, p.smem, st>>>(mx, mw, p.shape, ep, err);
-            break;
-        default:
-            e = set_smem(k_conv_fwd<16>, p.smem);
-            if (e == cudaSuccess) k_conv_fwd<16><<<p.grid, 192, p.smem, st>>>(mx, mw, p.shape, ep, err);
-            break;
-    }
+    WRK_FWD_CASE(16, true, 1)
+    WRK_FWD_CASE(32, true, 1)
+    WRK_FWD_CASE(32, true, 3)
+    WRK_FWD_CASE(64, true, 1)
+    WRK_FWD_CASE(16, true, 0)
+    WRK_FWD_CASE(32, true, 0)
+    WRK_FWD_CASE(64, true, 0)
+    WRK_FWD_CASE(16, false, 0)
+    WRK_FWD_CASE(32, false, 0)
+    WRK_FWD_CASE(64, false, 0)
+#undef WRK_FWD_CASE
     return e != cudaSuccess ? e : cudaGetLastError();
 }
 

@@ -9,23 +9,34 @@ namespace wrk {
 namespace conv {
 
 struct FwdShape {
-    uint32_t B, H, W, Cin, N;  // N = output channels padded to a multiple of 16 (<= 256)
-    uint32_t tilesX, tilesY;   // 16 x 8 pixel tiles
-    uint32_t stages, tmemCols;
-    uint32_t wRow0;            // first weight row (output channel) this launch computes
+    uint32_t B, H, W, Cin;
+    uint32_t N, nSplit;       // output channels of one work item (a multiple of 16, <= 256); items per tile
+    uint32_t tilesX, tilesY;  // 8 x 16 pixel tiles (the last row of tiles may overhang the image)
+    uint32_t stagesA, stagesB;  // ring slots: halo chunks, weight slices
+    uint32_t stagingBytes;      // one staged output slice (the epilogue warps' 4 x 32 pixels)
+    uint32_t tmemCols;
 };
 
-// What the forward kernel does with the accumulator of output channel co < coutValid:
-// (+ bias[co]) -> (ReLU) -> (x 0 where mask <= 0) -> store to out[pixel*outStride + outOffset + co]
-// as bf16 or f32 (f32 may accumulate into what is there).
+// What the forward kernel does with the accumulator of output channel co:
+// (+ bias[co]) -> (ReLU) -> (x 0 where mask <= 0) -> store.  nOut > 0: by TMA through the
+// launch's output maps (bf16 or f32; four maps = the 2x nearest upsample), and the 2x2
+// average of the stored bf16 values into `pool` when it is set.  nOut = 0: the cropped
+// output image when headDst is set, else element stores to
+// out[pixel*outStride + outOffset + co] for co < coutValid.
 struct Epilogue {
-    const float* bias;  // bias[co] added for co < nBias
+    const float* bias;  // bias[co] added for co < nBias (f32, at most 256 channels)
     uint32_t nBias;
+    uint32_t nOut;
     void* out;
     uint32_t outStride, outOffset, coutValid;
-    uint32_t relu, outF32, accumulate;
+    uint32_t relu, outF32;
     const __nv_bfloat16* mask;
     uint32_t maskStride, maskOffset;
+    __nv_bfloat16* pool;  // [B][H/2][W/2][poolStride]
+    uint32_t poolStride;
+    const float* headRgb;  // [B][headH][headW][3]
+    float* headDst;
+    uint32_t headH, headW;
 };
 
 struct WgradShape {
@@ -37,11 +48,16 @@ struct WgradShape {
     uint32_t stages, tmemCols;
 };
 
+// Output tensor maps of a forward launch: one, or one per child pixel of an upsample.
+struct OutMaps {
+    CUtensorMap m[4];
+};
 struct FwdPlan {
     FwdShape shape;
-    int chunk;
+    int chunk;        // input channels per halo chunk
+    uint32_t sliceC;  // output channels per staged slice
     uint32_t smem, grid;
-    bool halo;  // small-N kernel: resident weights, one halo load per 8 x 16 tile
+    bool resident;    // the whole weight tensor stays in shared memory
 };
 struct WgradPlan {
     WgradShape shape;
@@ -50,17 +66,18 @@ struct WgradPlan {
 };
 
 int chunk_for(uint32_t channels);
-// Tensor maps: activations NHWC bf16 (box = boxC channels x 16 x 8 pixels); weights
-// as a 2-D [rows][K] bf16 matrix (box = boxK x boxRows).  Return 0 on success.
+// Activation map for the weight gradient: NHWC bf16, box = boxC channels x 16 x 8 pixels.
+// All map functions return 0 on success.
 int make_act_map(CUtensorMap* m, const void* base, uint32_t C, uint32_t W, uint32_t H, uint32_t B, uint32_t boxC);
-int make_weight_map(CUtensorMap* m, const void* base, uint32_t K, uint32_t rows, uint32_t boxK, uint32_t boxRows);
-int plan_fwd(uint32_t B, uint32_t H, uint32_t W, uint32_t Cin, uint32_t N, uint32_t numSMs, FwdPlan* p);
+int plan_fwd(uint32_t B, uint32_t H, uint32_t W, uint32_t Cin, uint32_t N, bool outF32, uint32_t numSMs, FwdPlan* p);
 int plan_wgrad(uint32_t B, uint32_t H, uint32_t W, uint32_t Cin, uint32_t Cout, uint32_t numSMs, WgradPlan* p);
-// Input tensor map for a forward plan (tiled or halo boxes); 0 on success.  The halo
-// kernel reads the weights straight from memory: its `mw` is not used, so only the
-// tiled kernel needs make_weight_map.
+// Tensor maps of a forward plan: the input, the weights [N * nSplit][9 * Cin] bf16, and
+// the output (channel `offset` on of a buffer `stride` channels wide; up = the 2x nearest
+// upsample of the output, whose buffer is 2W x 2H).
 int make_input_map(const FwdPlan& p, const void* x, CUtensorMap* mx);
-cudaError_t launch_fwd(const FwdPlan& p, const CUtensorMap& mx, const CUtensorMap& mw, const void* w,
+int make_weight_map(const FwdPlan& p, const void* w, CUtensorMap* mw);
+int make_out_maps(const FwdPlan& p, void* out, uint32_t stride, uint32_t offset, bool f32, bool up, OutMaps* mo);
+cudaError_t launch_fwd(const FwdPlan& p, const CUtensorMap& mx, const CUtensorMap& mw, const OutMaps& mo,
                        const Epilogue& ep, uint32_t* err, cudaStream_t st);
 cudaError_t launch_wgrad(const WgradPlan& p, const CUtensorMap& mg, const CUtensorMap& mx, float* dW, uint32_t* err,
                          cudaStream_t st);

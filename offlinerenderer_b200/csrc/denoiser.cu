@@ -12,11 +12,12 @@
 //
 // Activations NHWC bf16.  Buffers per level l (resolution H/2^l):
 //   x0[16] a0[32] cat0[96] a6[32] dec0[32] out[16 f32]       level 0
-//   p1[32] a1[64] cat1[192] a5[64] dec1[64]                   level 1
-//   p2[64] a2[128] cat2[384] a4[128] dec2[128]                level 2
-//   p3[128] a3[256] b3[256]                                   level 3
+//   p1[32] a1[64] cat1[192] a5[64]                            level 1
+//   p2[64] a2[128] cat2[384] a4[128]                          level 2
+//   p3[128] a3[256]                                           level 3
 // cat_l = [up(deeper) | skip s_l]; the encoder's second convolution writes s_l
-// straight into its slice of cat_l, the upsample writes the other slice.
+// straight into its slice of cat_l (and pools it into p_{l+1}), the layer below the
+// upsample writes each output to its four pixels of the other slice.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -99,45 +100,10 @@ __device__ __forceinline__ uint4 f_to_bf8(const float (&f)[8]) {
     return u;
 }
 
-// 2x2 average pool: src [B][H][W][stride] channels [off, off+C) -> dst [B][H/2][W/2][C]
-__global__ void k_pool2(const __nv_bfloat16* src, uint32_t stride, uint32_t off, uint32_t C, uint32_t B, uint32_t H,
-                        uint32_t W, __nv_bfloat16* dst) {
-    const uint32_t g = C / 8, h = H / 2, w = W / 2;
-    size_t n = (size_t)B * h * w * g;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        uint32_t cg = (uint32_t)(i % g);
-        size_t p = i / g;
-        uint32_t x = (uint32_t)(p % w), y = (uint32_t)((p / w) % h), b = (uint32_t)(p / ((size_t)w * h));
-        float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-        for (int dy = 0; dy < 2; ++dy)
-            for (int dx = 0; dx < 2; ++dx) {
-                size_t sp = ((size_t)b * H + 2 * y + dy) * W + 2 * x + dx;
-                float f[8];
-                bf8_to_f(*(const uint4*)(src + sp * stride + off + cg * 8), f);
-                for (int j = 0; j < 8; ++j) acc[j] += f[j];
-            }
-        for (int j = 0; j < 8; ++j) acc[j] *= 0.25f;
-        *(uint4*)(dst + p * C + cg * 8) = f_to_bf8(acc);
-    }
-}
-
-// nearest 2x upsample: src [B][h][w][C] -> dst [B][2h][2w][stride] channels [0, C)
-__global__ void k_up2(const __nv_bfloat16* src, uint32_t C, uint32_t B, uint32_t h, uint32_t w, __nv_bfloat16* dst,
-                      uint32_t stride) {
-    const uint32_t g = C / 8, H = 2 * h, W = 2 * w;
-    size_t n = (size_t)B * H * W * g;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        uint32_t cg = (uint32_t)(i % g);
-        size_t p = i / g;
-        uint32_t x = (uint32_t)(p % W), y = (uint32_t)((p / W) % H), b = (uint32_t)(p / ((size_t)W * H));
-        size_t sp = ((size_t)b * h + y / 2) * w + x / 2;
-        *(uint4*)(dst + p * stride + cg * 8) = *(const uint4*)(src + sp * C + cg * 8);
-    }
-}
-
-// gradient of the upsample: g[B][h][w][C] = sum of the 4 children of dcat[.., 0:C), x (mask > 0)
+// gradient of the upsample: g[B][h][w][C] = sum of the 4 children of dcat[.., 0:C), x (the
+// upsampled activation, in cat, > 0)
 __global__ void k_up2_bwd(const float* dcat, uint32_t stride, uint32_t C, uint32_t B, uint32_t h, uint32_t w,
-                          const __nv_bfloat16* mask, __nv_bfloat16* g) {
+                          const __nv_bfloat16* cat, __nv_bfloat16* g) {
     const uint32_t G = C / 8, H = 2 * h, W = 2 * w;
     size_t n = (size_t)B * h * w * G;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
@@ -153,7 +119,7 @@ __global__ void k_up2_bwd(const float* dcat, uint32_t stride, uint32_t C, uint32
                 acc[4] += v.x; acc[5] += v.y; acc[6] += v.z; acc[7] += v.w;
             }
         float m[8];
-        bf8_to_f(*(const uint4*)(mask + p * C + cg * 8), m);
+        bf8_to_f(*(const uint4*)(cat + (((size_t)b * H + 2 * y) * W + 2 * x) * stride + cg * 8), m);
         for (int j = 0; j < 8; ++j)
             if (!(m[j] > 0.0f)) acc[j] = 0.0f;
         *(uint4*)(g + p * C + cg * 8) = f_to_bf8(acc);
@@ -217,18 +183,6 @@ __global__ void k_loss(const float* out, const float* rgb, const float* target, 
     }
     for (int s = 16; s > 0; s >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, s);
     if ((threadIdx.x & 31) == 0) atomicAdd(lossSum, acc);
-}
-
-// denoised radiance = expm1(log1p(rgb) + head), cropped to [B][h][w][3]
-__global__ void k_unpack(const float* out, const float* rgb, uint32_t B, uint32_t h, uint32_t w, uint32_t H,
-                         uint32_t W, float* dst) {
-    size_t n = (size_t)B * h * w;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        uint32_t b = (uint32_t)(i / ((size_t)h * w)), r = (uint32_t)(i % ((size_t)h * w));
-        uint32_t y = r / w, x = r % w;
-        size_t q = ((size_t)b * H + y) * W + x;
-        for (int c = 0; c < 3; ++c) dst[3 * i + c] = fmaxf(expm1f(lg(rgb[3 * i + c]) + out[16 * q + c]), 0.0f);
-    }
 }
 
 // Adam (Kingma & Ba 2015) on the flat f32 parameter array.
@@ -316,14 +270,13 @@ struct wrk_denoiser {
     // activations / gradients for the current shape
     uint32_t B = 0, H = 0, W = 0;
     DBuf x0, a[kLayers], cat[3], pool[3], out, g[kLayers], dcat[3], dp[3];
-    DBuf inPad, scratchIn[3];
-    bool shapeReady = false;
+    bool shapeReady = false, trainReady = false;  // plans of the forward / backward pass for this shape
     // plans and tensor maps for the current shape
     conv::FwdPlan fplan[kLayers];
-    conv::FwdPlan dplan[kLayers][2];
+    conv::FwdPlan dplan[kLayers];
     conv::WgradPlan wplan[kLayers];
-    CUtensorMap fin[kLayers], fw[kLayers], din[kLayers], dwmap[kLayers][2], wg[kLayers], wx[kLayers];
-    uint32_t dsplit[kLayers];
+    CUtensorMap fin[kLayers], fw[kLayers], din[kLayers], dwmap[kLayers], wg[kLayers], wx[kLayers];
+    conv::OutMaps fout[kLayers], dout[kLayers];
     // device time of the last inference / training step (events on `stream`)
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     float lastMs = 0.0f;
@@ -339,31 +292,33 @@ namespace {
 uint32_t lvl_h(const wrk_denoiser* d, uint32_t l) { return d->H >> l; }
 uint32_t lvl_w(const wrk_denoiser* d, uint32_t l) { return d->W >> l; }
 
-// Input tensor (buffer, channels) of layer i, and where its output goes.
+// Input tensor (buffer, channels) of layer i, where its output goes, and whether the
+// output is upsampled on the way there.
 struct IO {
     void* in;
     uint32_t inC;
     void* out;
     uint32_t outStride, outOffset;
+    bool up;
 };
 IO layer_io(wrk_denoiser* d, int i) {
     auto A = [&](int k) { return d->a[k].p; };
     switch (i) {
-        case 0: return {d->x0.p, 16, A(0), 32, 0};
-        case 1: return {A(0), 32, d->cat[0].p, 96, 64};
-        case 2: return {d->pool[0].p, 32, A(2), 64, 0};
-        case 3: return {A(2), 64, d->cat[1].p, 192, 128};
-        case 4: return {d->pool[1].p, 64, A(4), 128, 0};
-        case 5: return {A(4), 128, d->cat[2].p, 384, 256};
-        case 6: return {d->pool[2].p, 128, A(6), 256, 0};
-        case 7: return {A(6), 256, A(7), 256, 0};
-        case 8: return {d->cat[2].p, 384, A(8), 128, 0};
-        case 9: return {A(8), 128, A(9), 128, 0};
-        case 10: return {d->cat[1].p, 192, A(10), 64, 0};
-        case 11: return {A(10), 64, A(11), 64, 0};
-        case 12: return {d->cat[0].p, 96, A(12), 32, 0};
-        case 13: return {A(12), 32, A(13), 32, 0};
-        default: return {A(13), 32, d->out.p, 16, 0};
+        case 0: return {d->x0.p, 16, A(0), 32, 0, false};
+        case 1: return {A(0), 32, d->cat[0].p, 96, 64, false};
+        case 2: return {d->pool[0].p, 32, A(2), 64, 0, false};
+        case 3: return {A(2), 64, d->cat[1].p, 192, 128, false};
+        case 4: return {d->pool[1].p, 64, A(4), 128, 0, false};
+        case 5: return {A(4), 128, d->cat[2].p, 384, 256, false};
+        case 6: return {d->pool[2].p, 128, A(6), 256, 0, false};
+        case 7: return {A(6), 256, d->cat[2].p, 384, 0, true};
+        case 8: return {d->cat[2].p, 384, A(8), 128, 0, false};
+        case 9: return {A(8), 128, d->cat[1].p, 192, 0, true};
+        case 10: return {d->cat[1].p, 192, A(10), 64, 0, false};
+        case 11: return {A(10), 64, d->cat[0].p, 96, 0, true};
+        case 12: return {d->cat[0].p, 96, A(12), 32, 0, false};
+        case 13: return {A(12), 32, A(13), 32, 0, false};
+        default: return {A(13), 32, d->out.p, 16, 0, false};
     }
 }
 
@@ -415,36 +370,62 @@ int relayout_all(wrk_denoiser* d) {
     return WRK_OK;
 }
 
-// Buffers, launch plans and tensor maps for batch B at H x W (multiples of 128 x 64).
-int set_shape(wrk_denoiser* d, uint32_t B, uint32_t H, uint32_t W) {
-    if (d->shapeReady && d->B == B && d->H == H && d->W == W) return WRK_OK;
+// Where the data gradient of layer i > 0 goes: the G of the layer below (bf16, masked), or
+// an f32 buffer that the combine kernels split (concatenated and pooled inputs).
+void* dgrad_out(wrk_denoiser* d, int i, bool* f32) {
+    *f32 = true;
+    switch (i) {
+        case 12: return d->dcat[0].p;
+        case 10: return d->dcat[1].p;
+        case 8: return d->dcat[2].p;
+        case 6: return d->dp[2].p;
+        case 4: return d->dp[1].p;
+        case 2: return d->dp[0].p;
+        default: *f32 = false; return d->g[i - 1].p;
+    }
+}
+
+// Buffers, launch plans and tensor maps for batch B at H x W (multiples of 128 x 64); those
+// of the backward pass only once it is asked for.
+int set_shape(wrk_denoiser* d, uint32_t B, uint32_t H, uint32_t W, bool train) {
+    const bool same = d->shapeReady && d->B == B && d->H == H && d->W == W;
+    if (same && (d->trainReady || !train)) return WRK_OK;
     if (B == 0 || H % 64 || W % 128) return dfail(WRK_ERR_INVALID, "denoiser shape %ux%u not a multiple of 128x64", W, H);
-    d->shapeReady = false;
-    d->B = B;
-    d->H = H;
-    d->W = W;
-    auto px = [&](uint32_t l) { return (size_t)B * lvl_h(d, l) * lvl_w(d, l); };
-    bool bad = d->x0.alloc(px(0) * 16 * 2) || d->out.alloc(px(0) * 16 * 4);
     const uint32_t catC[3] = {96, 192, 384}, poolC[3] = {32, 64, 128};
-    for (int l = 0; l < 3; ++l) {
-        bad = bad || d->cat[l].alloc(px(l) * catC[l] * 2) || d->dcat[l].alloc(px(l) * catC[l] * 4) ||
-              d->pool[l].alloc(px(l + 1) * poolC[l] * 2) || d->dp[l].alloc(px(l + 1) * poolC[l] * 4);
+    auto px = [&](uint32_t l) { return (size_t)B * lvl_h(d, l) * lvl_w(d, l); };
+    if (!same) {
+        d->shapeReady = d->trainReady = false;
+        d->B = B;
+        d->H = H;
+        d->W = W;
+        bool bad = d->x0.alloc(px(0) * 16 * 2) || d->out.alloc(px(0) * 16 * 4);
+        for (int l = 0; l < 3; ++l)
+            bad = bad || d->cat[l].alloc(px(l) * catC[l] * 2) || d->pool[l].alloc(px(l + 1) * poolC[l] * 2);
+        for (int i : {0, 2, 4, 6, 8, 10, 12, 13}) bad = bad || d->a[i].alloc(px(kDefs[i].level) * kDefs[i].cout * 2);
+        if (bad) return dfail(WRK_ERR_CUDA, "denoiser activation allocation failed (%ux%u x %u)", W, H, B);
+        for (int i = 0; i < kLayers; ++i) {
+            const LayerDef& L = kDefs[i];
+            IO io = layer_io(d, i);
+            const bool head = i == kLayers - 1;
+            if (conv::plan_fwd(B, lvl_h(d, L.level), lvl_w(d, L.level), L.cin, pad16(L.cout), head, d->numSMs, &d->fplan[i]))
+                return dfail(WRK_ERR_INVALID, "no forward plan for layer %d", i);
+            if (conv::make_input_map(d->fplan[i], io.in, &d->fin[i]) ||
+                conv::make_weight_map(d->fplan[i], d->wf[i].p, &d->fw[i]) ||
+                conv::make_out_maps(d->fplan[i], io.out, io.outStride, io.outOffset, head, io.up, &d->fout[i]))
+                return dfail(WRK_ERR_CUDA, "tensor map encoding failed (layer %d)", i);
+        }
+        d->shapeReady = true;
     }
-    for (int i = 0; i < kLayers; ++i) {
-        const LayerDef& L = kDefs[i];
-        bad = bad || d->a[i].alloc(px(L.level) * pad16(L.cout) * 2) || d->g[i].alloc(px(L.level) * pad16(L.cout) * 2);
-    }
+    if (!train) return WRK_OK;
+    bool bad = false;
+    for (int l = 0; l < 3; ++l)
+        bad = bad || d->dcat[l].alloc(px(l) * catC[l] * 4) || d->dp[l].alloc(px(l + 1) * poolC[l] * 4);
+    for (int i = 0; i < kLayers; ++i) bad = bad || d->g[i].alloc(px(kDefs[i].level) * pad16(kDefs[i].cout) * 2);
     if (bad) return dfail(WRK_ERR_CUDA, "denoiser activation allocation failed (%ux%u x %u)", W, H, B);
     for (int i = 0; i < kLayers; ++i) {
         const LayerDef& L = kDefs[i];
         const uint32_t h = lvl_h(d, L.level), w = lvl_w(d, L.level), coPad = pad16(L.cout);
         IO io = layer_io(d, i);
-        if (conv::plan_fwd(B, h, w, L.cin, coPad, d->numSMs, &d->fplan[i]))
-            return dfail(WRK_ERR_INVALID, "no forward plan for layer %d", i);
-        int ch = d->fplan[i].chunk;
-        if (conv::make_input_map(d->fplan[i], io.in, &d->fin[i]) ||
-            (!d->fplan[i].halo && conv::make_weight_map(&d->fw[i], d->wf[i].p, 9 * L.cin, coPad, ch, coPad)))
-            return dfail(WRK_ERR_CUDA, "tensor map encoding failed (layer %d)", i);
         // weight gradient: G = g[i] (coPad channels), X = layer input
         if (conv::plan_wgrad(B, h, w, L.cin, coPad, d->numSMs, &d->wplan[i]))
             return dfail(WRK_ERR_INVALID, "no weight-gradient plan for layer %d", i);
@@ -454,63 +435,47 @@ int set_shape(wrk_denoiser* d, uint32_t B, uint32_t H, uint32_t W) {
             return dfail(WRK_ERR_CUDA, "tensor map encoding failed (layer %d wgrad)", i);
         // data gradient: input g[i] (coPad), weights Wd [cin][9][coPad], output cin channels
         if (i > 0) {
-            d->dsplit[i] = L.cin > 256 ? 2 : 1;
-            uint32_t n = L.cin / d->dsplit[i];
-            for (uint32_t s = 0; s < d->dsplit[i]; ++s) {
-                if (conv::plan_fwd(B, h, w, coPad, n, d->numSMs, &d->dplan[i][s]))
-                    return dfail(WRK_ERR_INVALID, "no data-gradient plan for layer %d", i);
-                d->dplan[i][s].shape.wRow0 = s * n;
-                int dc = d->dplan[i][s].chunk;
-                if (!d->dplan[i][s].halo && conv::make_weight_map(&d->dwmap[i][s], d->wd[i].p, 9 * coPad, L.cin, dc, n))
-                    return dfail(WRK_ERR_CUDA, "tensor map encoding failed (layer %d dgrad)", i);
-            }
-            if (conv::make_input_map(d->dplan[i][0], d->g[i].p, &d->din[i]))
-                return dfail(WRK_ERR_CUDA, "tensor map encoding failed (layer %d dgrad input)", i);
+            bool f32 = false;
+            void* dst = dgrad_out(d, i, &f32);
+            if (conv::plan_fwd(B, h, w, coPad, L.cin, f32, d->numSMs, &d->dplan[i]))
+                return dfail(WRK_ERR_INVALID, "no data-gradient plan for layer %d", i);
+            if (conv::make_input_map(d->dplan[i], d->g[i].p, &d->din[i]) ||
+                conv::make_weight_map(d->dplan[i], d->wd[i].p, &d->dwmap[i]) ||
+                conv::make_out_maps(d->dplan[i], dst, L.cin, 0, f32, false, &d->dout[i]))
+                return dfail(WRK_ERR_CUDA, "tensor map encoding failed (layer %d dgrad)", i);
         }
     }
-    d->shapeReady = true;
+    d->trainReady = true;
     return WRK_OK;
 }
 
-int conv_forward(wrk_denoiser* d, int i) {
-    const LayerDef& L = kDefs[i];
-    IO io = layer_io(d, i);
-    Epilogue ep{};
-    ep.bias = d->params.as<float>() + d->boff[i];
-    ep.nBias = L.cout;
-    ep.out = io.out;
-    ep.outStride = io.outStride;
-    ep.outOffset = io.outOffset;
-    ep.coutValid = i == kLayers - 1 ? 16u : L.cout;  // head: padded channels are written as zero
-    ep.relu = L.relu;
-    ep.outF32 = i == kLayers - 1;
-    DCK(conv::launch_fwd(d->fplan[i], d->fin[i], d->fw[i], d->wf[i].p, ep, d->err.as<uint32_t>(), d->stream));
-    return WRK_OK;
-}
-
-int forward(wrk_denoiser* d) {
-    const uint32_t B = d->B;
-    int rc;
+// The forward pass on x0.  dst (with rgb, h, w): the last layer writes the denoised image
+// there, cropped; otherwise its residual goes to d->out (f32, 16 channels).
+int forward(wrk_denoiser* d, const float* rgb, uint32_t h, uint32_t w, float* dst) {
     for (int i = 0; i < kLayers; ++i) {
-        if ((rc = conv_forward(d, i))) return rc;
-        // pool after each encoder level's second convolution
-        if (i == 1 || i == 3 || i == 5) {
-            int l = (i - 1) / 2;
-            const uint32_t catC[3] = {96, 192, 384}, off[3] = {64, 128, 256}, C[3] = {32, 64, 128};
-            size_t n = (size_t)B * lvl_h(d, l + 1) * lvl_w(d, l + 1) * C[l] / 8;
-            k_pool2<<<grid_for(n), 256, 0, d->stream>>>(d->cat[l].as<__nv_bfloat16>(), catC[l], off[l], C[l], B,
-                                                        lvl_h(d, l), lvl_w(d, l), d->pool[l].as<__nv_bfloat16>());
+        const LayerDef& L = kDefs[i];
+        IO io = layer_io(d, i);
+        const bool head = i == kLayers - 1;
+        Epilogue ep{};
+        ep.bias = d->params.as<float>() + d->boff[i];
+        ep.nBias = L.cout;
+        ep.nOut = io.up ? 4 : 1;
+        ep.outF32 = head;
+        ep.relu = L.relu;
+        if (i == 1 || i == 3 || i == 5) {  // the encoder levels' second convolutions are pooled
+            ep.pool = d->pool[i / 2].as<__nv_bfloat16>();
+            ep.poolStride = L.cout;
         }
-        // upsample into the decoder's concat buffer before its first convolution
-        if (i == 7 || i == 9 || i == 11) {
-            int l = i == 7 ? 2 : i == 9 ? 1 : 0;
-            const uint32_t C[3] = {64, 128, 256}, catC[3] = {96, 192, 384};
-            size_t n = (size_t)B * lvl_h(d, l) * lvl_w(d, l) * C[l] / 8;
-            k_up2<<<grid_for(n), 256, 0, d->stream>>>(d->a[i].as<__nv_bfloat16>(), C[l], B, lvl_h(d, l + 1),
-                                                      lvl_w(d, l + 1), d->cat[l].as<__nv_bfloat16>(), catC[l]);
+        if (head && dst) {
+            ep.nOut = 0;
+            ep.coutValid = L.cout;
+            ep.headRgb = rgb;
+            ep.headDst = dst;
+            ep.headH = h;
+            ep.headW = w;
         }
+        DCK(conv::launch_fwd(d->fplan[i], d->fin[i], d->fw[i], d->fout[i], ep, d->err.as<uint32_t>(), d->stream));
     }
-    DCK(cudaGetLastError());
     return WRK_OK;
 }
 
@@ -550,39 +515,14 @@ int backward(wrk_denoiser* d) {
         }
         if (i == 0) break;
         // data gradient into the layer's input
-        const void* mask = input_mask(d, i);
-        const uint32_t targetLayer = (uint32_t)i - 1;  // the G it produces (when masked)
-        for (uint32_t s = 0; s < d->dsplit[i]; ++s) {
+        {
             Epilogue ep{};
-            uint32_t n = L.cin / d->dsplit[i];
-            ep.coutValid = n;
-            ep.relu = 0;
-            if (mask) {
-                ep.out = d->g[targetLayer].p;
-                ep.outStride = L.cin;
-                ep.outOffset = s * n;
-                ep.outF32 = 0;
-                ep.mask = (const __nv_bfloat16*)mask;
-                ep.maskStride = L.cin;
-                ep.maskOffset = s * n;
-            } else {
-                // concat or pooled input: f32 gradient, split by the combine kernels
-                void* dst = nullptr;
-                switch (i) {
-                    case 12: dst = d->dcat[0].p; break;
-                    case 10: dst = d->dcat[1].p; break;
-                    case 8: dst = d->dcat[2].p; break;
-                    case 6: dst = d->dp[2].p; break;
-                    case 4: dst = d->dp[1].p; break;
-                    case 2: dst = d->dp[0].p; break;
-                }
-                ep.out = dst;
-                ep.outStride = L.cin;
-                ep.outOffset = s * n;
-                ep.outF32 = 1;
-            }
-            DCK(conv::launch_fwd(d->dplan[i][s], d->din[i], d->dwmap[i][s], d->wd[i].p, ep, d->err.as<uint32_t>(),
-                                 d->stream));
+            const void* mask = input_mask(d, i);
+            ep.nOut = 1;
+            ep.outF32 = mask ? 0 : 1;
+            ep.mask = (const __nv_bfloat16*)mask;
+            ep.maskStride = L.cin;
+            DCK(conv::launch_fwd(d->dplan[i], d->din[i], d->dwmap[i], d->dout[i], ep, d->err.as<uint32_t>(), d->stream));
         }
         // combine kernels that produce the G of the layer below
         const uint32_t catC[3] = {96, 192, 384};
@@ -592,7 +532,7 @@ int backward(wrk_denoiser* d) {
             const uint32_t C[3] = {64, 128, 256};
             size_t n = (size_t)B * lvl_h(d, l + 1) * lvl_w(d, l + 1) * C[l] / 8;
             k_up2_bwd<<<grid_for(n), 256, 0, d->stream>>>(d->dcat[l].as<float>(), catC[l], C[l], B, lvl_h(d, l + 1),
-                                                          lvl_w(d, l + 1), d->a[below].as<__nv_bfloat16>(),
+                                                          lvl_w(d, l + 1), d->cat[l].as<__nv_bfloat16>(),
                                                           d->g[below].as<__nv_bfloat16>());
         }
         if (i == 6 || i == 4 || i == 2) {  // pooled input -> G of the skip tensor s_l (layer i-1)
@@ -639,12 +579,12 @@ int fwd_bwd(wrk_denoiser* d, const float* rgb, const float* alb, const float* nr
             uint32_t H, uint32_t W, float* loss) {
     if (!d || !rgb || !target) return dfail(WRK_ERR_INVALID, "null denoiser argument");
     DCK(cudaSetDevice(d->device));
-    int rc = set_shape(d, B, H, W);
+    int rc = set_shape(d, B, H, W, true);
     if (rc) return rc;
     DCK(cudaMemsetAsync(d->err.p, 0, 4, d->stream));
     size_t P = (size_t)B * H * W;
     k_pack<<<grid_for(P), 256, 0, d->stream>>>(rgb, alb, nrm, B, H, W, H, W, d->x0.as<__nv_bfloat16>());
-    if ((rc = forward(d)) || (rc = run_loss(d, rgb, target, nullptr)) || (rc = backward(d))) return rc;
+    if ((rc = forward(d, nullptr, 0, 0, nullptr)) || (rc = run_loss(d, rgb, target, nullptr)) || (rc = backward(d))) return rc;
     if (loss) {
         float s = 0;
         DCK(cudaMemcpyAsync(&s, d->lossSum.p, 4, cudaMemcpyDeviceToHost, d->stream));
@@ -690,11 +630,11 @@ int wrk_conv3x3_forward(const void* x, uint32_t B, uint32_t H, uint32_t W, uint3
     if (err.alloc(4)) return dfail(WRK_ERR_CUDA, "allocation failed");
     DCK(cudaMemset(err.p, 0, 4));
     conv::FwdPlan plan;
-    if (conv::plan_fwd(B, H, W, Cin, N, (uint32_t)sms, &plan)) return dfail(WRK_ERR_INVALID, "no conv plan");
+    const bool f32 = (flags >> 1) & 1u;
+    if (conv::plan_fwd(B, H, W, Cin, N, f32, (uint32_t)sms, &plan)) return dfail(WRK_ERR_INVALID, "no conv plan");
     CUtensorMap mx, mw;
-    memset(&mw, 0, sizeof(mw));
-    if (conv::make_input_map(plan, x, &mx) ||
-        (!plan.halo && conv::make_weight_map(&mw, wp, 9 * Cin, N, plan.chunk, N)))
+    conv::OutMaps mo{};
+    if (conv::make_input_map(plan, x, &mx) || conv::make_weight_map(plan, wp, &mw))
         return dfail(WRK_ERR_CUDA, "tensor map encoding failed (pointers must be 16-byte aligned)");
     Epilogue ep{};
     ep.bias = bias;
@@ -703,8 +643,10 @@ int wrk_conv3x3_forward(const void* x, uint32_t B, uint32_t H, uint32_t W, uint3
     ep.outStride = Cout;
     ep.coutValid = Cout;
     ep.relu = flags & 1u;
-    ep.outF32 = (flags >> 1) & 1u;
-    DCK(conv::launch_fwd(plan, mx, mw, wp, ep, err.as<uint32_t>(), 0));
+    ep.outF32 = f32;
+    // whole 16-byte rows leave by TMA; a padded Cout or an unaligned output by element stores
+    if (N == Cout && conv::make_out_maps(plan, out, Cout, 0, f32, false, &mo) == 0) ep.nOut = 1;
+    DCK(conv::launch_fwd(plan, mx, mw, mo, ep, err.as<uint32_t>(), 0));
     uint32_t e = 0;
     DCK(cudaMemcpy(&e, err.p, 4, cudaMemcpyDeviceToHost));
     if (e) return dfail(WRK_ERR_DEVICE, "conv kernel timed out (flags 0x%x)", e);
@@ -878,14 +820,13 @@ int wrk_denoiser_infer(wrk_denoiser* d, const float* rgb, const float* alb, cons
     if (!d || !rgb || !out || B == 0 || H == 0 || W == 0) return dfail(WRK_ERR_INVALID, "bad denoiser arguments");
     DCK(cudaSetDevice(d->device));
     const uint32_t Hp = (H + 63) / 64 * 64, Wp = (W + 127) / 128 * 128;
-    int rc = set_shape(d, B, Hp, Wp);
+    int rc = set_shape(d, B, Hp, Wp, false);
     if (rc) return rc;
     DCK(cudaMemsetAsync(d->err.p, 0, 4, d->stream));
     DCK(cudaEventRecord(d->ev0, d->stream));
     size_t P = (size_t)B * Hp * Wp;
     k_pack<<<grid_for(P), 256, 0, d->stream>>>(rgb, alb, nrm, B, H, W, Hp, Wp, d->x0.as<__nv_bfloat16>());
-    if ((rc = forward(d))) return rc;
-    k_unpack<<<grid_for((size_t)B * H * W), 256, 0, d->stream>>>(d->out.as<float>(), rgb, B, H, W, Hp, Wp, out);
+    if ((rc = forward(d, rgb, H, W, out))) return rc;
     DCK(cudaGetLastError());
     DCK(cudaEventRecord(d->ev1, d->stream));
     rc = check_err(d, "denoiser inference");
