@@ -12,6 +12,33 @@
 
 namespace wrk {
 
+// Packed FP32 pairs (sm_100's two-wide FMA pipe instructions): one issue slot for two
+// independent, correctly rounded operations.  A mul2 whose result only add2 reads may be
+// contracted into one rounding by ptxas, whatever --fmad says: where the two roundings
+// matter, use scalars.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float a, float b) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
 // float pi: sampling.cuh:6-8 / material_common.cuh:9 (both the same float).
 constexpr float kPi = 3.14159265358979323846f;
 
@@ -288,6 +315,55 @@ __device__ __forceinline__ uint8_t aces_byte(float lin) {
     float g = 1.0f / 2.2f;
     float p = (float)pow((double)v, (double)g);
     return (uint8_t)(p * 255.0f);
+}
+// The same byte from the hardware's approximate reciprocal, log2 and exp2 (relative errors
+// of about 2^-22 each: together below 1.3e-4 of a byte step over the curve).  `sure` is
+// cleared within 5e-4 of a step between bytes, and for the inputs whose curve value is
+// not an ordinary quotient (negative, huge or NaN radiance): aces_byte decides those.
+// Two values at a time.
+__device__ __forceinline__ void aces_bytes_fast(float lin0, float lin1, uint32_t& b0, uint32_t& b1, bool& sure0,
+                                                bool& sure1) {
+    constexpr float kEps = 5e-4f, kTwo23 = 8388608.0f;
+    auto both = [](float c) { return pack2(c, c); };
+    const float xs[2] = {lin0 * 2.2f, lin1 * 2.2f};
+    float num[2], den[2], q[2], t[2], f[2];
+    // (scalar: ptxas contracts a packed product and sum into one rounding)
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        num[k] = xs[k] * (2.51f * xs[k] + 0.03f);
+        den[k] = xs[k] * (2.43f * xs[k] + 0.59f) + 0.14f;
+    }
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        float r, l;
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(den[k]));
+        asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(l) : "f"(num[k] * r));
+        asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(q[k]) : "f"(l * (1.0f / 2.2f)));
+    }
+    const f32x2 q2 = mul2(pack2(q[0], q[1]), both(255.0f));
+    unpack2(q2, q[0], q[1]);
+    t[0] = __fadd_rd(q[0], kTwo23);  // floor(q) in the low mantissa bits
+    t[1] = __fadd_rd(q[1], kTwo23);
+    unpack2(add2(q2, mul2(add2(pack2(t[0], t[1]), both(-kTwo23)), both(-1.0f))), f[0], f[1]);
+    const bool one0 = num[0] >= den[0], one1 = num[1] >= den[1];  // the quotient is at least 1
+    sure0 = xs[0] >= 0.0f && num[0] < 3.0e38f && (one0 || ((f[0] >= kEps || q[0] < 1.0f) && f[0] <= 1.0f - kEps));
+    sure1 = xs[1] >= 0.0f && num[1] < 3.0e38f && (one1 || ((f[1] >= kEps || q[1] < 1.0f) && f[1] <= 1.0f - kEps));
+    b0 = one0 ? 255u : __float_as_uint(t[0]) & 0xffu;
+    b1 = one1 ? 255u : __float_as_uint(t[1]) & 0xffu;
+}
+__device__ __forceinline__ uchar4 aces_bytes4(float4 v) {
+    bool s0, s1, s2, s3;
+    uint32_t b0, b1, b2, b3;
+    aces_bytes_fast(v.x, v.y, b0, b1, s0, s1);
+    aces_bytes_fast(v.z, v.w, b2, b3, s2, s3);
+    uchar4 b = make_uchar4(b0, b1, b2, b3);
+    if (!(s0 && s1 && s2 && s3)) {
+        if (!s0) b.x = aces_byte(v.x);
+        if (!s1) b.y = aces_byte(v.y);
+        if (!s2) b.z = aces_byte(v.z);
+        if (!s3) b.w = aces_byte(v.w);
+    }
+    return b;
 }
 
 }  // namespace wrk
