@@ -778,8 +778,49 @@ void fill_frame(Frame& f, const wrk_camera& cam, const wrk_render_params& p) {
 
 extern "C" {
 
+// The statistics of a finished render, from the counters read back and the events.
+static void fill_stats(wrk_renderer* r, uint32_t iters, const float* stageMs, const uint32_t* stageN,
+                       wrk_render_stats* stats) {
+    if (!stats) return;
+    const Counters& h = *r->eng.hCtr;
+    stats->paths = h.paths;
+    stats->extensionRays = h.extRays;
+    stats->shadowRays = h.shdRays + h.shadowAnswered.v;  // + the last iteration's answered queries
+    stats->shadowTraced = h.shdTraced;
+    for (int b = 0; b < kNumBuckets; ++b) stats->bucketPaths[b] = h.bucketTotal[b] + h.bucket[b].v;
+    stats->bucketPaths[kBucketLambert] += h.lambertTex.v;
+    stats->iterations = iters;
+    stats->deviceErrors = h.error;
+    cudaEventElapsedTime(&stats->gpuMs, r->evLoop0, r->evLoop1);
+    cudaEventElapsedTime(&stats->totalMs, r->ev0, r->ev1);
+    for (int j = 0; j < WRK_NUM_STAGES; ++j) {
+        stats->stageMs[j] = stageMs[j];
+        stats->stageLaunches[j] = stageN[j];
+    }
+}
+
+// Resolves the sums, copies the images out when `host` buffers are given, and waits.
+static int finish_render(wrk_renderer* r, const Frame& f, const wrk_render_params* p, float* d_rgb, float* d_alb,
+                         float* d_nrm, float* const* host) {
+    cudaStream_t st = r->eng.stream;
+    launch_resolve(f, p->flags & WRK_FLAG_RAW_GUIDES, d_rgb, d_alb, d_nrm, st);
+    CK(cudaGetLastError());
+    CK(cudaEventRecord(r->ev1, st));
+    if (host) {
+        float* const dev[3] = {d_rgb, d_alb, d_nrm};
+        for (int k = 0; k < 3; ++k)
+            if (host[k])
+                CK(cudaMemcpyAsync(host[k], dev[k], (size_t)p->width * p->height * 3 * sizeof(float),
+                                   cudaMemcpyDeviceToHost, st));
+    }
+    CK(cudaStreamSynchronize(st));
+    return WRK_OK;
+}
+
+// `host` (may be null): three host buffers the resolved images are copied to behind the
+// last kernel, so that the call waits for the device once.
 static int render_impl(wrk_renderer* r, wrk_scene* s, const wrk_camera* cam, const wrk_render_params* p, float* d_rgb,
-                       float* d_alb, float* d_nrm, wrk_render_stats* stats) {
+                       float* d_alb, float* d_nrm, float* const* host, wrk_render_stats* stats) {
     Engine& E = r->eng;
     Frame f;
     fill_frame(f, *cam, *p);
@@ -794,12 +835,38 @@ static int render_impl(wrk_renderer* r, wrk_scene* s, const wrk_camera* cam, con
     f.err = &E.q.ctr->error;
     f.scene = 0;
     cudaStream_t st = E.stream;
+    const unsigned long long work = (unsigned long long)np * p->spp;
+    const bool timing = (p->flags & WRK_FLAG_STAGE_TIMING) != 0;
+    float stageMs[WRK_NUM_STAGES] = {0};
+    uint32_t stageN[WRK_NUM_STAGES] = {0};
+    uint32_t iters = 0;
+    // (only the sums that are asked for are cleared: radiance | albedo | normal)
+    const size_t sums = d_nrm ? 3 : d_alb ? 2 : 1;
     CK(cudaEventRecord(r->ev0, st));
-    CK(cudaMemsetAsync(f.accum, 0, np * 3 * sizeof(float4), st));
+    CK(cudaMemsetAsync(f.accum, 0, np * sums * sizeof(float4), st));
+    // One launch when every path has a thread of its own (64 x 64 to 256 x 256 paths: the
+    // plain Cornell box 325 -> 140 and 351 -> 188 us, the showcase 642 -> 269 and 739 -> 543;
+    // at four times as many the wavefront is faster, 433 and 882 us against 469 and 1921)
+    // and the queues would have taken them at once, too.
+    if (!timing && work <= (unsigned long long)E.numSMs * kSmallBlocksPerSM * 128 && work <= E.capacity) {
+        CK(cudaMemsetAsync(E.q.ctr, 0, sizeof(Counters), st));
+        CK(cudaEventRecord(r->evLoop0, st));
+        launch_render_small(s->view, f, E.q.ctr, work, E.numSMs, st);
+        CK(cudaEventRecord(r->evLoop1, st));
+        CK(cudaMemcpyAsync(E.hCtr, E.q.ctr, sizeof(Counters), cudaMemcpyDeviceToHost, st));
+        if ((rc = finish_render(r, f, p, d_rgb, d_alb, d_nrm, host))) return rc;
+        if (E.hCtr->error) return fail(WRK_ERR_DEVICE, "device error flags 0x%x during render", E.hCtr->error);
+        // as the wavefront loop counts: whole chunks of iterations, from the first path's
+        // first to the last one's last
+        iters = (E.hCtr->iteration + E.cfg.chunk - 1) / E.cfg.chunk * E.cfg.chunk;
+        E.hCtr->paths = work;
+        fill_stats(r, iters, stageMs, stageN, stats);
+        return WRK_OK;
+    }
     E.hReq[0] = f;
     E.hScenes[0] = s->view;
     SlotCtl sc{};
-    sc.workTotal = (unsigned long long)np * p->spp;
+    sc.workTotal = work;
     sc.state = kSlotActive;
     E.hCtl[0] = sc;
     E.hGenOrder[0] = 1;
@@ -812,10 +879,6 @@ static int render_impl(wrk_renderer* r, wrk_scene* s, const wrk_camera* cam, con
     // bound on iterations: every path needs <= maxIter; waves of `capacity` paths
     unsigned long long waves = sc.workTotal / E.capacity + 2;
     unsigned long long maxIters = waves * (unsigned long long)(f.maxIter + 2) * 4ull + 64ull;
-    uint32_t iters = 0;
-    const bool timing = (p->flags & WRK_FLAG_STAGE_TIMING) != 0;
-    float stageMs[WRK_NUM_STAGES] = {0};
-    uint32_t stageN[WRK_NUM_STAGES] = {0};
     CK(cudaEventRecord(r->evLoop0, st));
     bool looped = false;
     if (!timing) {
@@ -842,27 +905,8 @@ static int render_impl(wrk_renderer* r, wrk_scene* s, const wrk_camera* cam, con
         if (iters > maxIters) return fail(WRK_ERR_DEVICE, "render did not converge after %u iterations", iters);
     }
     CK(cudaEventRecord(r->evLoop1, st));
-    launch_resolve(f, p->flags & WRK_FLAG_RAW_GUIDES, d_rgb, d_alb, d_nrm, st);
-    CK(cudaGetLastError());
-    CK(cudaEventRecord(r->ev1, st));
-    CK(cudaEventSynchronize(r->ev1));
-    if (stats) {
-        const Counters& h = *E.hCtr;
-        stats->paths = h.paths;
-        stats->extensionRays = h.extRays;
-        stats->shadowRays = h.shdRays + h.shadowAnswered.v;  // + the last iteration's answered queries
-        stats->shadowTraced = h.shdTraced;
-        for (int b = 0; b < kNumBuckets; ++b) stats->bucketPaths[b] = h.bucketTotal[b] + h.bucket[b].v;
-        stats->bucketPaths[kBucketLambert] += h.lambertTex.v;
-        stats->iterations = iters;
-        stats->deviceErrors = h.error;
-        cudaEventElapsedTime(&stats->gpuMs, r->evLoop0, r->evLoop1);
-        cudaEventElapsedTime(&stats->totalMs, r->ev0, r->ev1);
-        for (int j = 0; j < WRK_NUM_STAGES; ++j) {
-            stats->stageMs[j] = stageMs[j];
-            stats->stageLaunches[j] = stageN[j];
-        }
-    }
+    if ((rc = finish_render(r, f, p, d_rgb, d_alb, d_nrm, host))) return rc;
+    fill_stats(r, iters, stageMs, stageN, stats);
     return WRK_OK;
 }
 
@@ -881,7 +925,7 @@ int wrk_render_device(wrk_renderer* r, wrk_scene* s, const wrk_camera* cam, cons
     int rc = check_render_args(r, s, cam, p);
     if (rc) return rc;
     if (!d_rgb) return fail(WRK_ERR_INVALID, "null output");
-    return render_impl(r, s, cam, p, d_rgb, d_alb, d_nrm, stats);
+    return render_impl(r, s, cam, p, d_rgb, d_alb, d_nrm, nullptr, stats);
 }
 
 int wrk_render(wrk_renderer* r, wrk_scene* s, const wrk_camera* cam, const wrk_render_params* p, float* rgb,
@@ -892,12 +936,8 @@ int wrk_render(wrk_renderer* r, wrk_scene* s, const wrk_camera* cam, const wrk_r
     size_t np = (size_t)p->width * p->height;
     if ((rc = r->outBufs.alloc(np * 9 * sizeof(float)))) return rc;
     float* o = r->outBufs.as<float>();
-    if ((rc = render_impl(r, s, cam, p, o, albedo ? o + 3 * np : nullptr, normal ? o + 6 * np : nullptr, stats)))
-        return rc;
-    CK(cudaMemcpy(rgb, o, np * 3 * sizeof(float), cudaMemcpyDeviceToHost));
-    if (albedo) CK(cudaMemcpy(albedo, o + 3 * np, np * 3 * sizeof(float), cudaMemcpyDeviceToHost));
-    if (normal) CK(cudaMemcpy(normal, o + 6 * np, np * 3 * sizeof(float), cudaMemcpyDeviceToHost));
-    return WRK_OK;
+    float* const host[3] = {rgb, albedo, normal};
+    return render_impl(r, s, cam, p, o, albedo ? o + 3 * np : nullptr, normal ? o + 6 * np : nullptr, host, stats);
 }
 
 // ---------------------------------------------------------------------------

@@ -23,11 +23,15 @@
 // RNG is keyed by (pixel, sample), so the image does not depend on queue order.
 #include "wrk_internal.h"
 #include "wrk_shading.cuh"
+#include "wrk_trav.cuh"
 #include "wrk_tri.cuh"
 
 namespace wrk {
 
 constexpr int kShadeBlock = 256;
+// Range of a camera ray and of every later extension ray (whose tmin is 0).
+constexpr uint32_t kSmallCounters = 8;  // rays, shadow rays traced / answered, hits of four buckets, last iteration
+constexpr float kCameraTmin = 0.0001f, kRayTmax = 1e20f;
 
 __device__ __forceinline__ uint32_t append_pos(uint32_t* counter, bool pred, uint32_t cap, uint32_t* err) {
     uint32_t b = __ballot_sync(0xffffffffu, pred);
@@ -148,7 +152,54 @@ void launch_loop_cond(cudaGraphConditionalHandle h, const Queues& q, cudaStream_
     k_loop_cond<<<1, 1, 0, st>>>(h, q);
 }
 
-// Camera ray for (pixel, sample) of the request a work item belongs to: trace.cu:54-125.
+// The camera path of a request's work item w (trace.cu:54-125): pixel, seed, ray.
+__device__ __forceinline__ void camera_path(const Frame& f, unsigned long long w, uint32_t& pixel, uint32_t& seed,
+                                            float3& ro, float3& rd) {
+    const uint32_t perSample = f.perSample, width = f.width, tilesX = f.tilesX;
+    // blocks of K samples: within a block, each group of 32 work items covers
+    // 32/K consecutive pixel positions, with the K samples of a pixel adjacent
+    const uint32_t K = f.interleave;
+    const unsigned long long blk = (unsigned long long)perSample * K;
+    const uint32_t idx = (uint32_t)(w % blk), ln = idx & 31u;
+    uint32_t sample = f.sampleOffset + (uint32_t)(w / blk) * K + ln % K;
+    uint32_t j = (idx >> 5) * (32u / K) + ln / K;
+    uint32_t x, y;
+    if (tilesX) {
+        uint32_t tile = j >> 5, lane = j & 31u;
+        x = (tile % tilesX) * 8u + (lane & 7u);
+        y = (tile / tilesX) * 4u + (lane >> 3);
+    } else {
+        x = j % width;
+        y = j / width;
+    }
+    pixel = y * width + x;
+    seed = path_seed(pixel, sample, f.seed);
+    uint32_t js = seed;
+    float r1 = lcg_randf(js);
+    float r2 = lcg_randf(js);
+    float nx = (2.0f * ((float)x + r1) / (float)width - 1.0f) * f.aspect;
+    float ny = 1.0f - 2.0f * ((float)y + r2) / (float)f.height;
+    float3 fwd = f3(f.fwd[0], f.fwd[1], f.fwd[2]), rt = f3(f.right[0], f.right[1], f.right[2]),
+           up = f3(f.up[0], f.up[1], f.up[2]), pos = f3(f.pos[0], f.pos[1], f.pos[2]);
+    const float tanHalf = f.tanHalf;
+    float3 dir = normalize(add(add(fwd, mul(mul(rt, nx), tanHalf)), mul(mul(up, ny), tanHalf)));
+    ro = pos;
+    rd = dir;
+    const float lens = f.lens, focal = f.focal;
+    if (lens > 0.0f && focal > 0.0f) {
+        float r3 = lcg_randf(js), r4 = lcg_randf(js);
+        float th = 2.0f * 3.14159265f * r3;
+        float rad = sqrtf(r4) * lens;
+        float sn, ct;
+        sincosf(th, &sn, &ct);
+        float3 off = f3(rt.x * rad * ct + up.x * rad * sn, rt.y * rad * ct + up.y * rad * sn,
+                        rt.z * rad * ct + up.z * rad * sn);
+        float3 fp = f3(pos.x + dir.x * focal, pos.y + dir.y * focal, pos.z + dir.z * focal);
+        ro = f3(pos.x + off.x, pos.y + off.y, pos.z + off.z);
+        rd = normalize(f3(fp.x - ro.x, fp.y - ro.y, fp.z - ro.z));
+    }
+}
+
 __global__ void __launch_bounds__(kShadeBlock) k_generate(Queues q) {
     __shared__ GenSeg seg[kMaxSlots];
     Counters* c = q.ctr;
@@ -166,53 +217,12 @@ __global__ void __launch_bounds__(kShadeBlock) k_generate(Queues q) {
             else hi = mid;
         }
         const GenSeg sg = seg[lo];
-        const Frame& f = q.req[sg.slot];
         const uint32_t e = eb + i;
-        const unsigned long long w = sg.workBase + (i - sg.extOffset);
-        const uint32_t perSample = f.perSample, width = f.width, tilesX = f.tilesX;
-        // blocks of K samples: within a block, each group of 32 work items covers
-        // 32/K consecutive pixel positions, with the K samples of a pixel adjacent
-        const uint32_t K = f.interleave;
-        const unsigned long long blk = (unsigned long long)perSample * K;
-        const uint32_t idx = (uint32_t)(w % blk), ln = idx & 31u;
-        uint32_t sample = f.sampleOffset + (uint32_t)(w / blk) * K + ln % K;
-        uint32_t j = (idx >> 5) * (32u / K) + ln / K;
-        uint32_t x, y;
-        if (tilesX) {
-            uint32_t tile = j >> 5, lane = j & 31u;
-            x = (tile % tilesX) * 8u + (lane & 7u);
-            y = (tile / tilesX) * 4u + (lane >> 3);
-        } else {
-            x = j % width;
-            y = j / width;
-        }
-        uint32_t pixel = y * width + x;
-        uint32_t seed = path_seed(pixel, sample, f.seed);
-        uint32_t js = seed;
-        float r1 = lcg_randf(js);
-        float r2 = lcg_randf(js);
-        float nx = (2.0f * ((float)x + r1) / (float)width - 1.0f) * f.aspect;
-        float ny = 1.0f - 2.0f * ((float)y + r2) / (float)f.height;
-        float3 fwd = f3(f.fwd[0], f.fwd[1], f.fwd[2]), rt = f3(f.right[0], f.right[1], f.right[2]),
-               up = f3(f.up[0], f.up[1], f.up[2]), pos = f3(f.pos[0], f.pos[1], f.pos[2]);
-        const float tanHalf = f.tanHalf;
-        float3 dir = normalize(add(add(fwd, mul(mul(rt, nx), tanHalf)), mul(mul(up, ny), tanHalf)));
-        float3 ro = pos, rd = dir;
-        const float lens = f.lens, focal = f.focal;
-        if (lens > 0.0f && focal > 0.0f) {
-            float r3 = lcg_randf(js), r4 = lcg_randf(js);
-            float th = 2.0f * 3.14159265f * r3;
-            float rad = sqrtf(r4) * lens;
-            float sn, ct;
-            sincosf(th, &sn, &ct);
-            float3 off = f3(rt.x * rad * ct + up.x * rad * sn, rt.y * rad * ct + up.y * rad * sn,
-                            rt.z * rad * ct + up.z * rad * sn);
-            float3 fp = f3(pos.x + dir.x * focal, pos.y + dir.y * focal, pos.z + dir.z * focal);
-            ro = f3(pos.x + off.x, pos.y + off.y, pos.z + off.z);
-            rd = normalize(f3(fp.x - ro.x, fp.y - ro.y, fp.z - ro.z));
-        }
-        __stcs(o.ray_o + e, make_float4(ro.x, ro.y, ro.z, 0.0001f));
-        __stcs(o.ray_d + e, make_float4(rd.x, rd.y, rd.z, 1e20f));
+        uint32_t pixel, seed;
+        float3 ro, rd;
+        camera_path(q.req[sg.slot], sg.workBase + (i - sg.extOffset), pixel, seed, ro, rd);
+        __stcs(o.ray_o + e, make_float4(ro.x, ro.y, ro.z, kCameraTmin));
+        __stcs(o.ray_d + e, make_float4(rd.x, rd.y, rd.z, kRayTmax));
         __stcs(o.thr + e, make_float4(1.0f, 1.0f, 1.0f, 1.0f));
         __stcs(o.rad + e, make_float4(0.0f, 0.0f, 0.0f, __uint_as_float(pixel)));
         __stcs(o.st + e, make_uint4(seed, 0u, 0u, kFlagFirstHit | kFlagPrevDelta | (sg.slot << kSlotShift)));
@@ -675,7 +685,7 @@ __global__ void __launch_bounds__(kBlock, WRK_SHADE_MIN_BLOCKS * 256 / kBlock) k
             const PathQ o = pe != kInvalidSlot ? ext : (cur ? q.ext[1] : q.ext[0]);
             const uint32_t p = pe != kInvalidSlot ? pe : pc;
             __stcs(o.ray_o + p, make_float4(r.o.x, r.o.y, r.o.z, 0.0f));
-            __stcs(o.ray_d + p, make_float4(r.d.x, r.d.y, r.d.z, 1e20f));
+            __stcs(o.ray_d + p, make_float4(r.d.x, r.d.y, r.d.z, kRayTmax));
             __stcs(o.thr + p, make_float4(r.thr.x, r.thr.y, r.thr.z, r.prevPdf));
             __stcs(o.rad + p, make_float4(r.rad.x, r.rad.y, r.rad.z, __uint_as_float(r.pixel)));
             __stcs(o.st + p, make_uint4(r.seed, r.dim, (r.depth & 0xffffu) | (r.iter << 16), r.flags));
@@ -713,6 +723,121 @@ void launch_shade_bucket(uint32_t b, const DevScene& s, const Queues& q, bool mu
         if (multi) launch_shade_t<true, 256>(b, s, q, grid, st);
         else launch_shade_t<false, 256>(b, s, q, grid, st);
     }
+}
+
+// ---------------------------------------------------------------------------
+// One-launch renderer of small images: a thread carries a path from its camera ray to its
+// end in registers -- closest hit, shade, shadow ray, next bounce -- and then takes its
+// next work item.  Same device functions and per-path decisions as the wavefront kernels;
+// only the order of the f32 sums into a pixel differs.  No queues, no per-iteration
+// launches: a wavefront of a few thousand paths is eight times seven dependent launches.
+// At scale the wavefront wins, whose warps hold rays and hits of one kind.
+__global__ void __launch_bounds__(kTraceBlock, kSmallBlocksPerSM) k_render_small(DevScene s, Frame f, Counters* c,
+                                                                                unsigned long long work,
+                                                                                uint32_t lanes) {
+    __shared__ uint2 sstack[kStackSmem * kTraceBlock];
+    __shared__ float4 sdir[kTraceBlock];
+    __shared__ uint32_t sum[kSmallCounters];
+    uint2 lstack[kStackLocal];
+    if (threadIdx.x < kSmallCounters) sum[threadIdx.x] = 0;
+    __syncthreads();
+    const TraceGeom geo{s.nodes, s.tris, s.pairs, s.numNodes, s.numTris};
+    const uint32_t warp = blockIdx.x * (kTraceBlock / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
+    const unsigned long long stride = (unsigned long long)gridDim.x * (kTraceBlock / 32) * lanes;
+    unsigned long long w = lane < lanes ? (unsigned long long)warp * lanes + lane : work;
+    uint32_t nExt = 0, nShadow = 0, nAnswered = 0, nBucket[kBucketLambertResume] = {0, 0, 0, 0}, lastIter = 0;
+    PathRegs r;
+    float tmin = 0.0f;
+    bool alive = false;
+    PathQ none{};
+    while (true) {
+        if (!alive) {
+            if (w >= work) break;
+            camera_path(f, w, r.pixel, r.seed, r.o, r.d);
+            w += stride;
+            r.thr = f3(1.0f, 1.0f, 1.0f);
+            r.rad = f3(0.0f, 0.0f, 0.0f);
+            r.prevPdf = 1.0f;
+            r.dim = r.depth = r.iter = 0;
+            r.flags = kFlagFirstHit | kFlagPrevDelta;
+            tmin = kCameraTmin;
+        }
+        Trav t;
+        trav_init(t, sdir, Ray{r.o.x, r.o.y, r.o.z, r.d.x, r.d.y, r.d.z, tmin, kRayTmax});
+        while (!trav_step<false, true>(geo, t, sdir, sstack, lstack, f.err)) {
+        }
+        ++nExt;
+        alive = false;
+        lastIter = max(lastIter, r.iter + 1u);
+        if (t.lBest == kNoHit) {
+            miss_accumulate(s, f, make_float4(r.thr.x, r.thr.y, r.thr.z, r.prevPdf),
+                            make_float4(r.rad.x, r.rad.y, r.rad.z, __uint_as_float(r.pixel)), r.d);
+            continue;
+        }
+        const uint32_t word = __float_as_uint(__ldg(s.tris + 3 * (size_t)t.lBest + 2).w);
+        const uint32_t bucket = min(word & ~kRecTextured, (uint32_t)kBucketOther);
+        const float4 o4 = make_float4(r.o.x, r.o.y, r.o.z, tmin), d4 = make_float4(r.d.x, r.d.y, r.d.z, t.tBest),
+                     h4 = make_float4(t.tBest, __uint_as_float(record_prim(s.tris, t.lBest)),
+                                      __uint_as_float(record_material(s.tris, t.lBest)), __uint_as_float(t.lBest)),
+                     t4 = make_float4(r.thr.x, r.thr.y, r.thr.z, r.prevPdf),
+                     r4 = make_float4(r.rad.x, r.rad.y, r.rad.z, __uint_as_float(r.pixel));
+        const uint4 st = make_uint4(r.seed, r.dim, (r.depth & 0xffffu) | (r.iter << 16), r.flags);
+        ShadowOut so;
+        so.cont = kContDrop;
+        so.answered = false;
+        int out;
+        switch (bucket) {
+            case kBucketLambert: out = shade_one<kBucketLambert>(s, none, 0, f, r, so, o4, d4, h4, t4, r4, st); break;
+            case kBucketDielectric: out = shade_one<kBucketDielectric>(s, none, 0, f, r, so, o4, d4, h4, t4, r4, st); break;
+            case kBucketGGX: out = shade_one<kBucketGGX>(s, none, 0, f, r, so, o4, d4, h4, t4, r4, st); break;
+            default: out = shade_one<kBucketOther>(s, none, 0, f, r, so, o4, d4, h4, t4, r4, st); break;
+        }
+#pragma unroll
+        for (uint32_t b = 0; b < kBucketLambertResume; ++b) nBucket[b] += bucket == b ? 1u : 0u;
+        nAnswered += so.answered ? 1u : 0u;
+        alive = out == kOutExt || out == kOutCont;
+        if (out == kOutShadow) {
+            ++nShadow;
+            lastIter = max(lastIter, (st.z >> 16) + 2u);  // traced an iteration later
+            trav_init(t, sdir, Ray{so.o.x, so.o.y, so.o.z, so.d.x, so.d.y, so.d.z, kShadowTmin, so.dist - kShadowTmin});
+            while (!trav_step<true, true>(geo, t, sdir, sstack, lstack, f.err)) {
+            }
+            if (t.lBest == kNoHit && so.cont != kContDrop)
+                r.rad = f3(r.rad.x + so.c.x, r.rad.y + so.c.y, r.rad.z + so.c.z);
+            if (so.cont == kContAccumulate) accumulate(f, r);
+            alive = so.cont == kContExt;
+        }
+        tmin = 0.0f;
+    }
+    const uint32_t mine[kSmallCounters] = {nExt,       nShadow,    nAnswered, nBucket[0],
+                                           nBucket[1], nBucket[2], nBucket[3], lastIter};
+#pragma unroll
+    for (uint32_t k = 0; k < kSmallCounters; ++k) {
+        if (k + 1 < kSmallCounters) atomicAdd(&sum[k], mine[k]);
+        else atomicMax(&sum[k], mine[k]);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        atomicAdd(&c->extRays, (unsigned long long)sum[0]);
+        atomicAdd(&c->shdTraced, (unsigned long long)sum[1]);
+        atomicAdd(&c->shdRays, (unsigned long long)sum[1] + sum[2]);
+        for (uint32_t b = 0; b < kBucketLambertResume; ++b) atomicAdd(&c->bucketTotal[b], (unsigned long long)sum[3 + b]);
+        atomicAdd(&c->bucketTotal[kBucketLambertResume], (unsigned long long)sum[1]);
+        atomicMax(&c->iteration, sum[kSmallCounters - 1]);
+    }
+}
+
+void launch_render_small(const DevScene& s, const Frame& f, Counters* c, unsigned long long work, int numSMs,
+                         cudaStream_t st) {
+    // few paths spread over one warp per scheduler, with `lanes` of each warp in use: a path
+    // then waits for few others' traversals and materials (more warps would compete for
+    // issue slots: 128 x 128 paths of the showcase 377 us with 8 lanes a warp, 294 with 32)
+    const unsigned long long warps = (unsigned long long)numSMs * 4;
+    uint32_t lanes = 32;
+    while (lanes > 1 && work * 2 <= warps * lanes) lanes /= 2;
+    const unsigned long long perBlock = (unsigned long long)lanes * (kTraceBlock / 32), blocks = (work + perBlock - 1) / perBlock;
+    const unsigned long long most = (unsigned long long)numSMs * kSmallBlocksPerSM;
+    k_render_small<<<(int)(blocks < most ? blocks : most), kTraceBlock, 0, st>>>(s, f, c, work, lanes);
 }
 
 // rgb = sum * (1/spp) as renderer.cpp:308-313; guides averaged unless raw.

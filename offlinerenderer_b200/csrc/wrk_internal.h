@@ -238,6 +238,13 @@ void launch_trace_extension(const DevScene& s, const Queues& q, bool multi, int 
 void launch_trace_shadow(const DevScene& s, const Queues& q, bool multi, int numSMs, cudaStream_t st);
 void launch_shade_bucket(uint32_t bucket, const DevScene& s, const Queues& q, bool multi, int grid, int block,
                          cudaStream_t st);
+// The one-launch renderer's blocks of 128 threads per SM (127 registers a thread).
+constexpr int kSmallBlocksPerSM = 4;
+// Renders `work` work items of request `f` in one launch (small images; no queues).  The
+// statistics go to zeroed counters; `iteration` receives the wavefront iterations the
+// longest path would take.
+void launch_render_small(const DevScene& s, const Frame& f, Counters* c, unsigned long long work, int numSMs,
+                         cudaStream_t st);
 void launch_resolve(const Frame& f, uint32_t rawGuides, float* rgb, float* albedo, float* normal, cudaStream_t st);
 // End of one chunk of the device-driven loop: keeps the enclosing conditional
 // WHILE graph node running while a request in the admission order has work left.
