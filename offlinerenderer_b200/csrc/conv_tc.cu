@@ -252,6 +252,11 @@ __global__ void __launch_bounds__(fwd_threads(kResident), kResident && BLOCKS !=
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmemSlot;
+    // The next launch may set itself up from here on; this one touches what earlier
+    // launches produce only after they are done (weights and biases are older: they change
+    // between passes, in launches that wait).
+    grid_launch_dependents();
+    if (warp != kEpiWarps + 2) grid_wait();
 
     const uint32_t perImg = sh.tilesX * sh.tilesY;
     const uint32_t items = sh.B * perImg * sh.nSplit;
@@ -876,7 +881,10 @@ int plan_wgrad(uint32_t B, uint32_t H, uint32_t W, uint32_t Cin, uint32_t Cout, 
     sh.stages = S;
     p->smem = smem_for(S * stage + (2 * S + 1) * 8 + 16 + 1024, sh.tmemCols);
     const uint32_t cells = 9 * sh.ciBlocks * sh.coBlocks;
-    uint32_t splits = std::max(1u, (2 * numSMs + cells - 1) / cells);
+    // Two waves of blocks (each takes an SM's shared memory): rounded up, 9 cells x 33 splits
+    // were 297 blocks, three waves of 148.  One wave takes as long, and its sums, twice as
+    // long in TMEM before they meet in dW, were ten times further from two waves' ones.
+    uint32_t splits = std::max(1u, 2 * numSMs / cells);
     splits = std::min(splits, sh.tilesTotal);
     sh.tilesPerCta = (sh.tilesTotal + splits - 1) / splits;
     splits = (sh.tilesTotal + sh.tilesPerCta - 1) / sh.tilesPerCta;
@@ -890,13 +898,26 @@ static cudaError_t set_smem(K kern, uint32_t bytes) {
 }
 
 cudaError_t launch_fwd(const FwdPlan& p, const CUtensorMap& mx, const CUtensorMap& mw, const OutMaps& mo,
-                       const Epilogue& ep, uint32_t* err, cudaStream_t st) {
+                       const Epilogue& ep, bool overlap, uint32_t* err, cudaStream_t st) {
     cudaError_t e = cudaErrorInvalidValue;
+    // overlap: launched while its predecessor drains (see the kernel's grid_wait), so that its
+    // barriers, TMEM and resident weights are ready when the predecessor ends (300 x 170
+    // frame 226 -> 180 us)
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t lc{};
+    lc.gridDim = dim3(p.grid);
+    lc.blockDim = dim3(fwd_threads(p.resident));
+    lc.dynamicSmemBytes = p.smem;
+    lc.stream = st;
+    lc.attrs = &at;
+    lc.numAttrs = overlap ? 1 : 0;
 #define WRK_FWD_CASE(CHUNK, RES, BLOCKS)                                                                  \
     if (p.chunk == CHUNK && p.resident == RES && (BLOCKS == 0 || p.shape.Cin == CHUNK * BLOCKS)) {        \
         e = set_smem(k_conv_fwd<CHUNK, RES, BLOCKS>, p.smem);                                             \
         if (e == cudaSuccess)                                                                             \
-            k_conv_fwd<CHUNK, RES, BLOCKS><<<p.grid, fwd_threads(RES), p.smem, st>>>(mx, mw, mo, p.shape, ep, err); \
+            e = cudaLaunchKernelEx(&lc, k_conv_fwd<CHUNK, RES, BLOCKS>, mx, mw, mo, p.shape, ep, err);        \
         return e != cudaSuccess ? e : cudaGetLastError();                                                 \
     }
     WRK_FWD_CASE(16, true, 1)

@@ -77,8 +77,10 @@ int plan_wgrad(uint32_t B, uint32_t H, uint32_t W, uint32_t Cin, uint32_t Cout, 
 int make_input_map(const FwdPlan& p, const void* x, CUtensorMap* mx);
 int make_weight_map(const FwdPlan& p, const void* w, CUtensorMap* mw);
 int make_out_maps(const FwdPlan& p, void* out, uint32_t stride, uint32_t offset, bool f32, bool up, OutMaps* mo);
+// overlap: the launch may begin before the stream's previous kernel has ended; the weights
+// and the bias must then be older than that kernel.
 cudaError_t launch_fwd(const FwdPlan& p, const CUtensorMap& mx, const CUtensorMap& mw, const OutMaps& mo,
-                       const Epilogue& ep, uint32_t* err, cudaStream_t st);
+                       const Epilogue& ep, bool overlap, uint32_t* err, cudaStream_t st);
 cudaError_t launch_wgrad(const WgradPlan& p, const CUtensorMap& mg, const CUtensorMap& mx, float* dW, uint32_t* err,
                          cudaStream_t st);
 

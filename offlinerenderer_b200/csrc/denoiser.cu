@@ -484,7 +484,7 @@ int forward(wrk_denoiser* d, const float* rgb, uint32_t h, uint32_t w, float* ds
             ep.headH = h;
             ep.headW = w;
         }
-        DCK(conv::launch_fwd(d->fplan[i], d->fin[i], d->fw[i], d->fout[i], ep, d->err.as<uint32_t>(), d->stream));
+        DCK(conv::launch_fwd(d->fplan[i], d->fin[i], d->fw[i], d->fout[i], ep, true, d->err.as<uint32_t>(), d->stream));
     }
     return WRK_OK;
 }
@@ -531,7 +531,8 @@ int backward(wrk_denoiser* d) {
             ep.outF32 = mask ? 0 : 1;
             ep.mask = (const __nv_bfloat16*)mask;
             ep.maskStride = L.cin;
-            DCK(conv::launch_fwd(d->dplan[i], d->din[i], d->dwmap[i], d->dout[i], ep, d->err.as<uint32_t>(), d->stream));
+            DCK(conv::launch_fwd(d->dplan[i], d->din[i], d->dwmap[i], d->dout[i], ep, true, d->err.as<uint32_t>(),
+                                 d->stream));
         }
         // combine kernels that produce the G of the layer below
         const uint32_t catC[3] = {96, 192, 384};
@@ -655,7 +656,7 @@ int wrk_conv3x3_forward(const void* x, uint32_t B, uint32_t H, uint32_t W, uint3
     ep.outF32 = f32;
     // whole 16-byte rows leave by TMA; a padded Cout or an unaligned output by element stores
     if (N == Cout && conv::make_out_maps(plan, out, Cout, 0, f32, false, &mo) == 0) ep.nOut = 1;
-    DCK(conv::launch_fwd(plan, mx, mw, mo, ep, err.as<uint32_t>(), 0));
+    DCK(conv::launch_fwd(plan, mx, mw, mo, ep, false, err.as<uint32_t>(), 0));
     uint32_t e = 0;
     DCK(cudaMemcpy(&e, err.p, 4, cudaMemcpyDeviceToHost));
     if (e) return dfail(WRK_ERR_DEVICE, "conv kernel timed out (flags 0x%x)", e);
