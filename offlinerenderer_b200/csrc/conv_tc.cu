@@ -604,6 +604,8 @@ __global__ void __launch_bounds__(128, 1)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmemSlot;
+    grid_launch_dependents();
+    grid_wait();
     const uint32_t perImg = sh.tilesX * sh.tilesY;
     const uint32_t kSteps = t1 > t0 ? t1 - t0 : 0;
 
@@ -934,15 +936,26 @@ cudaError_t launch_fwd(const FwdPlan& p, const CUtensorMap& mx, const CUtensorMa
     return e != cudaSuccess ? e : cudaGetLastError();
 }
 
-#define WRK_WGRAD_CASE(A, B)                                                                        \
-    if (p.ca == A && p.cb == B) {                                                                   \
-        e = set_smem(k_conv_wgrad<A, B>, p.smem);                                                   \
-        if (e == cudaSuccess) k_conv_wgrad<A, B><<<p.grid, 128, p.smem, st>>>(mg, mx, p.shape, dW, err); \
-        return e != cudaSuccess ? e : cudaGetLastError();                                           \
+#define WRK_WGRAD_CASE(A, B)                                                              \
+    if (p.ca == A && p.cb == B) {                                                         \
+        e = set_smem(k_conv_wgrad<A, B>, p.smem);                                         \
+        if (e == cudaSuccess)                                                             \
+            e = cudaLaunchKernelEx(&lc, k_conv_wgrad<A, B>, mg, mx, p.shape, dW, err);    \
+        return e != cudaSuccess ? e : cudaGetLastError();                                 \
     }
 
-cudaError_t launch_wgrad(const WgradPlan& p, const CUtensorMap& mg, const CUtensorMap& mx, float* dW, uint32_t* err,
-                         cudaStream_t st) {
+cudaError_t launch_wgrad(const WgradPlan& p, const CUtensorMap& mg, const CUtensorMap& mx, float* dW, bool overlap,
+                         uint32_t* err, cudaStream_t st) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t lc{};
+    lc.gridDim = p.grid;
+    lc.blockDim = dim3(128);
+    lc.dynamicSmemBytes = p.smem;
+    lc.stream = st;
+    lc.attrs = &at;
+    lc.numAttrs = overlap ? 1 : 0;
     cudaError_t e = cudaSuccess;
     WRK_WGRAD_CASE(64, 64)
     WRK_WGRAD_CASE(64, 32)

@@ -81,8 +81,8 @@ int make_out_maps(const FwdPlan& p, void* out, uint32_t stride, uint32_t offset,
 // and the bias must then be older than that kernel.
 cudaError_t launch_fwd(const FwdPlan& p, const CUtensorMap& mx, const CUtensorMap& mw, const OutMaps& mo,
                        const Epilogue& ep, bool overlap, uint32_t* err, cudaStream_t st);
-cudaError_t launch_wgrad(const WgradPlan& p, const CUtensorMap& mg, const CUtensorMap& mx, float* dW, uint32_t* err,
-                         cudaStream_t st);
+cudaError_t launch_wgrad(const WgradPlan& p, const CUtensorMap& mg, const CUtensorMap& mx, float* dW, bool overlap,
+                         uint32_t* err, cudaStream_t st);
 
 }  // namespace conv
 }  // namespace wrk

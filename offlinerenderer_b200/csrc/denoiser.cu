@@ -145,31 +145,40 @@ __global__ void k_skip_bwd(const float* dcat, uint32_t stride, uint32_t off, uin
     }
 }
 
-// bias gradient: db[c] += sum_p g[p][c].  A thread sums one 8-channel group (16 bytes a
-// load) of every (threads / groups)-th pixel; the block's partial sums meet in shared
-// memory.  (With 2-byte loads a layer took 10-18 us, the fifteen of a training pass of 16
-// 128 x 128 crops 190 us; now 5-11 and 115.)
-__global__ void __launch_bounds__(256) k_bias_grad(const __nv_bfloat16* __restrict__ g, size_t P, uint32_t C,
-                                                   uint32_t cValid, float* db) {
+// Bias gradients of all layers: db[c] += sum_p g[p][c], layer blockIdx.y.  A thread sums one
+// 8-channel group (16 bytes a load) of every (threads / groups)-th pixel; the block's
+// partial sums meet in shared memory.  (One launch per layer with 2-byte loads took 10-18
+// us each, 190 us of a training pass of 16 128 x 128 crops; 112 with 16-byte loads.)
+struct BiasJob {
+    const __nv_bfloat16* g;  // [P][C]
+    float* db;
+    uint32_t P, C, cValid;
+};
+struct BiasJobs {
+    BiasJob j[kLayers];
+};
+__global__ void __launch_bounds__(256) k_bias_grad(const __grid_constant__ BiasJobs jobs) {
     __shared__ float red[8][256 + 1];
-    const uint32_t G = C / 8, lanes = blockDim.x / G;  // groups of a pixel, pixels a block takes at a time
+    const BiasJob& job = jobs.j[blockIdx.y];
+    const uint32_t G = job.C / 8, lanes = blockDim.x / G;  // groups of a pixel, pixels a block takes at a time
+    if (blockIdx.x * lanes >= job.P) return;
     const uint32_t grp = threadIdx.x % G, r = threadIdx.x / G;
     float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     if (r < lanes) {
-        const size_t step = (size_t)gridDim.x * lanes;
+        const uint32_t step = gridDim.x * lanes;
 #pragma unroll 4
-        for (size_t p = blockIdx.x * (size_t)lanes + r; p < P; p += step) {
+        for (uint32_t p = blockIdx.x * lanes + r; p < job.P; p += step) {
             float f[8];
-            bf8_to_f(__ldg((const uint4*)(g + p * C) + grp), f);
+            bf8_to_f(__ldg((const uint4*)(job.g + (size_t)p * job.C) + grp), f);
             for (int j = 0; j < 8; ++j) acc[j] += f[j];
         }
     }
     for (int j = 0; j < 8; ++j) red[j][threadIdx.x] = acc[j];
     __syncthreads();
-    for (uint32_t c = threadIdx.x; c < cValid; c += blockDim.x) {
+    for (uint32_t c = threadIdx.x; c < job.cValid; c += blockDim.x) {
         float s = 0.0f;
         for (uint32_t k = 0; k < lanes; ++k) s += red[c % 8][k * G + c / 8];
-        atomicAdd(db + c, s);
+        atomicAdd(job.db + c, s);
     }
 }
 
@@ -509,20 +518,10 @@ const void* input_mask(wrk_denoiser* d, int i) {
 int backward(wrk_denoiser* d) {
     const uint32_t B = d->B;
     DCK(cudaMemsetAsync(d->grads.p, 0, d->nparams * 4, d->stream));
-    for (int i = kLayers - 1; i >= 0; --i) {
+    // the data gradients first, down to the first layer's G; then the weight and bias
+    // gradients, which only read the Gs and the activations
+    for (int i = kLayers - 1; i > 0; --i) {
         const LayerDef& L = kDefs[i];
-        const uint32_t h = lvl_h(d, L.level), w = lvl_w(d, L.level), coPad = pad16(L.cout);
-        // weight and bias gradients
-        DCK(conv::launch_wgrad(d->wplan[i], d->wg[i], d->wx[i], d->grads.as<float>() + d->woff[i],
-                               d->err.as<uint32_t>(), d->stream));
-        {
-            // g has coPad channels; only the layer's real output channels have a bias
-            const size_t P = (size_t)B * h * w;
-            const size_t perBlock = 256 / (coPad / 8);
-            k_bias_grad<<<(unsigned)std::min<size_t>(296, (P + perBlock - 1) / perBlock), 256, 0, d->stream>>>(
-                d->g[i].as<__nv_bfloat16>(), P, coPad, L.cout, d->grads.as<float>() + d->boff[i]);
-        }
-        if (i == 0) break;
         // data gradient into the layer's input
         {
             Epilogue ep{};
@@ -554,6 +553,16 @@ int backward(wrk_denoiser* d) {
                                                            d->cat[l].as<__nv_bfloat16>(), d->g[i - 1].as<__nv_bfloat16>());
         }
     }
+    BiasJobs jobs;
+    for (int i = kLayers - 1; i >= 0; --i) {
+        const LayerDef& L = kDefs[i];
+        DCK(conv::launch_wgrad(d->wplan[i], d->wg[i], d->wx[i], d->grads.as<float>() + d->woff[i], true,
+                               d->err.as<uint32_t>(), d->stream));
+        // g has coPad channels; only the layer's real output channels have a bias
+        jobs.j[i] = BiasJob{d->g[i].as<__nv_bfloat16>(), d->grads.as<float>() + d->boff[i],
+                            B * lvl_h(d, L.level) * lvl_w(d, L.level), pad16(L.cout), L.cout};
+    }
+    k_bias_grad<<<dim3(148, kLayers), 256, 0, d->stream>>>(jobs);
     DCK(cudaGetLastError());
     return WRK_OK;
 }
@@ -678,7 +687,7 @@ int wrk_conv3x3_wgrad(const void* g, const void* x, uint32_t B, uint32_t H, uint
     CUtensorMap mg, mx;
     if (conv::make_act_map(&mg, g, Cout, W, H, B, plan.ca) || conv::make_act_map(&mx, x, Cin, W, H, B, plan.cb))
         return dfail(WRK_ERR_CUDA, "tensor map encoding failed (pointers must be 16-byte aligned)");
-    DCK(conv::launch_wgrad(plan, mg, mx, dw, err.as<uint32_t>(), 0));
+    DCK(conv::launch_wgrad(plan, mg, mx, dw, false, err.as<uint32_t>(), 0));
     uint32_t e = 0;
     DCK(cudaMemcpy(&e, err.p, 4, cudaMemcpyDeviceToHost));
     if (e) return dfail(WRK_ERR_DEVICE, "weight-gradient kernel timed out (flags 0x%x)", e);
