@@ -124,8 +124,10 @@ struct wrk_scene {
     std::vector<float> envMap;
     uint32_t envW = 0, envH = 0;
     bool finalized = false;
-    DevBuf dEnvMap;
-    DevBuf dVtx, dNrm, dUv, dIdx, dTriMat, dMats, dTexels, dTexInfo, dEmissive, dCdf, dLights, dErr, dPairs;
+    // one device allocation holds everything but the tree (a dozen of them, 0.1-0.3 ms each
+    // to make and to free, were a quarter of a 676k-triangle scene's life)
+    DevBuf arena;
+    uint32_t* dErr = nullptr;
     uint4* nodes = nullptr;
     float4* tris = nullptr;
     std::vector<uint32_t> emissive;
@@ -444,13 +446,20 @@ void build_light_cdf(wrk_scene* s) {
     for (float& c : s->cdf) c /= total;
 }
 
+// Lays arrays out in one allocation: place() returns each one's offset.
+struct ArenaPlan {
+    size_t bytes = 0;
+    template <class T> size_t place(size_t n) {
+        const size_t at = bytes;
+        bytes += (n * sizeof(T) + 255) & ~size_t(255);
+        return at;
+    }
+};
+
 template <class T>
-int upload(DevBuf& b, const std::vector<T>& v) {
-    if (v.empty()) return WRK_OK;
-    int rc = b.alloc(sizeof(T) * v.size());
-    if (rc) return rc;
-    CK(cudaMemcpy(b.p, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice));
-    return WRK_OK;
+cudaError_t copy_in(const DevBuf& arena, size_t at, const std::vector<T>& v) {
+    if (v.empty()) return cudaSuccess;
+    return cudaMemcpyAsync(arena.as<uint8_t>() + at, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice, 0);
 }
 
 int check_scene(wrk_scene* s) {
@@ -521,7 +530,9 @@ int wrk_scene_set_geometry(wrk_scene* s, const float* vertices, uint32_t nv, con
     if (!s || !vertices || !indices || !triMaterial) return fail(WRK_ERR_INVALID, "null geometry argument");
     if (s->finalized) return fail(WRK_ERR_STATE, "scene already finalized");
     if (nv == 0 || nt == 0) return fail(WRK_ERR_INVALID, "Scene has no geometry");
-    for (size_t i = 0; i < 3 * (size_t)nt; ++i)
+    uint32_t top = 0;  // (one pass without branches; the offender is looked up only if there is one)
+    for (size_t i = 0; i < 3 * (size_t)nt; ++i) top = std::max(top, indices[i]);
+    for (size_t i = 0; top >= nv && i < 3 * (size_t)nt; ++i)
         if (indices[i] >= nv) return fail(WRK_ERR_INVALID, "index %u out of range (vertex count %u)", indices[i], nv);
     s->vtx.assign(vertices, vertices + 3 * (size_t)nv);
     s->nrm.clear();
@@ -589,37 +600,68 @@ int wrk_scene_finalize(wrk_scene* s) {
         lights.push_back(make_float4(c[0], c[1], c[2], 0.0f));
         lights.push_back(make_float4(m.emission[0], m.emission[1], m.emission[2], 0.0f));
     }
-    if ((rc = upload(s->dLights, lights))) return rc;
-    if ((rc = upload(s->dVtx, s->vtx)) || (rc = upload(s->dNrm, s->nrm)) || (rc = upload(s->dUv, s->uv)) ||
-        (rc = upload(s->dIdx, s->idx)) || (rc = upload(s->dTriMat, s->triMat)) || (rc = upload(s->dMats, s->mats)) ||
-        (rc = upload(s->dEmissive, s->emissive)) || (rc = upload(s->dCdf, s->cdf)))
-        return rc;
-    // texel pool + per-texture info
     std::vector<TexInfo> ti;
-    size_t total = 0;
+    size_t texelBytes = 0;
     for (size_t i = 0; i < s->tex.size(); ++i) {
-        ti.push_back(TexInfo{total, s->texW[i], s->texH[i]});
-        total += (s->tex[i].size() + 15) & ~size_t(15);
+        ti.push_back(TexInfo{texelBytes, s->texW[i], s->texH[i]});
+        texelBytes += (s->tex[i].size() + 15) & ~size_t(15);
     }
-    if (!s->tex.empty()) {
-        if ((rc = s->dTexels.alloc(total))) return rc;
-        for (size_t i = 0; i < s->tex.size(); ++i)
-            CK(cudaMemcpy(s->dTexels.as<uint8_t>() + ti[i].offset, s->tex[i].data(), s->tex[i].size(),
-                          cudaMemcpyHostToDevice));
-        if ((rc = upload(s->dTexInfo, ti))) return rc;
+    ArenaPlan plan;
+    const size_t oVtx = plan.place<float>(s->vtx.size()), oNrm = plan.place<float>(s->nrm.size()),
+                 oUv = plan.place<float>(s->uv.size()), oIdx = plan.place<uint32_t>(s->idx.size()),
+                 oTriMat = plan.place<uint32_t>(s->triMat.size()), oMats = plan.place<wrk_material>(s->mats.size()),
+                 oTexels = plan.place<uint8_t>(texelBytes), oTi = plan.place<TexInfo>(ti.size()),
+                 oEmissive = plan.place<uint32_t>(s->emissive.size()), oCdf = plan.place<float>(s->cdf.size()),
+                 oLights = plan.place<float4>(lights.size()), oEnv = plan.place<float>(s->envMap.size()),
+                 oErr = plan.place<uint32_t>(1), oPairs = plan.place<float4>(5 * (size_t)nt);
+    if ((rc = s->arena.alloc(plan.bytes))) return rc;
+    uint8_t* const base = s->arena.as<uint8_t>();
+    CK(copy_in(s->arena, oVtx, s->vtx));
+    CK(copy_in(s->arena, oNrm, s->nrm));
+    CK(copy_in(s->arena, oUv, s->uv));
+    CK(copy_in(s->arena, oIdx, s->idx));
+    CK(copy_in(s->arena, oTriMat, s->triMat));
+    CK(copy_in(s->arena, oMats, s->mats));
+    for (size_t i = 0; i < s->tex.size(); ++i) CK(copy_in(s->arena, oTexels + ti[i].offset, s->tex[i]));
+    CK(copy_in(s->arena, oTi, ti));
+    CK(copy_in(s->arena, oEmissive, s->emissive));
+    CK(copy_in(s->arena, oCdf, s->cdf));
+    CK(copy_in(s->arena, oLights, lights));
+    CK(copy_in(s->arena, oEnv, s->envMap));
+    DevScene& v = s->view;
+    auto at = [&](size_t off, bool have) { return have ? base + off : nullptr; };
+    v.vtx = (const float*)(base + oVtx);
+    v.nrm = (const float*)at(oNrm, !s->nrm.empty());
+    v.uv = (const float*)at(oUv, !s->uv.empty());
+    v.idx = (const uint32_t*)(base + oIdx);
+    v.triMat = (const uint32_t*)(base + oTriMat);
+    v.mats = (const wrk_material*)at(oMats, !s->mats.empty());
+    v.numMats = (uint32_t)s->mats.size();
+    v.texels = at(oTexels, !s->tex.empty());
+    v.tex = (const TexInfo*)at(oTi, !s->tex.empty());
+    v.numTex = (uint32_t)s->tex.size();
+    v.emissive = (const uint32_t*)at(oEmissive, !s->emissive.empty());
+    v.cdf = (const float*)at(oCdf, !s->cdf.empty());
+    v.lights = (const float4*)at(oLights, !lights.empty());
+    v.numEmissive = (uint32_t)s->emissive.size();
+    v.numTris = nt;
+    for (int k = 0; k < 3; ++k) v.env[k] = s->env[k];
+    if (!s->envMap.empty()) {
+        v.envMap = (const float4*)(base + oEnv);
+        v.envW = s->envW;
+        v.envH = s->envH;
     }
-    if ((rc = s->dErr.alloc(sizeof(uint32_t)))) return rc;
+    s->dErr = (uint32_t*)(base + oErr);
+    float4* const pairs = (float4*)(base + oPairs);
     BvhBuildResult br{};
     char err[256] = {0};
-    rc = build_bvh8(s->dVtx.as<float>(), s->dIdx.as<uint32_t>(), s->dTriMat.as<uint32_t>(), nt, 0, &br, err,
-                    sizeof(err));
+    rc = build_bvh8(v.vtx, v.idx, v.triMat, nt, 0, &br, err, sizeof(err));
     if (rc) return fail(rc, "%s", err);
     s->nodes = br.nodes;
     s->tris = br.tris;
     // the shade bucket of each record's material, so the trace kernel sorts a hit
     // with one load from its record, and the two-triangle records traversal tests
-    if ((rc = s->dPairs.alloc(5 * sizeof(float4) * (size_t)nt))) return rc;
-    launch_leaf_records(br.tris, nt, s->dMats.as<wrk_material>(), (uint32_t)s->mats.size(), s->dPairs.as<float4>(), 0);
+    launch_leaf_records(br.tris, nt, v.mats, v.numMats, pairs, 0);
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(0));
     s->info.numTriangles = nt;
@@ -629,33 +671,10 @@ int wrk_scene_finalize(wrk_scene* s) {
     s->info.numEmissive = (uint32_t)s->emissive.size();
     s->info.buildMs = br.ms;
     s->info.sahCost = br.sah;
-    DevScene& v = s->view;
-    v.vtx = s->dVtx.as<float>();
-    v.nrm = s->nrm.empty() ? nullptr : s->dNrm.as<float>();
-    v.uv = s->uv.empty() ? nullptr : s->dUv.as<float>();
-    v.idx = s->dIdx.as<uint32_t>();
-    v.triMat = s->dTriMat.as<uint32_t>();
-    v.mats = s->dMats.as<wrk_material>();
-    v.numMats = (uint32_t)s->mats.size();
-    v.texels = s->dTexels.as<uint8_t>();
-    v.tex = s->dTexInfo.as<TexInfo>();
-    v.numTex = (uint32_t)s->tex.size();
-    v.emissive = s->dEmissive.as<uint32_t>();
-    v.cdf = s->dCdf.as<float>();
-    v.lights = s->dLights.as<float4>();
-    v.numEmissive = (uint32_t)s->emissive.size();
-    v.numTris = nt;
-    for (int k = 0; k < 3; ++k) v.env[k] = s->env[k];
     v.nodes = s->nodes;
     v.tris = s->tris;
-    v.pairs = s->dPairs.as<float4>();
+    v.pairs = pairs;
     v.numNodes = br.numNodes;
-    if (!s->envMap.empty()) {
-        if ((rc = upload(s->dEnvMap, s->envMap))) return rc;
-        v.envMap = s->dEnvMap.as<float4>();
-        v.envW = s->envW;
-        v.envH = s->envH;
-    }
     s->finalized = true;
     return WRK_OK;
 }
@@ -677,8 +696,8 @@ int wrk_scene_light_cdf(wrk_scene* s, uint32_t* tris, float* cdf, uint32_t capac
     if (n > capacity) return fail(WRK_ERR_INVALID, "capacity %u < %u emissive triangles", capacity, n);
     if (n) {
         // read back what the device holds
-        if (tris) CK(cudaMemcpy(tris, s->dEmissive.p, sizeof(uint32_t) * n, cudaMemcpyDeviceToHost));
-        if (cdf) CK(cudaMemcpy(cdf, s->dCdf.p, sizeof(float) * n, cudaMemcpyDeviceToHost));
+        if (tris) CK(cudaMemcpy(tris, s->view.emissive, sizeof(uint32_t) * n, cudaMemcpyDeviceToHost));
+        if (cdf) CK(cudaMemcpy(cdf, s->view.cdf, sizeof(float) * n, cudaMemcpyDeviceToHost));
     }
     return WRK_OK;
 }
@@ -945,11 +964,11 @@ int wrk_trace_closest(wrk_scene* s, const float* rays, uint32_t n, float* t, uin
     int rc = check_scene(s);
     if (rc) return rc;
     if (n && (!rays || !t || !prim)) return fail(WRK_ERR_INVALID, "null buffer");
-    CK(cudaMemset(s->dErr.p, 0, sizeof(uint32_t)));
-    launch_closest_query(s->view, rays, n, t, prim, s->dErr.as<uint32_t>(), 0);
+    CK(cudaMemset(s->dErr, 0, sizeof(uint32_t)));
+    launch_closest_query(s->view, rays, n, t, prim, s->dErr, 0);
     CK(cudaGetLastError());
     uint32_t e = 0;
-    CK(cudaMemcpy(&e, s->dErr.p, sizeof(uint32_t), cudaMemcpyDeviceToHost));
+    CK(cudaMemcpy(&e, s->dErr, sizeof(uint32_t), cudaMemcpyDeviceToHost));
     if (e) return fail(WRK_ERR_DEVICE, "trace error flags 0x%x", e);
     return WRK_OK;
 }
@@ -957,11 +976,11 @@ int wrk_trace_occluded(wrk_scene* s, const float* rays, uint32_t n, uint32_t* oc
     int rc = check_scene(s);
     if (rc) return rc;
     if (n && (!rays || !occ)) return fail(WRK_ERR_INVALID, "null buffer");
-    CK(cudaMemset(s->dErr.p, 0, sizeof(uint32_t)));
-    launch_occluded_query(s->view, rays, n, occ, s->dErr.as<uint32_t>(), 0);
+    CK(cudaMemset(s->dErr, 0, sizeof(uint32_t)));
+    launch_occluded_query(s->view, rays, n, occ, s->dErr, 0);
     CK(cudaGetLastError());
     uint32_t e = 0;
-    CK(cudaMemcpy(&e, s->dErr.p, sizeof(uint32_t), cudaMemcpyDeviceToHost));
+    CK(cudaMemcpy(&e, s->dErr, sizeof(uint32_t), cudaMemcpyDeviceToHost));
     if (e) return fail(WRK_ERR_DEVICE, "trace error flags 0x%x", e);
     return WRK_OK;
 }
@@ -997,7 +1016,7 @@ int wrk_texture_batch(wrk_scene* s, uint32_t id, const float* uv, uint32_t n, fl
     if (id == 0 || id > s->tex.size()) return fail(WRK_ERR_INVALID, "texture id %u out of range", id);
     size_t off = 0;
     for (uint32_t i = 0; i + 1 < id; ++i) off += (s->tex[i].size() + 15) & ~size_t(15);
-    launch_texture(s->dTexels.as<uint8_t>() + off, s->texW[id - 1], s->texH[id - 1], uv, n, out, 0);
+    launch_texture(s->view.texels + off, s->texW[id - 1], s->texH[id - 1], uv, n, out, 0);
     CK(cudaGetLastError());
     CK(cudaDeviceSynchronize());
     return WRK_OK;
