@@ -12,11 +12,9 @@
 //                2x2 average pool, the nearest 2x upsample (four stores) or the network's
 //                output image, so those take no passes of their own.
 // k_conv_wgrad -- weight gradient dW[co][tap][ci] = sum_p G[p][co] X[p+tap][ci]:
-//                M = 128 output channels, N = input channels, K = pixels; both
-//                operands are loaded channel-contiguous (MN-major) so the tap shift
-//                lands on the pixel coordinates of the TMA box, never on the
-//                16-byte-aligned channel coordinate.  Split over pixel ranges, f32
-//                vector atomics into dW.
+//                M = 3 taps x input channels (128 rows), N = output channels, K = pixels;
+//                both operands channel-contiguous (MN-major), the taps are descriptors into
+//                one halo.  Split over pixel ranges, f32 atomics into dW.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -34,9 +32,9 @@ namespace conv {
 
 using namespace tc;
 
-constexpr uint32_t kTileW = 16, kTileH = 8, kTileP = 128;
+constexpr uint32_t kTileP = 128;  // pixels of a tile
 
-__host__ __device__ inline uint32_t round_up(uint32_t x, uint32_t a) { return (x + a - 1) / a * a; }
+__host__ __device__ constexpr uint32_t round_up(uint32_t x, uint32_t a) { return (x + a - 1) / a * a; }
 
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
@@ -83,6 +81,11 @@ __host__ __device__ constexpr uint32_t fwd_threads(bool resident) { return (fwd_
 __host__ __device__ constexpr uint32_t halo_block_bytes(uint32_t chunk) {
     return (kHaloPix * chunk * 2 + 1023) / 1024 * 1024;
 }
+
+// Rows of the halo that a weight-gradient block with one or all three rows of taps reads,
+// and TMEM columns of one row's sums
+__host__ __device__ constexpr uint32_t wgrad_halo_rows(uint32_t rows) { return kHTileH + rows - 1; }
+__host__ __device__ constexpr uint32_t wgrad_cols(uint32_t cout) { return (cout + 31) / 32 * 32; }
 
 // ---- epilogue ----
 // 16-byte unit u of row r in a staging tile of rowBytes-wide rows, swizzled as the TMA
@@ -546,21 +549,32 @@ __global__ void __launch_bounds__(fwd_threads(kResident), kResident && BLOCKS !=
 }
 
 // ---------------------------------------------------------------------------
-template <int CA, int CB>
+// Weight gradient.  A block keeps the sums of one row of taps, or of all three (ROWS), of CB
+// input and CA output channels in TMEM.  Per 8 x 16 pixel tile it loads G once and the
+// input's halo once (10 pixels wide, 16 or 18 high); both are channel-contiguous (MN-major),
+// K = pixels.  M holds the taps of a row times the input channels: the operand's channel
+// groups are one pixel apart (LBO), so group dx reads the halo shifted by dx pixels (groups
+// past the third are padding and not stored), and rows of 8 pixels are 10 halo rows apart as
+// in k_conv_fwd.  N = the output channels, with an accumulator per dy.  f32 atomics into dW,
+// a warp's lanes along its input channels.
+//
+// What bounds it: a block per tap loaded both operands nine times and padded M from the 16
+// to 64 output channels of the wide layers to 128 (32 x 32 channels over 16 x 128 x 128
+// pixels 63 us, 31 of them MMAs; L2 at 4.8 TB/s).  Now 16 us, 10 of them MMAs, the rest
+// its start and its atomics; 192 -> 64 channels at half the width 37 -> 28 us, 256 -> 256 at
+// an eighth 25 -> 17 us; a training pass at 16 x 128 x 128 1106 -> 850 us.
+template <int CA, int CB, int ROWS>
 __global__ void __launch_bounds__(128, 1)
     k_conv_wgrad(const __grid_constant__ CUtensorMap mg, const __grid_constant__ CUtensorMap mx, WgradShape sh,
-                 float* dW, uint32_t* err) {
+                  float* dW, uint32_t* err) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     constexpr uint32_t kRowA = CA * 2, kRowB = CB * 2;
-    constexpr uint32_t kAtomA = kTileP * kRowA, kAtomB = kTileP * kRowB;  // one channel group x 128 pixels
-    constexpr uint32_t kAtomsA = 128 / CA;
-    constexpr uint32_t kABytes = kAtomsA * kAtomA;  // 32 KB
-    const uint32_t nAtomsB = sh.NB / CB;
-    const uint32_t bBytes = nAtomsB * kAtomB;
-    const uint32_t stageBytes = kABytes + bBytes;
+    constexpr uint32_t kHalo = wgrad_halo_rows(ROWS) * kHaloW, kHaloBytes = round_up(kHalo * kRowB, 1024), kStage = kHaloBytes + kTileP * kRowA;
+    constexpr uint32_t kCols = wgrad_cols(CA);
+    static_assert(ROWS * kCols <= (ROWS == 1 ? 128 : 256), "the plan's TMEM columns");
     const uint32_t S = sh.stages;
-    uint64_t* bars = (uint64_t*)(smem + S * stageBytes);
+    uint64_t* bars = (uint64_t*)(smem + S * kStage);
     uint32_t* tmemSlot = (uint32_t*)(bars + 2 * S + 1);
     volatile uint32_t* abortFlag = tmemSlot + 1;
     const uint32_t base = smem_u32(smem);
@@ -568,23 +582,10 @@ __global__ void __launch_bounds__(128, 1)
     auto empty = [&](uint32_t s) { return smem_u32(bars + S + s); };
     const uint32_t accum = smem_u32(bars + 2 * S);
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    const uint32_t ci0 = blockIdx.y * CB, co0 = blockIdx.z / (3 / ROWS) * CA;
+    const uint32_t dy0 = blockIdx.z % (3 / ROWS);  // the block's first row of taps
+    const uint32_t t0 = blockIdx.x * sh.tilesPerCta, t1 = min(sh.tilesTotal, t0 + sh.tilesPerCta);
 
-    const uint32_t tap = blockIdx.z % 9, coBlock = blockIdx.z / 9;
-    const uint32_t co0 = coBlock * 128, ci0 = blockIdx.y * sh.NB;
-    const uint32_t loadedA = min(kAtomsA, (sh.Cout - co0 + CA - 1) / CA);
-    const uint32_t t0 = blockIdx.x * sh.tilesPerCta;
-    const uint32_t t1 = min(sh.tilesTotal, t0 + sh.tilesPerCta);
-    const int dy = (int)(tap / 3) - 1, dx = (int)(tap % 3) - 1;
-
-    // output-channel groups past Cout are never loaded: zero them once
-    if (loadedA < kAtomsA) {
-        for (uint32_t s = 0; s < S; ++s) {
-            uint4* z = (uint4*)(smem + s * stageBytes + loadedA * kAtomA);
-            const uint32_t n16 = (kAtomsA - loadedA) * kAtomA / 16;
-            for (uint32_t i = threadIdx.x; i < n16; i += blockDim.x) z[i] = make_uint4(0, 0, 0, 0);
-        }
-        fence_proxy_async();
-    }
     if (threadIdx.x == 0) {
         for (uint32_t s = 0; s < S; ++s) {
             mbar_init(full(s), 1);
@@ -619,13 +620,11 @@ __global__ void __launch_bounds__(128, 1)
                 }
                 const uint32_t t = t0 + k;
                 const uint32_t b = t / perImg, rem = t % perImg;
-                const int h0 = (int)((rem / sh.tilesX) * kTileH), w0 = (int)((rem % sh.tilesX) * kTileW);
-                mbar_expect_tx(full(s), loadedA * kAtomA + bBytes);
-                const uint32_t sa = base + s * stageBytes;
-                for (uint32_t a = 0; a < loadedA; ++a)
-                    tma_load_4d(sa + a * kAtomA, &mg, full(s), (int)(co0 + a * CA), w0, h0, (int)b);
-                for (uint32_t a = 0; a < nAtomsB; ++a)
-                    tma_load_4d(sa + kABytes + a * kAtomB, &mx, full(s), (int)(ci0 + a * CB), w0 + dx, h0 + dy, (int)b);
+                const int h0 = (int)((rem / sh.tilesX) * kHTileH), w0 = (int)((rem % sh.tilesX) * kHTileW);
+                mbar_expect_tx(full(s), kHalo * kRowB + kTileP * kRowA);
+                const uint32_t sa = base + s * kStage;
+                tma_load_4d(sa, &mx, full(s), (int)ci0, w0 - 1, h0 - 1 + (int)dy0, (int)b);
+                tma_load_4d(sa + kHaloBytes, &mg, full(s), (int)co0, w0, h0, (int)b);
                 ++issued;
                 if (++s == S) {
                     s = 0;
@@ -637,26 +636,24 @@ __global__ void __launch_bounds__(128, 1)
             }
         }
     } else if (warp == 1) {
-        // the whole warp waits (uniform control flow), one elected lane issues; the operands
-        // come from TMA and need only their barriers, not a tcgen05 fence per step (32 x 32
-        // channels over 16 x 128 x 128 pixels: 88 -> 63 us, 31 of it MMAs, three quarters
-        // of their 128 rows padding)
         const bool leader = elect_one();
-        const uint32_t idesc = idesc_bf16(sh.NB, true, true);
-        const uint32_t layA = layout_for_row_bytes(kRowA), layB = layout_for_row_bytes(kRowB);
+        const uint32_t idesc = idesc_bf16(CA, true, true);
+        const uint32_t layG = layout_for_row_bytes(kRowA), layX = layout_for_row_bytes(kRowB);
         uint32_t s = 0, ph = 0;
         for (uint32_t k = 0; k < kSteps; ++k) {
             if (!warp_wait(full(s), ph)) {
                 *abortFlag = 1;
                 break;
             }
-            const uint32_t a0 = base + s * stageBytes, b0 = a0 + kABytes;
-            // 16 pixels = two 8-row groups; LBO = next channel group, SBO = next 8 pixels
-            const uint64_t ad = sdesc(a0, kAtomA, 8 * kRowA, layA), bd = sdesc(b0, kAtomB, 8 * kRowB, layB);
+            const uint32_t b0 = base + s * kStage;
+            const uint64_t xd = sdesc(b0, kRowB, kHaloW * kRowB, layX), gd = sdesc(b0 + kHaloBytes, 0, 8 * kRowA, layG);
             if (leader) {
 #pragma unroll
                 for (uint32_t kk = 0; kk < kTileP / 16; ++kk)
-                    umma_bf16(tmem, ad + kk * kRowA, bd + kk * kRowB, idesc, (k | kk) ? 1u : 0u);
+#pragma unroll
+                    for (uint32_t dy = 0; dy < ROWS; ++dy)  // 16 pixels: two rows of the tile
+                        umma_bf16(tmem + dy * kCols, xd + (2 * kk + dy) * (kHaloW * kRowB / 16), gd + kk * kRowA, idesc,
+                                  (k | kk) ? 1u : 0u);
                 umma_commit(empty(s));
             }
             __syncwarp();
@@ -675,14 +672,19 @@ __global__ void __launch_bounds__(128, 1)
     if (!ready || *abortFlag) {
         if (threadIdx.x == 0) atomicOr(err, 1u);
     } else if (kSteps > 0) {
-        const uint32_t co = co0 + warp * 32 + lane;
-        for (uint32_t c0 = 0; c0 < sh.NB; c0 += 16) {
-            float v[16];
-            tmem_ld16(tmem + ((warp * 32u) << 16) + c0, v);
-            if (co < sh.coutStore) {
-                float* o = dW + ((size_t)co * 9 + tap) * sh.Cin + ci0 + c0;
+        // row dx * CB + ci, column co: a warp adds 32 (or 2 x 16) consecutive weights at a time
+        const uint32_t row = warp * 32 + lane, dx = row / CB, ci = row % CB;
+        if (warp * 32 < 3 * CB) {
+#pragma unroll 1
+            for (uint32_t j = 0; j < ROWS * CA / 16; ++j) {
+                const uint32_t dy = j / (CA / 16), c0 = j % (CA / 16) * 16, co = co0 + c0;
+                float v[16];
+                tmem_ld16(tmem + ((warp * 32u) << 16) + dy * kCols + c0, v);
+                if (dx >= 3) continue;
+                float* o = dW + ((size_t)co * 9 + (dy0 + dy) * 3 + dx) * sh.Cin + ci0 + ci;
 #pragma unroll
-                for (uint32_t j = 0; j < 16; j += 4) atomicAdd((float4*)(o + j), make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]));
+                for (uint32_t i = 0; i < 16; ++i)
+                    if (co + i < sh.coutStore) atomicAdd(o + (size_t)i * 9 * sh.Cin, v[i]);
             }
         }
     }
@@ -712,20 +714,6 @@ static EncodeTiledFn encode_fn() {
 static CUtensorMapSwizzle swizzle_for(uint32_t rowBytes) {
     return rowBytes == 128 ? CU_TENSOR_MAP_SWIZZLE_128B
                            : rowBytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B;
-}
-
-int make_act_map(CUtensorMap* m, const void* base, uint32_t C, uint32_t W, uint32_t H, uint32_t B, uint32_t boxC) {
-    EncodeTiledFn enc = encode_fn();
-    if (!enc) return 1;
-    if (((uintptr_t)base & 15u) || (C * 2) % 16 || boxC * 2 > 128 || (boxC * 2) % 32) return 2;
-    cuuint64_t dims[4] = {C, W, H, B};
-    cuuint64_t strides[3] = {(cuuint64_t)C * 2, (cuuint64_t)W * C * 2, (cuuint64_t)H * W * C * 2};
-    cuuint32_t box[4] = {boxC, kTileW, kTileH, 1};
-    cuuint32_t es[4] = {1, 1, 1, 1};
-    CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, es,
-                     CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle_for(boxC * 2), CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return r == CUDA_SUCCESS ? 0 : 3;
 }
 
 static uint32_t pow2_cols(uint32_t n) {
@@ -858,39 +846,47 @@ int make_out_maps(const FwdPlan& p, void* out, uint32_t stride, uint32_t offset,
     return 0;
 }
 
+int make_wgrad_maps(const WgradPlan& p, const void* g, const void* x, uint32_t B, uint32_t H, uint32_t W, uint32_t Cin,
+                    uint32_t Cout, CUtensorMap* mg, CUtensorMap* mx) {
+    auto nhwc = [&](CUtensorMap* m, const void* base, uint32_t C, uint32_t boxC, uint32_t boxW, uint32_t boxH) {
+        return encode4(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, base, {C, W, H, B},
+                       {(cuuint64_t)C * 2, (cuuint64_t)W * C * 2, (cuuint64_t)H * W * C * 2}, {boxC, boxW, boxH, 1},
+                       boxC * 2);
+    };
+    const int rc = nhwc(mg, g, Cout, p.ca, kHTileW, kHTileH);
+    return rc ? rc : nhwc(mx, x, Cin, p.cb, kHaloW, wgrad_halo_rows(p.rows));
+}
+
 int plan_wgrad(uint32_t B, uint32_t H, uint32_t W, uint32_t Cin, uint32_t Cout, uint32_t numSMs, WgradPlan* p) {
-    if (Cin == 0 || Cin % 16 || Cout == 0 || Cout % 16 || W % kTileW || H % kTileH || B == 0) return 1;
+    if (Cin == 0 || Cin % 16 || Cout == 0 || Cout % 16 || W % 16 || H % 8 || B == 0) return 1;
+    if (Cin > 512 || (Cin > 256 && Cin % 32)) return 1;
     WgradShape& sh = p->shape;
-    sh.B = B;
-    sh.H = H;
-    sh.W = W;
     sh.Cin = Cin;
-    sh.Cout = Cout;
     sh.coutStore = Cout;
-    sh.tilesX = W / kTileW;
-    sh.tilesY = H / kTileH;
+    sh.tilesX = W / kHTileW;
+    sh.tilesY = (H + kHTileH - 1) / kHTileH;
     sh.tilesTotal = B * sh.tilesX * sh.tilesY;
-    sh.NB = Cin <= 256 ? Cin : (Cin % 2 == 0 && (Cin / 2) % 16 == 0 ? Cin / 2 : 0);
-    if (sh.NB == 0 || sh.NB > 256) return 1;
-    sh.ciBlocks = Cin / sh.NB;
-    sh.coBlocks = (Cout + 127) / 128;
-    p->ca = std::min<uint32_t>(64, (uint32_t)chunk_for(Cout));
-    p->cb = chunk_for(sh.NB);
-    if (128 % p->ca) return 1;
-    sh.tmemCols = pow2_cols(sh.NB);
-    const uint32_t stage = 128 * kTileP * 2 + sh.NB * kTileP * 2;
-    uint32_t S = std::max(2u, std::min(6u, (200u * 1024u) / stage));
-    sh.stages = S;
-    p->smem = smem_for(S * stage + (2 * S + 1) * 8 + 16 + 1024, sh.tmemCols);
-    const uint32_t cells = 9 * sh.ciBlocks * sh.coBlocks;
-    // Two waves of blocks (each takes an SM's shared memory): rounded up, 9 cells x 33 splits
-    // were 297 blocks, three waves of 148.  One wave takes as long, and its sums, twice as
-    // long in TMEM before they meet in dW, were ten times further from two waves' ones.
-    uint32_t splits = std::max(1u, 2 * numSMs / cells);
-    splits = std::min(splits, sh.tilesTotal);
+    p->ca = chunk_for(Cout);
+    p->cb = Cin % 32 == 0 ? 32 : 16;
+    // One wave of blocks, two an SM: one covers the other's start and atomics (one an SM:
+    // 36 us for 96 -> 32 channels at full width, 32 with two), and a second wave would cost
+    // a start (256 -> 256 channels at an eighth: 17 us, 24 with twice the blocks).  The
+    // full-width layers (up to 32 output channels, the most pixels) give each row of taps
+    // its own blocks: a third of the splits' atomics for G loaded three times (a training
+    // pass 862 -> 850 us); with several blocks of input channels their splits would be so
+    // few that a block's sums in TMEM, which truncate, grow longer than they were, so four
+    // blocks share an SM there.
+    p->rows = p->ca == 64 ? 3 : 1;
+    const uint32_t ciBlocks = Cin / p->cb, coBlocks = Cout / p->ca * (3 / p->rows);
+    const uint32_t perSM = p->rows == 1 && ciBlocks > 1 ? 4 : 2;
+    sh.tmemCols = 512 / perSM;  // of which rows * wgrad_cols(ca) are used: 192 of 256, or 32
+    const uint32_t stage = round_up(wgrad_halo_rows(p->rows) * kHaloW * p->cb * 2, 1024) + kTileP * p->ca * 2;
+    sh.stages = std::min(6u, (224u * 1024u / perSM - 2048u) / stage);
+    p->smem = smem_for(sh.stages * stage + (2 * sh.stages + 1) * 8 + 16 + 1024, sh.tmemCols);
+    uint32_t splits = std::min(std::max(1u, perSM * numSMs / (ciBlocks * coBlocks)), sh.tilesTotal);
     sh.tilesPerCta = (sh.tilesTotal + splits - 1) / splits;
     splits = (sh.tilesTotal + sh.tilesPerCta - 1) / sh.tilesPerCta;
-    p->grid = dim3(splits, sh.ciBlocks, 9 * sh.coBlocks);
+    p->grid = dim3(splits, ciBlocks, coBlocks);
     return 0;
 }
 
@@ -936,14 +932,6 @@ cudaError_t launch_fwd(const FwdPlan& p, const CUtensorMap& mx, const CUtensorMa
     return e != cudaSuccess ? e : cudaGetLastError();
 }
 
-#define WRK_WGRAD_CASE(A, B)                                                              \
-    if (p.ca == A && p.cb == B) {                                                         \
-        e = set_smem(k_conv_wgrad<A, B>, p.smem);                                         \
-        if (e == cudaSuccess)                                                             \
-            e = cudaLaunchKernelEx(&lc, k_conv_wgrad<A, B>, mg, mx, p.shape, dW, err);    \
-        return e != cudaSuccess ? e : cudaGetLastError();                                 \
-    }
-
 cudaError_t launch_wgrad(const WgradPlan& p, const CUtensorMap& mg, const CUtensorMap& mx, float* dW, bool overlap,
                          uint32_t* err, cudaStream_t st) {
     cudaLaunchAttribute at{};
@@ -957,15 +945,20 @@ cudaError_t launch_wgrad(const WgradPlan& p, const CUtensorMap& mg, const CUtens
     lc.attrs = &at;
     lc.numAttrs = overlap ? 1 : 0;
     cudaError_t e = cudaSuccess;
-    WRK_WGRAD_CASE(64, 64)
-    WRK_WGRAD_CASE(64, 32)
-    WRK_WGRAD_CASE(64, 16)
-    WRK_WGRAD_CASE(32, 64)
-    WRK_WGRAD_CASE(32, 32)
-    WRK_WGRAD_CASE(32, 16)
-    WRK_WGRAD_CASE(16, 64)
-    WRK_WGRAD_CASE(16, 32)
-    WRK_WGRAD_CASE(16, 16)
+#define WRK_WGRAD_CASE(A, B, ROWS)                                                           \
+    if (p.ca == A && p.cb == B && p.rows == ROWS) {                                          \
+        e = set_smem(k_conv_wgrad<A, B, ROWS>, p.smem);                                      \
+        if (e == cudaSuccess)                                                                \
+            e = cudaLaunchKernelEx(&lc, k_conv_wgrad<A, B, ROWS>, mg, mx, p.shape, dW, err); \
+        return e != cudaSuccess ? e : cudaGetLastError();                                    \
+    }
+    WRK_WGRAD_CASE(64, 32, 3)
+    WRK_WGRAD_CASE(64, 16, 3)
+    WRK_WGRAD_CASE(32, 32, 1)
+    WRK_WGRAD_CASE(32, 16, 1)
+    WRK_WGRAD_CASE(16, 32, 1)
+    WRK_WGRAD_CASE(16, 16, 1)
+#undef WRK_WGRAD_CASE
     return cudaErrorInvalidValue;
 }
 

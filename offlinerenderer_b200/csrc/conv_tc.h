@@ -40,11 +40,9 @@ struct Epilogue {
 };
 
 struct WgradShape {
-    uint32_t B, H, W, Cin, Cout;  // Cout = channels of G (a multiple of 16)
-    uint32_t coutStore;           // rows of dW that exist (<= Cout)
+    uint32_t Cin;
+    uint32_t coutStore;  // rows of dW that exist (<= the channels of G)
     uint32_t tilesX, tilesY, tilesTotal, tilesPerCta;
-    uint32_t NB;  // input channels per block (= N of the MMA)
-    uint32_t ciBlocks, coBlocks;
     uint32_t stages, tmemCols;
 };
 
@@ -61,14 +59,15 @@ struct FwdPlan {
 };
 struct WgradPlan {
     WgradShape shape;
-    uint32_t ca, cb, smem;
+    uint32_t ca, cb, rows, smem;  // output channels, input channels and rows of taps of a block
     dim3 grid;
 };
 
 int chunk_for(uint32_t channels);
-// Activation map for the weight gradient: NHWC bf16, box = boxC channels x 16 x 8 pixels.
 // All map functions return 0 on success.
-int make_act_map(CUtensorMap* m, const void* base, uint32_t C, uint32_t W, uint32_t H, uint32_t B, uint32_t boxC);
+// Maps of a weight gradient: G and the layer's input, NHWC bf16.
+int make_wgrad_maps(const WgradPlan& p, const void* g, const void* x, uint32_t B, uint32_t H, uint32_t W, uint32_t Cin,
+                    uint32_t Cout, CUtensorMap* mg, CUtensorMap* mx);
 int plan_fwd(uint32_t B, uint32_t H, uint32_t W, uint32_t Cin, uint32_t N, bool outF32, uint32_t numSMs, FwdPlan* p);
 int plan_wgrad(uint32_t B, uint32_t H, uint32_t W, uint32_t Cin, uint32_t Cout, uint32_t numSMs, WgradPlan* p);
 // Tensor maps of a forward plan: the input, the weights [N * nSplit][9 * Cin] bf16, and

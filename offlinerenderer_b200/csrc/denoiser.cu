@@ -449,8 +449,7 @@ int set_shape(wrk_denoiser* d, uint32_t B, uint32_t H, uint32_t W, bool train) {
         if (conv::plan_wgrad(B, h, w, L.cin, coPad, d->numSMs, &d->wplan[i]))
             return dfail(WRK_ERR_INVALID, "no weight-gradient plan for layer %d", i);
         d->wplan[i].shape.coutStore = L.cout;
-        if (conv::make_act_map(&d->wg[i], d->g[i].p, coPad, w, h, B, d->wplan[i].ca) ||
-            conv::make_act_map(&d->wx[i], io.in, L.cin, w, h, B, d->wplan[i].cb))
+        if (conv::make_wgrad_maps(d->wplan[i], d->g[i].p, io.in, B, h, w, L.cin, coPad, &d->wg[i], &d->wx[i]))
             return dfail(WRK_ERR_CUDA, "tensor map encoding failed (layer %d wgrad)", i);
         // data gradient: input g[i] (coPad), weights Wd [cin][9][coPad], output cin channels
         if (i > 0) {
@@ -685,7 +684,7 @@ int wrk_conv3x3_wgrad(const void* g, const void* x, uint32_t B, uint32_t H, uint
     if (err.alloc(4)) return dfail(WRK_ERR_CUDA, "allocation failed");
     DCK(cudaMemset(err.p, 0, 4));
     CUtensorMap mg, mx;
-    if (conv::make_act_map(&mg, g, Cout, W, H, B, plan.ca) || conv::make_act_map(&mx, x, Cin, W, H, B, plan.cb))
+    if (conv::make_wgrad_maps(plan, g, x, B, H, W, Cin, Cout, &mg, &mx))
         return dfail(WRK_ERR_CUDA, "tensor map encoding failed (pointers must be 16-byte aligned)");
     DCK(conv::launch_wgrad(plan, mg, mx, dw, false, err.as<uint32_t>(), 0));
     uint32_t e = 0;
