@@ -4,8 +4,11 @@
 //   Scene (resident):  vertices / normals / uvs / indices / per-triangle material
 //                      (the flat soup libWR uploads, scene.cpp:360-390), 64 B materials,
 //                      RGBA8 texels, emissive list + power CDF, the 8-wide BVH
-//                      (80 B nodes = 5 x uint4) and leaf-ordered triangle records
-//                      (48 B = 3 x float4: v0|prim, e1|material, e2).
+//                      (80 B nodes = 5 x uint4), leaf-ordered triangle records
+//                      (48 B = 3 x float4: v0|prim, e1|material, e2) and pair records
+//                      (80 B per leaf position: it and its follower, component by
+//                      component, for the two-triangle test).  One allocation holds all
+//                      but the nodes and triangle records.
 //   Path queues: a path's state travels with it from queue to queue.  Every queue
 //   stores its entries SoA -- one array per field, one float4 / uint4 per entry --
 //   so a kernel reading entries i..i+31 of a field, or writing the consecutive
