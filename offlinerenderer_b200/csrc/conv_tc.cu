@@ -248,6 +248,7 @@ __global__ void __launch_bounds__(fwd_threads(kResident), kResident && BLOCKS !=
     if (ep.bias)
         for (uint32_t c = threadIdx.x; c < 256; c += blockDim.x) biasS[c] = c < ep.nBias ? ep.bias[c] : 0.0f;
     if (warp == 0) {
+        __syncwarp();
         tmem_alloc(smem_u32(tmemSlot), sh.tmemCols);
         tmem_relinquish();
     }
@@ -273,7 +274,7 @@ __global__ void __launch_bounds__(fwd_threads(kResident), kResident && BLOCKS !=
         for (uint32_t item = blockIdx.x; ok && item < items; item += gridDim.x) {
             const TileAt at = tile_at(sh, perImg, invImg, invX, item);
             for (uint32_t g = 0; g < G; ++g) {
-                if (*abortFlag || !warp_wait(emptyA(s), ph)) {
+                if (warp_any(*abortFlag) || !warp_wait(emptyA(s), ph)) {
                     ok = false;
                     break;
                 }
@@ -411,7 +412,7 @@ __global__ void __launch_bounds__(fwd_threads(kResident), kResident && BLOCKS !=
                     umma_commit(accFull(buf));
                 }
                 __syncwarp();
-                ok = !*abortFlag;
+                ok = !warp_any(*abortFlag);
             }
             sa0 += G;
             if (sa0 >= RA) {
@@ -446,7 +447,7 @@ __global__ void __launch_bounds__(fwd_threads(kResident), kResident && BLOCKS !=
             float rgb[3] = {0.0f, 0.0f, 0.0f};  // (fetched ahead of the wait)
             if (ep.headDst && h < ep.headH && w < ep.headW)
                 for (uint32_t j = 0; j < 3; ++j) rgb[j] = ep.headRgb[3 * headAt + j];
-            if (*abortFlag || !warp_wait(accFull(buf), use & 1u)) {
+            if (warp_any(*abortFlag) || !warp_wait(accFull(buf), use & 1u)) {
                 *abortFlag = 1;
                 break;
             }
@@ -464,15 +465,15 @@ __global__ void __launch_bounds__(fwd_threads(kResident), kResident && BLOCKS !=
                             tmem_ld_wait();
                             if (plain) {
                                 stage32(rowAddr, rowSwz, c, biasS + n0 + c0 + c, ep.relu, r);
-                                continue;
-                            }
+                            } else {
 #pragma unroll
-                            for (uint32_t q = 0; q < 2; ++q) {
-                                float v[16];
+                                for (uint32_t q = 0; q < 2; ++q) {
+                                    float v[16];
 #pragma unroll
-                                for (uint32_t j = 0; j < 16; ++j) v[j] = __uint_as_float(r[16 * q + j]);
-                                finish16(ep, biasS, n0 + c0 + c + 16 * q, pix, inside, v);
-                                stage16(rowAddr, rowSwz, c + 16 * q, ep.outF32, v);
+                                    for (uint32_t j = 0; j < 16; ++j) v[j] = __uint_as_float(r[16 * q + j]);
+                                    finish16(ep, biasS, n0 + c0 + c + 16 * q, pix, inside, v);
+                                    stage16(rowAddr, rowSwz, c + 16 * q, ep.outF32, v);
+                                }
                             }
                         }
                     } else {
@@ -518,21 +519,23 @@ __global__ void __launch_bounds__(fwd_threads(kResident), kResident && BLOCKS !=
                 for (uint32_t c0 = 0; c0 < sh.N; c0 += 16) {
                     float v[16];
                     tmem_ld16(tAcc + c0, v);
-                    if (n0 + c0 >= ep.coutValid || !inside) continue;
-                    finish16(ep, biasS, n0 + c0, pix, inside, v);
-                    if (ep.headDst) {
-                        // the network's last layer: radiance = expm1(log1p(rgb) + residual), cropped
-                        if (h < ep.headH && w < ep.headW)
-                            for (uint32_t j = 0; j < 3; ++j)
-                                ep.headDst[3 * headAt + j] = fmaxf(expm1f(log_radiance(rgb[j]) + v[j]), 0.0f);
-                        continue;
+                    if (n0 + c0 < ep.coutValid && inside) {
+                        finish16(ep, biasS, n0 + c0, pix, inside, v);
+                        if (ep.headDst) {
+                            // the network's last layer: radiance = expm1(log1p(rgb) + residual), cropped
+                            if (h < ep.headH && w < ep.headW)
+                                for (uint32_t j = 0; j < 3; ++j)
+                                    ep.headDst[3 * headAt + j] = fmaxf(expm1f(log_radiance(rgb[j]) + v[j]), 0.0f);
+                        } else {
+                            const uint32_t nv = min(16u, ep.coutValid - n0 - c0);
+                            const size_t at = pix * ep.outStride + ep.outOffset + n0 + c0;
+                            for (uint32_t j = 0; j < nv; ++j) {
+                                if (ep.outF32) ((float*)ep.out)[at + j] = v[j];
+                                else ((__nv_bfloat16*)ep.out)[at + j] = __float2bfloat16_rn(v[j]);
+                            }
+                        }
                     }
-                    const uint32_t nv = min(16u, ep.coutValid - n0 - c0);
-                    const size_t at = pix * ep.outStride + ep.outOffset + n0 + c0;
-                    for (uint32_t j = 0; j < nv; ++j) {
-                        if (ep.outF32) ((float*)ep.out)[at + j] = v[j];
-                        else ((__nv_bfloat16*)ep.out)[at + j] = __float2bfloat16_rn(v[j]);
-                    }
+                    __syncwarp();  // (the next load is .aligned)
                 }
             }
             tc_fence_before();
@@ -545,6 +548,7 @@ __global__ void __launch_bounds__(fwd_threads(kResident), kResident && BLOCKS !=
     tc_fence_before();
     __syncthreads();
     if (threadIdx.x == 0 && *abortFlag) atomicOr(err, 1u);
+    __syncwarp();
     if (warp == 0) tmem_dealloc(tmem, sh.tmemCols);
 }
 
@@ -666,11 +670,10 @@ __global__ void __launch_bounds__(128, 1)
     }
     __syncwarp();
 
-    const bool ready = mbar_wait(accum, 0);
-    __syncwarp();
+    const bool ready = warp_wait(accum, 0) && !warp_any(*abortFlag);
     tc_fence_after();
-    if (!ready || *abortFlag) {
-        if (threadIdx.x == 0) atomicOr(err, 1u);
+    if (!ready) {
+        if (lane == 0) atomicOr(err, 1u);
     } else if (kSteps > 0) {
         // row dx * CB + ci, column co: a warp adds 32 (or 2 x 16) consecutive weights at a time
         const uint32_t row = warp * 32 + lane, dx = row / CB, ci = row % CB;
@@ -680,14 +683,17 @@ __global__ void __launch_bounds__(128, 1)
                 const uint32_t dy = j / (CA / 16), c0 = j % (CA / 16) * 16, co = co0 + c0;
                 float v[16];
                 tmem_ld16(tmem + ((warp * 32u) << 16) + dy * kCols + c0, v);
-                if (dx >= 3) continue;
-                float* o = dW + ((size_t)co * 9 + (dy0 + dy) * 3 + dx) * sh.Cin + ci0 + ci;
+                if (dx < 3) {
+                    float* o = dW + ((size_t)co * 9 + (dy0 + dy) * 3 + dx) * sh.Cin + ci0 + ci;
 #pragma unroll
-                for (uint32_t i = 0; i < 16; ++i)
-                    if (co + i < sh.coutStore) atomicAdd(o + (size_t)i * 9 * sh.Cin, v[i]);
+                    for (uint32_t i = 0; i < 16; ++i)
+                        if (co + i < sh.coutStore) atomicAdd(o + (size_t)i * 9 * sh.Cin, v[i]);
+                }
+                __syncwarp();  // (the next load is .aligned)
             }
         }
     }
+    __syncwarp();
     tc_fence_before();
     __syncthreads();
     if (warp == 1) tmem_dealloc(tmem, sh.tmemCols);

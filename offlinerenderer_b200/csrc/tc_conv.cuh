@@ -46,7 +46,11 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
         if (clock64() - t0 > (1ll << 32)) return false;
     }
 }
-// The same for a converged warp: one result for all lanes.
+// Collectives of a whole warp.  The lanes need one answer: a lane that left a loop alone
+// would leave the others waiting in the next vote, and tcgen05.ld, alloc and dealloc are
+// .aligned, undefined in a warp that has diverged.
+__device__ __forceinline__ bool warp_any(uint32_t x) { return __any_sync(0xffffffffu, x != 0); }
+// mbar_wait for a warp: one result for all lanes.
 __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity) {
     if (__all_sync(0xffffffffu, mbar_try(bar, parity))) return true;
     return __all_sync(0xffffffffu, mbar_wait(bar, parity));
