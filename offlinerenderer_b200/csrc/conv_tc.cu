@@ -53,12 +53,14 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 // across work items, so the next item's input loads while this one computes.
 //
 // Weights: kResident keeps the layer's whole weight tensor in shared memory; otherwise
-// (tap, chunk) slices stream through a second ring.
+// (tap, chunk) slices stream through a second ring.  Where all chunks of a wide input do not
+// fit beside a ring of them, the item runs chunk by chunk (kByChunk): nine taps of one
+// chunk, then its slot is free for the next, so any channel count does.
 //
 // Warps: epilogue (four or eight), input loads, MMA, weight loads.  The accumulator is
 // double-buffered in TMEM (columns [0, N) and [N, 2N)), so the epilogue of one item
-// overlaps the next one's MMAs.  K runs tap-major, then by channel, whatever the plan:
-// every output sums in the same order.
+// overlaps the next one's MMAs.  K runs tap-major, then by channel, so every output sums in
+// the same order whatever the plan; kByChunk alone runs by chunk, then tap-major.
 //
 // What bounds it, on a 1920 x 1088 frame (device time per layer, before -> now, with the
 // pools and upsamples that were passes of their own, 66 + 178 us, now in it): an M128 K16
@@ -201,7 +203,7 @@ __device__ __forceinline__ float log_radiance(float x) { return log1pf(fmaxf(x, 
 
 // BLOCKS > 0: the channel chunks of a resident layer, so that the MMA issue is straight
 // code with constant descriptor offsets (0 = sh.Cin / CHUNK at run time).
-template <int CHUNK, bool kResident, int BLOCKS>
+template <int CHUNK, bool kResident, int BLOCKS, bool kByChunk = false>
 __global__ void __launch_bounds__(fwd_threads(kResident), kResident && BLOCKS != 3 ? 2 : 1)
     k_conv_fwd(const __grid_constant__ CUtensorMap mx, const __grid_constant__ CUtensorMap mw,
                const __grid_constant__ OutMaps mo, FwdShape sh, Epilogue ep, uint32_t* err) {
@@ -316,7 +318,8 @@ __global__ void __launch_bounds__(fwd_threads(kResident), kResident && BLOCKS !=
                             break;
                         }
                         mbar_expect_tx(fullB(s), wSlice);
-                        tma_load_2d(wBase + s * wSlice, &mw, fullB(s), (int)(j * CHUNK), row);
+                        const uint32_t k = kByChunk ? j % 9 * G + j / 9 : j;  // tap * G + chunk
+                        tma_load_2d(wBase + s * wSlice, &mw, fullB(s), (int)(k * CHUNK), row);
                         ++issued;
                         if (++s == RB) {
                             s = 0;
@@ -378,6 +381,37 @@ __global__ void __launch_bounds__(fwd_threads(kResident), kResident && BLOCKS !=
                     umma_commit(accFull(buf));
                 }
                 __syncwarp();
+            } else if constexpr (kByChunk) {
+                if (leader) {
+                    bool good = true;  // (once a wait gave up: garbage sums, the error flag, no more waits)
+                    for (uint32_t g = 0; g < G; ++g) {
+                        good = good && mbar_wait(fullA(sa0), phA);
+#pragma unroll
+                        for (uint32_t tap = 0; tap < 9; ++tap) {
+                            const uint32_t shift = ((tap / 3) * kHaloW + (tap % 3)) * (kRow >> 4);
+                            good = good && mbar_wait(fullB(sb), phB);
+                            const uint64_t ad = a0 + (sa0 * (kBlock >> 4) + shift), bd = b0 + sb * (wSlice >> 4);
+#pragma unroll
+                            for (uint32_t kk = 0; kk < CHUNK / 16; ++kk)
+                                umma_bf16(acc, ad + 2 * kk, bd + 2 * kk, idesc, (tap | g | kk) ? 1u : 0u);
+                            umma_commit(emptyB(sb));
+                            if (++sb == RB) {
+                                sb = 0;
+                                phB ^= 1u;
+                            }
+                        }
+                        umma_commit(emptyA(sa0));
+                        if (++sa0 == RA) {
+                            sa0 = 0;
+                            phA ^= 1u;
+                        }
+                    }
+                    if (!good) *abortFlag = 1;
+                    umma_commit(accFull(buf));
+                }
+                __syncwarp();
+                ok = !warp_any(*abortFlag);
+                continue;  // (the leader keeps the ring positions)
             } else {
                 for (uint32_t g = 0; g < G && ok; ++g) {
                     const bool wrap = sa0 + g >= RA;
@@ -758,6 +792,7 @@ int plan_fwd(uint32_t B, uint32_t H, uint32_t W, uint32_t Cin, uint32_t N, bool 
     const uint32_t tiles = B * sh.tilesX * sh.tilesY;
     sh.nSplit = 1;
     p->resident = N <= 128 && 9 * Cin * N * 2 <= 72u * 1024u;
+    p->byChunk = false;
     if (!p->resident) {
         // at most 192 channels an item, so that the weight ring holds several slices
         while (N / sh.nSplit > 192 || N % sh.nSplit || (N / sh.nSplit) % 16)
@@ -795,6 +830,19 @@ int plan_fwd(uint32_t B, uint32_t H, uint32_t W, uint32_t Cin, uint32_t N, bool 
         while (sh.stagesA > G && need(sh.stagesA, 6) > limit) --sh.stagesA;
         sh.stagesB = 16;
         while (sh.stagesB > 2 && need(sh.stagesA, sh.stagesB) > limit) --sh.stagesB;
+        // Where the halos leave room for fewer than sixteen MMAs' weights (more than 384
+        // channels, or many 16- and 32-channel chunks), the item runs chunk by chunk with the
+        // room for weights: the MMAs waited for their slices otherwise (528 -> 64 channels at
+        // 960 x 544 1224 us with five slices, 846 by chunk; 288 -> 32 356, 195), and inputs
+        // whose chunks do not fit at all are held no other way (512 -> 128 at 1920 x 1088 1690 us).
+        const uint32_t mmas = p->chunk / 16;
+        p->byChunk = need(sh.stagesA, sh.stagesB) > limit || sh.stagesB * mmas < 16;
+        if (p->byChunk) {
+            sh.stagesA = std::min(G, 4u);
+            while (sh.stagesA > 2 && need(sh.stagesA, 16 / mmas) > limit) --sh.stagesA;
+            sh.stagesB = 16;
+            while (sh.stagesB > 2 && need(sh.stagesA, sh.stagesB) > limit) --sh.stagesB;
+        }
     }
     if (need(sh.stagesA, sh.stagesB) > limit) return 1;
     p->smem = smem_for(need(sh.stagesA, sh.stagesB), sh.tmemCols);
@@ -917,23 +965,26 @@ cudaError_t launch_fwd(const FwdPlan& p, const CUtensorMap& mx, const CUtensorMa
     lc.stream = st;
     lc.attrs = &at;
     lc.numAttrs = overlap ? 1 : 0;
-#define WRK_FWD_CASE(CHUNK, RES, BLOCKS)                                                                  \
-    if (p.chunk == CHUNK && p.resident == RES && (BLOCKS == 0 || p.shape.Cin == CHUNK * BLOCKS)) {        \
-        e = set_smem(k_conv_fwd<CHUNK, RES, BLOCKS>, p.smem);                                             \
-        if (e == cudaSuccess)                                                                             \
-            e = cudaLaunchKernelEx(&lc, k_conv_fwd<CHUNK, RES, BLOCKS>, mx, mw, mo, p.shape, ep, err);        \
-        return e != cudaSuccess ? e : cudaGetLastError();                                                 \
+#define WRK_FWD_CASE(CHUNK, RES, BLOCKS, BY)                                                                               \
+    if (p.chunk == CHUNK && p.resident == RES && p.byChunk == BY && (BLOCKS == 0 || p.shape.Cin == CHUNK * BLOCKS)) {      \
+        e = set_smem(k_conv_fwd<CHUNK, RES, BLOCKS, BY>, p.smem);                                                          \
+        if (e == cudaSuccess)                                                                                              \
+            e = cudaLaunchKernelEx(&lc, k_conv_fwd<CHUNK, RES, BLOCKS, BY>, mx, mw, mo, p.shape, ep, err);                 \
+        return e != cudaSuccess ? e : cudaGetLastError();                                                                  \
     }
-    WRK_FWD_CASE(16, true, 1)
-    WRK_FWD_CASE(32, true, 1)
-    WRK_FWD_CASE(32, true, 3)
-    WRK_FWD_CASE(64, true, 1)
-    WRK_FWD_CASE(16, true, 0)
-    WRK_FWD_CASE(32, true, 0)
-    WRK_FWD_CASE(64, true, 0)
-    WRK_FWD_CASE(16, false, 0)
-    WRK_FWD_CASE(32, false, 0)
-    WRK_FWD_CASE(64, false, 0)
+    WRK_FWD_CASE(16, true, 1, false)
+    WRK_FWD_CASE(32, true, 1, false)
+    WRK_FWD_CASE(32, true, 3, false)
+    WRK_FWD_CASE(64, true, 1, false)
+    WRK_FWD_CASE(16, true, 0, false)
+    WRK_FWD_CASE(32, true, 0, false)
+    WRK_FWD_CASE(64, true, 0, false)
+    WRK_FWD_CASE(16, false, 0, false)
+    WRK_FWD_CASE(32, false, 0, false)
+    WRK_FWD_CASE(64, false, 0, false)
+    WRK_FWD_CASE(16, false, 0, true)
+    WRK_FWD_CASE(32, false, 0, true)
+    WRK_FWD_CASE(64, false, 0, true)
 #undef WRK_FWD_CASE
     return e != cudaSuccess ? e : cudaGetLastError();
 }

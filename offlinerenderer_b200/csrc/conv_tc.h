@@ -56,6 +56,7 @@ struct FwdPlan {
     uint32_t sliceC;  // output channels per staged slice
     uint32_t smem, grid;
     bool resident;    // the whole weight tensor stays in shared memory
+    bool byChunk;     // streamed weights: an item runs chunk by chunk (its chunks do not fit together)
 };
 struct WgradPlan {
     WgradShape shape;
