@@ -794,9 +794,13 @@ int plan_fwd(uint32_t B, uint32_t H, uint32_t W, uint32_t Cin, uint32_t N, bool 
     p->resident = N <= 128 && 9 * Cin * N * 2 <= 72u * 1024u;
     p->byChunk = false;
     if (!p->resident) {
-        // at most 192 channels an item, so that the weight ring holds several slices
-        while (N / sh.nSplit > 192 || N % sh.nSplit || (N / sh.nSplit) % 16)
-            if (++sh.nSplit > N / 16) return 1;
+        // at most 192 channels an item, so that the weight ring holds several slices, where
+        // that takes four items at most; otherwise as few as an MMA's 256 channels allow
+        auto fits = [&](uint32_t most) { return N / sh.nSplit <= most && N % (16 * sh.nSplit) == 0; };
+        while (sh.nSplit <= 4 && !fits(192)) ++sh.nSplit;
+        if (!fits(192))
+            for (sh.nSplit = 1; !fits(256);)
+                if (++sh.nSplit > N / 16) return 1;
         while (tiles * sh.nSplit * 2 <= numSMs && (N / sh.nSplit) % 64 == 0) sh.nSplit *= 2;
     }
     sh.N = N / sh.nSplit;

@@ -23,6 +23,8 @@ int main() {
                         s.tmemCols >= 2 * s.N && s.tmemCols <= 512 && p.smem <= 227 * 1024 && p.grid > 0 &&
                         (2 * s.stagesA + 2 * s.stagesB + 5) * 8 + 8 <= 1024 &&  // the barriers' share
                         // all chunks of an item at once unless it runs chunk by chunk, and a ring of weights
+                        // (split further only where an image has few tiles)
+                        (s.nSplit <= 4 || z[1] < 128) &&
                         (p.byChunk ? s.stagesA >= 2 || s.stagesA == chunks : s.stagesA >= chunks) &&
                         (p.resident ? !p.byChunk : s.stagesB >= 2);
                     ++plans;

@@ -1,5 +1,5 @@
 """The forward convolution where an item's input chunks do not fit shared memory together (it
-runs chunk by chunk).  Against torch in fp64 on
+runs chunk by chunk), and where its output channels divide badly.  Against torch in fp64 on
 the same bf16-rounded operands.  A sum has 9 * Cin products in steps of 16, each step rounded
 or cut to f32 (2^-23 of partial sums that stay below the largest output), so an f32 output is
 within 9 * Cin / 16 * 2^-23 of the output scale and a bf16 store within half a bf16 ulp (2^-8
@@ -23,6 +23,8 @@ def _bf(a):
     (1, 1024, 16, 40, 48),    # the narrowest output
     (1, 528, 64, 24, 16),     # thirty-three 16-channel chunks
     (1, 544, 96, 16, 32),     # 32-channel chunks
+    (1, 544, 208, 16, 32),    # 32-channel chunks; 208 channels have no split of at most four
+    (1, 176, 208, 24, 32),    # the same where all chunks fit
     (1, 512, 5, 8, 16),       # padded output channels: element stores
     (2, 512, 128, 128, 192),  # more items than blocks: both rings wrap
 ])
