@@ -593,8 +593,9 @@ __global__ void __launch_bounds__(fwd_threads(kResident), kResident && BLOCKS !=
 // K = pixels.  M holds the taps of a row times the input channels: the operand's channel
 // groups are one pixel apart (LBO), so group dx reads the halo shifted by dx pixels (groups
 // past the third are padding and not stored), and rows of 8 pixels are 10 halo rows apart as
-// in k_conv_fwd.  N = the output channels, with an accumulator per dy.  f32 atomics into dW,
-// a warp's lanes along its input channels.
+// in k_conv_fwd.  N = the output channels, with an accumulator per dy.  Sums of a limited
+// number of tiles are added in registers; then f32 atomics into dW, a warp's lanes along
+// its input channels.
 //
 // What bounds it: a block per tap loaded both operands nine times and padded M from the 16
 // to 64 output channels of the wide layers to 128 (32 x 32 channels over 16 x 128 x 128
@@ -647,84 +648,112 @@ __global__ void __launch_bounds__(128, 1)
     grid_wait();
     const uint32_t perImg = sh.tilesX * sh.tilesY;
     const uint32_t kSteps = t1 > t0 ? t1 - t0 : 0;
+    const uint32_t idesc = idesc_bf16(CA, true, true);
+    const uint32_t layG = layout_for_row_bytes(kRowA), layX = layout_for_row_bytes(kRowB);
+    const bool leader = warp < 2 && elect_one();
+    uint32_t issued = 0, s = 0, ph = warp == 0 ? 1 : 0;  // the loading or the MMA warp's place in the ring
 
-    if (warp == 0) {
-        if (elect_one()) {
-            uint32_t issued = 0, s = 0, ph = 1;
-            for (uint32_t k = 0; k < kSteps; ++k) {
-                if (!mbar_wait(empty(s), ph)) {
+    // The block's tiles in sums of at most sh.sumTiles in TMEM (see plan_wgrad), which meet in
+    // registers: row (warp, lane), columns dy * CA + co.
+    const uint32_t rows = tmem + ((warp * 32u) << 16);  // this warp's rows of the accumulators
+    float total[ROWS * CA] = {};
+    bool ok = true;
+    for (uint32_t k0 = 0, sum = 0; ok && k0 < kSteps; k0 += sh.sumTiles, ++sum) {
+        const uint32_t k1 = min(kSteps, k0 + sh.sumTiles);
+        if (warp == 0) {
+            if (leader) {
+                // (the next sum's first tiles load while this one is read)
+                for (const uint32_t upTo = min(kSteps, k1 + S); issued < upTo; ++issued) {
+                    if (!mbar_wait(empty(s), ph)) {
+                        *abortFlag = 1;
+                        break;
+                    }
+                    const uint32_t t = t0 + issued;
+                    const uint32_t b = t / perImg, rem = t % perImg;
+                    const int h0 = (int)((rem / sh.tilesX) * kHTileH), w0 = (int)((rem % sh.tilesX) * kHTileW);
+                    mbar_expect_tx(full(s), kHalo * kRowB + kTileP * kRowA);
+                    const uint32_t sa = base + s * kStage;
+                    tma_load_4d(sa, &mx, full(s), (int)ci0, w0 - 1, h0 - 1 + (int)dy0, (int)b);
+                    tma_load_4d(sa + kHaloBytes, &mg, full(s), (int)co0, w0, h0, (int)b);
+                    if (++s == S) {
+                        s = 0;
+                        ph ^= 1u;
+                    }
+                }
+            }
+        } else if (warp == 1) {
+            for (uint32_t k = k0; k < k1; ++k) {
+                if (!warp_wait(full(s), ph)) {
                     *abortFlag = 1;
                     break;
                 }
-                const uint32_t t = t0 + k;
-                const uint32_t b = t / perImg, rem = t % perImg;
-                const int h0 = (int)((rem / sh.tilesX) * kHTileH), w0 = (int)((rem % sh.tilesX) * kHTileW);
-                mbar_expect_tx(full(s), kHalo * kRowB + kTileP * kRowA);
-                const uint32_t sa = base + s * kStage;
-                tma_load_4d(sa, &mx, full(s), (int)ci0, w0 - 1, h0 - 1 + (int)dy0, (int)b);
-                tma_load_4d(sa + kHaloBytes, &mg, full(s), (int)co0, w0, h0, (int)b);
-                ++issued;
+                const uint32_t b0 = base + s * kStage;
+                const uint64_t xd = sdesc(b0, kRowB, kHaloW * kRowB, layX), gd = sdesc(b0 + kHaloBytes, 0, 8 * kRowA, layG);
+                if (leader) {
+#pragma unroll
+                    for (uint32_t kk = 0; kk < kTileP / 16; ++kk)
+#pragma unroll
+                        for (uint32_t dy = 0; dy < ROWS; ++dy)  // 16 pixels: two rows of the tile
+                            umma_bf16(tmem + dy * kCols, xd + (2 * kk + dy) * (kHaloW * kRowB / 16), gd + kk * kRowA, idesc,
+                                      (k - k0 | kk) ? 1u : 0u);
+                    umma_commit(empty(s));
+                }
+                __syncwarp();
                 if (++s == S) {
                     s = 0;
                     ph ^= 1u;
                 }
             }
-            if (*abortFlag) {
-                for (uint32_t k = issued > S ? issued - S : 0; k < issued; ++k) mbar_wait(full(k % S), (k / S) & 1u);
-            }
+            if (leader) umma_commit(accum);
         }
-    } else if (warp == 1) {
-        const bool leader = elect_one();
-        const uint32_t idesc = idesc_bf16(CA, true, true);
-        const uint32_t layG = layout_for_row_bytes(kRowA), layX = layout_for_row_bytes(kRowB);
-        uint32_t s = 0, ph = 0;
-        for (uint32_t k = 0; k < kSteps; ++k) {
-            if (!warp_wait(full(s), ph)) {
-                *abortFlag = 1;
-                break;
-            }
-            const uint32_t b0 = base + s * kStage;
-            const uint64_t xd = sdesc(b0, kRowB, kHaloW * kRowB, layX), gd = sdesc(b0 + kHaloBytes, 0, 8 * kRowA, layG);
-            if (leader) {
-#pragma unroll
-                for (uint32_t kk = 0; kk < kTileP / 16; ++kk)
-#pragma unroll
-                    for (uint32_t dy = 0; dy < ROWS; ++dy)  // 16 pixels: two rows of the tile
-                        umma_bf16(tmem + dy * kCols, xd + (2 * kk + dy) * (kHaloW * kRowB / 16), gd + kk * kRowA, idesc,
-                                  (k | kk) ? 1u : 0u);
-                umma_commit(empty(s));
-            }
-            __syncwarp();
-            if (++s == S) {
-                s = 0;
-                ph ^= 1u;
-            }
-        }
-        if (leader) umma_commit(accum);
-    }
-    __syncwarp();
+        __syncwarp();
 
-    const bool ready = warp_wait(accum, 0) && !warp_any(*abortFlag);
-    tc_fence_after();
-    if (!ready) {
-        if (lane == 0) atomicOr(err, 1u);
-    } else if (kSteps > 0) {
-        // row dx * CB + ci, column co: a warp adds 32 (or 2 x 16) consecutive weights at a time
-        const uint32_t row = warp * 32 + lane, dx = row / CB, ci = row % CB;
-        if (warp * 32 < 3 * CB) {
-#pragma unroll 1
-            for (uint32_t j = 0; j < ROWS * CA / 16; ++j) {
-                const uint32_t dy = j / (CA / 16), c0 = j % (CA / 16) * 16, co = co0 + c0;
-                float v[16];
-                tmem_ld16(tmem + ((warp * 32u) << 16) + dy * kCols + c0, v);
-                if (dx < 3) {
-                    float* o = dW + ((size_t)co * 9 + (dy0 + dy) * 3 + dx) * sh.Cin + ci0 + ci;
+        const bool ready = warp_wait(accum, sum & 1u) && !warp_any(*abortFlag);
+        tc_fence_after();
+        if (!ready) {
+            if (lane == 0) atomicOr(err, 1u);
+        } else if (warp * 32 < 3 * CB && sh.sumTiles < sh.tilesPerCta) {
+            // one of several sums: added to the others, which the last one leaves in its columns
 #pragma unroll
-                    for (uint32_t i = 0; i < 16; ++i)
-                        if (co + i < sh.coutStore) atomicAdd(o + (size_t)i * 9 * sh.Cin, v[i]);
-                }
-                __syncwarp();  // (the next load is .aligned)
+            for (uint32_t j = 0; j < ROWS * CA / 16; ++j) {
+                float v[16];
+                tmem_ld16(rows + j / (CA / 16) * kCols + j % (CA / 16) * 16, v);
+#pragma unroll
+                for (uint32_t i = 0; i < 16; ++i) total[16 * j + i] += v[i];
             }
+            if (k1 == kSteps) {
+#pragma unroll
+                for (uint32_t j = 0; j < ROWS * CA / 16; ++j)
+                    tmem_st16(rows + j / (CA / 16) * kCols + j % (CA / 16) * 16, total + 16 * j);
+                tmem_st_wait();
+            }
+        }
+        tc_fence_before();
+        ok = !__syncthreads_or(!ready);
+        tc_fence_after();
+    }
+    if (ok && kSteps > 0 && warp * 32 < 3 * CB) {
+        // row dx * CB + ci, column co: a warp adds 32 (or 2 x 16) consecutive weights at a time
+        // (a short loop: unrolled over registers it ran from cold instruction memory, 2.4 us)
+        const uint32_t row = warp * 32 + lane, dx = row / CB, ci = row % CB;
+#pragma unroll 1
+        for (uint32_t j = 0; j < ROWS * CA / 16; ++j) {
+            const uint32_t dy = j / (CA / 16), c0 = j % (CA / 16) * 16, co = co0 + c0;
+            float v[16];
+            tmem_ld16(rows + dy * kCols + c0, v);
+            if (dx < 3) {
+                float* o = dW + ((size_t)co * 9 + (dy0 + dy) * 3 + dx) * sh.Cin + ci0 + ci;
+#pragma unroll
+                for (uint32_t i = 0; i < 16; ++i)
+                    if (co + i < sh.coutStore) atomicAdd(o + (size_t)i * 9 * sh.Cin, v[i]);
+            }
+            __syncwarp();  // (the next load is .aligned)
+        }
+    }
+    // a block that gave up lets its copies in flight land first (bounded)
+    if (warp == 0 && leader) {
+        if (*abortFlag) {
+            for (uint32_t k = issued > S ? issued - S : 0; k < issued; ++k) mbar_wait(full(k % S), (k / S) & 1u);
         }
     }
     __syncwarp();
@@ -945,6 +974,17 @@ int plan_wgrad(uint32_t B, uint32_t H, uint32_t W, uint32_t Cin, uint32_t Cout, 
     sh.tilesPerCta = (sh.tilesTotal + splits - 1) / splits;
     splits = (sh.tilesTotal + sh.tilesPerCta - 1) / sh.tilesPerCta;
     p->grid = dim3(splits, ciBlocks, coBlocks);
+    // A sum in TMEM is cut to f32 at every step, so its error grows with its length: a sum
+    // takes at most the tiles that two blocks an SM, of one tap, 128 output and 256 input
+    // channels each, would have (256 -> 256 channels over 16 x 16 x 16 pixels: 4.5e-7 from
+    // 64-bit sums with all 4 tiles of a block in one sum, 2.3e-7 with 2).  A block of more
+    // reads several sums and adds them in registers: more blocks would each add all their
+    // weights to memory (a training pass of 16 x 128 x 128 858 us without the limit, 862 with
+    // it, 874 with blocks of that length).
+    const uint32_t cells = 9 * ((Cin + 255) / 256) * ((Cout + 127) / 128);
+    const uint32_t parts = std::min((2 * numSMs + cells - 1) / cells, sh.tilesTotal);
+    const uint32_t most = (sh.tilesTotal + parts - 1) / parts, sums = (sh.tilesPerCta + most - 1) / most;
+    sh.sumTiles = (sh.tilesPerCta + sums - 1) / sums;
     return 0;
 }
 

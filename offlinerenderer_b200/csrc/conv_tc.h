@@ -43,6 +43,7 @@ struct WgradShape {
     uint32_t Cin;
     uint32_t coutStore;  // rows of dW that exist (<= the channels of G)
     uint32_t tilesX, tilesY, tilesTotal, tilesPerCta;
+    uint32_t sumTiles;    // tiles of one sum in TMEM
     uint32_t stages, tmemCols;
 };
 

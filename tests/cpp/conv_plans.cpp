@@ -1,6 +1,8 @@
-// Plans of the 3x3 convolution for every channel count the entry point takes, without a GPU:
-// one line "Cin Cout f32 H W B rc" per plan that is refused or that does not hold together.
+// Plans of the 3x3 convolution and of its weight gradient for every channel count the entry
+// points take, without a GPU: one line "Cin Cout f32 H W B rc" (f32 = 2: weight gradient) per
+// plan that is refused or that does not hold together.
 // Built and run by tests/test_conv_plans.py.
+#include <algorithm>
 #include <cstdio>
 
 #include "conv_tc.h"
@@ -31,5 +33,24 @@ int main() {
                     byChunk += p.byChunk;
                     if (!ok) std::printf("%u %u %d %u %u %u %d\n", cin, n, f32, z[1], z[2], z[0], rc);
                 }
+    for (uint32_t cin = 16; cin <= 512; cin += cin < 256 ? 16 : 32)
+        for (uint32_t cout = 16; cout <= 512; cout += 16)
+            for (auto& z : sizes) {
+                WgradPlan p{};
+                const int rc = plan_wgrad(z[0], z[1], z[2], cin, cout, 148, &p);
+                const WgradShape& s = p.shape;
+                const uint32_t tiles = z[0] * (z[2] / 8) * ((z[1] + 15) / 16);
+                // the longest sum a tensor-memory accumulator may take: the tiles that two
+                // blocks per SM of one tap, 128 output and 256 input channels each, would share
+                const uint32_t cells = 9 * ((cin + 255) / 256) * ((cout + 127) / 128);
+                const uint32_t parts = std::min((2 * 148 + cells - 1) / cells, tiles);
+                const bool ok = rc == 0 && s.tilesTotal == tiles && p.grid.x * s.tilesPerCta >= tiles &&
+                                (p.grid.x - 1) * s.tilesPerCta < tiles && p.grid.y * p.cb >= cin &&
+                                p.grid.z * p.rows / 3 * p.ca >= cout && p.smem <= 227 * 1024 && s.stages >= 2 &&
+                                p.rows * ((p.ca + 31) / 32 * 32) <= s.tmemCols && s.sumTiles > 0 &&
+                                s.sumTiles <= (tiles + parts - 1) / parts;
+                ++plans;
+                if (!ok) std::printf("%u %u 2 %u %u %u %d\n", cin, cout, z[1], z[2], z[0], rc);
+            }
     std::printf("plans %ld by chunk %ld\n", plans, byChunk);
 }
