@@ -741,7 +741,7 @@ __global__ void __launch_bounds__(128, 1)
             const uint32_t dy = j / (CA / 16), c0 = j % (CA / 16) * 16, co = co0 + c0;
             float v[16];
             tmem_ld16(rows + dy * kCols + c0, v);
-            if (dx < 3) {
+            if (dx < 3 && ci0 + ci < sh.Cin) {
                 float* o = dW + ((size_t)co * 9 + (dy0 + dy) * 3 + dx) * sh.Cin + ci0 + ci;
 #pragma unroll
                 for (uint32_t i = 0; i < 16; ++i)
@@ -953,8 +953,11 @@ int plan_wgrad(uint32_t B, uint32_t H, uint32_t W, uint32_t Cin, uint32_t Cout, 
     sh.tilesX = W / kHTileW;
     sh.tilesY = (H + kHTileH - 1) / kHTileH;
     sh.tilesTotal = B * sh.tilesX * sh.tilesY;
-    p->ca = chunk_for(Cout);
-    p->cb = Cin % 32 == 0 ? 32 : 16;
+    // Widths by what fills an MMA, not by what divides the channels: it takes the same time up
+    // to N = 64, and M holds three taps of 32 input channels; channels past the last are loaded
+    // as zeros and not stored (240 -> 240 over 4 x 64 x 64 in blocks of 16 x 16 171 us, here 34).
+    p->ca = Cout <= 16 ? 16 : Cout <= 32 ? 32 : 64;
+    p->cb = Cin <= 16 ? 16 : 32;
     // One wave of blocks, two an SM: one covers the other's start and atomics (one an SM:
     // 36 us for 96 -> 32 channels at full width, 32 with two), and a second wave would cost
     // a start (256 -> 256 channels at an eighth: 17 us, 24 with twice the blocks).  The
@@ -964,7 +967,7 @@ int plan_wgrad(uint32_t B, uint32_t H, uint32_t W, uint32_t Cin, uint32_t Cout, 
     // few that a block's sums in TMEM, which truncate, grow longer than they were, so four
     // blocks share an SM there.
     p->rows = p->ca == 64 ? 3 : 1;
-    const uint32_t ciBlocks = Cin / p->cb, coBlocks = Cout / p->ca * (3 / p->rows);
+    const uint32_t ciBlocks = (Cin + p->cb - 1) / p->cb, coBlocks = (Cout + p->ca - 1) / p->ca * (3 / p->rows);
     const uint32_t perSM = p->rows == 1 && ciBlocks > 1 ? 4 : 2;
     sh.tmemCols = 512 / perSM;  // of which rows * wgrad_cols(ca) are used: 192 of 256, or 32
     const uint32_t stage = round_up(wgrad_halo_rows(p->rows) * kHaloW * p->cb * 2, 1024) + kTileP * p->ca * 2;

@@ -48,7 +48,9 @@ int main() {
                                 (p.grid.x - 1) * s.tilesPerCta < tiles && p.grid.y * p.cb >= cin &&
                                 p.grid.z * p.rows / 3 * p.ca >= cout && p.smem <= 227 * 1024 && s.stages >= 2 &&
                                 p.rows * ((p.ca + 31) / 32 * 32) <= s.tmemCols && s.sumTiles > 0 &&
-                                s.sumTiles <= (tiles + parts - 1) / parts;
+                                s.sumTiles <= (tiles + parts - 1) / parts &&
+                                // no more blocks of channels than an MMA's rows and columns call for
+                                p.grid.y == (cin + 31) / 32 && p.grid.z * p.rows / 3 == (cout <= 32 ? 1 : (cout + 63) / 64);
                 ++plans;
                 if (!ok) std::printf("%u %u 2 %u %u %u %d\n", cin, cout, z[1], z[2], z[0], rc);
             }
