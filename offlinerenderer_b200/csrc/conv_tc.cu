@@ -602,6 +602,22 @@ __global__ void __launch_bounds__(fwd_threads(kResident), kResident && BLOCKS !=
 // pixels 63 us, 31 of them MMAs; L2 at 4.8 TB/s).  Now 16 us, 10 of them MMAs, the rest
 // its start and its atomics; 192 -> 64 channels at half the width 37 -> 28 us, 256 -> 256 at
 // an eighth 25 -> 17 us; a training pass at 16 x 128 x 128 1106 -> 850 us.
+
+// The 4 x 4 transpose of four lanes' (lane & ~3 on) four values each.
+__device__ __forceinline__ void transpose4(float* v, uint32_t lane) {
+#pragma unroll
+    for (uint32_t bit = 1; bit < 4; bit <<= 1) {
+        const bool hi = lane & bit;
+#pragma unroll
+        for (uint32_t k = 0; k < 4; ++k) {
+            if (k & bit) continue;
+            const float got = __shfl_xor_sync(0xffffffffu, hi ? v[k] : v[k + bit], bit);
+            if (hi) v[k] = got;
+            else v[k + bit] = got;
+        }
+    }
+}
+
 template <int CA, int CB, int ROWS>
 __global__ void __launch_bounds__(128, 1)
     k_conv_wgrad(const __grid_constant__ CUtensorMap mg, const __grid_constant__ CUtensorMap mx, WgradShape sh,
@@ -733,16 +749,29 @@ __global__ void __launch_bounds__(128, 1)
         tc_fence_after();
     }
     if (ok && kSteps > 0 && warp * 32 < 3 * CB) {
-        // row dx * CB + ci, column co: a warp adds 32 (or 2 x 16) consecutive weights at a time
-        // (a short loop: unrolled over registers it ran from cold instruction memory, 2.4 us)
-        const uint32_t row = warp * 32 + lane, dx = row / CB, ci = row % CB;
+        // row dx * CB + ci, column co (a short loop: unrolled over registers it ran from cold
+        // instruction memory, 2.4 us)
+        const uint32_t row = warp * 32 + lane, dx = row / CB, ci = ci0 + row % CB;
+        const bool vec = ((uintptr_t)dW & 15u) == 0, mine = dx < 3 && ci < sh.Cin;
 #pragma unroll 1
         for (uint32_t j = 0; j < ROWS * CA / 16; ++j) {
             const uint32_t dy = j / (CA / 16), c0 = j % (CA / 16) * 16, co = co0 + c0;
             float v[16];
             tmem_ld16(rows + dy * kCols + c0, v);
-            if (dx < 3 && ci0 + ci < sh.Cin) {
-                float* o = dW + ((size_t)co * 9 + (dy0 + dy) * 3 + dx) * sh.Cin + ci0 + ci;
+            if (vec) {
+                // four lanes' inputs of one output channel meet in a lane, an atomic per 16 bytes:
+                // 64 -> 64 channels over 16 x 8 pixels 10.1 -> 8.3 us, a training pass of
+                // 16 x 128 x 128 862 -> 846
+#pragma unroll
+                for (uint32_t i = 0; i < 16; i += 4) {
+                    transpose4(v + i, lane);
+                    const uint32_t c = co + i + (lane & 3u);
+                    if (mine && c < sh.coutStore)
+                        atomicAdd((float4*)(dW + ((size_t)c * 9 + (dy0 + dy) * 3 + dx) * sh.Cin + (ci & ~3u)),
+                                  make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]));
+                }
+            } else if (mine) {
+                float* o = dW + ((size_t)co * 9 + (dy0 + dy) * 3 + dx) * sh.Cin + ci;
 #pragma unroll
                 for (uint32_t i = 0; i < 16; ++i)
                     if (co + i < sh.coutStore) atomicAdd(o + (size_t)i * 9 * sh.Cin, v[i]);
@@ -965,11 +994,14 @@ int plan_wgrad(uint32_t B, uint32_t H, uint32_t W, uint32_t Cin, uint32_t Cout, 
     // its own blocks: a third of the splits' atomics for G loaded three times (a training
     // pass 862 -> 850 us); with several blocks of input channels their splits would be so
     // few that a block's sums in TMEM, which truncate, grow longer than they were, so four
-    // blocks share an SM there.
-    p->rows = p->ca == 64 ? 3 : 1;
-    const uint32_t ciBlocks = (Cin + p->cb - 1) / p->cb, coBlocks = (Cout + p->ca - 1) / p->ca * (3 / p->rows);
+    // blocks share an SM there.  So do narrow gradients of a few tiles, whose blocks of all
+    // taps would leave SMs idle (64 -> 64 channels over 16 x 8 pixels 8.3 us, 5.0 with a row
+    // a block).
+    const uint32_t ciBlocks = (Cin + p->cb - 1) / p->cb;
+    p->rows = p->ca == 64 && ciBlocks * ((Cout + 63) / 64) * sh.tilesTotal >= numSMs ? 3 : 1;
+    const uint32_t coBlocks = (Cout + p->ca - 1) / p->ca * (3 / p->rows);
     const uint32_t perSM = p->rows == 1 && ciBlocks > 1 ? 4 : 2;
-    sh.tmemCols = 512 / perSM;  // of which rows * wgrad_cols(ca) are used: 192 of 256, or 32
+    sh.tmemCols = 512 / perSM;  // of which rows * wgrad_cols(ca) are used: 192 of 256, or 32 or 64
     const uint32_t stage = round_up(wgrad_halo_rows(p->rows) * kHaloW * p->cb * 2, 1024) + kTileP * p->ca * 2;
     sh.stages = std::min(6u, (224u * 1024u / perSM - 2048u) / stage);
     p->smem = smem_for(sh.stages * stage + (2 * sh.stages + 1) * 8 + 16 + 1024, sh.tmemCols);
@@ -1058,6 +1090,8 @@ cudaError_t launch_wgrad(const WgradPlan& p, const CUtensorMap& mg, const CUtens
     }
     WRK_WGRAD_CASE(64, 32, 3)
     WRK_WGRAD_CASE(64, 16, 3)
+    WRK_WGRAD_CASE(64, 32, 1)
+    WRK_WGRAD_CASE(64, 16, 1)
     WRK_WGRAD_CASE(32, 32, 1)
     WRK_WGRAD_CASE(32, 16, 1)
     WRK_WGRAD_CASE(16, 32, 1)

@@ -49,6 +49,8 @@ int main() {
                                 p.grid.z * p.rows / 3 * p.ca >= cout && p.smem <= 227 * 1024 && s.stages >= 2 &&
                                 p.rows * ((p.ca + 31) / 32 * 32) <= s.tmemCols && s.sumTiles > 0 &&
                                 s.sumTiles <= (tiles + parts - 1) / parts &&
+                                // a row of taps a block where whole blocks would leave SMs idle
+                                (p.ca == 64 && ((cin + 31) / 32) * ((cout + 63) / 64) * tiles >= 148 ? p.rows == 3 : p.rows == 1) &&
                                 // no more blocks of channels than an MMA's rows and columns call for
                                 p.grid.y == (cin + 31) / 32 && p.grid.z * p.rows / 3 == (cout <= 32 ? 1 : (cout + 63) / 64);
                 ++plans;

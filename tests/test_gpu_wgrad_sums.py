@@ -19,12 +19,18 @@ pytestmark = pytest.mark.gpu
     (8, 128, 128, 64, 240),
     (3, 72, 80, 96, 96),
     (1, 256, 256, 256, 16),
+    (4, 64, 128, 16, 64),     # 16 input channels, all taps a block
+    (1, 24, 48, 16, 64),      # and a row of taps a block
 ])
 def test_several_sums(gpu, b, h, w, cin, cout):
     rng = np.random.default_rng(cin * 5 + cout + h)
     x = rng.random((b, h, w, cin)).astype(np.float32)
     g = rng.random((b, h, w, cout)).astype(np.float32)
-    dw = gpu.conv3x3_wgrad(g, x)
+    _check(gpu.conv3x3_wgrad(g, x), x, g)
+
+
+def _check(dw, x, g):
+    (b, h, w, cin), cout = x.shape, g.shape[3]
     bf = lambda a: torch.tensor(a, device="cuda").to(torch.bfloat16).to(torch.float64)
     xp, gf = torch.nn.functional.pad(bf(x), (0, 0, 1, 1, 1, 1)), bf(g).reshape(-1, cout)
     ref = torch.stack([torch.stack([gf.T @ xp[:, dy:dy + h, dx:dx + w].reshape(-1, cin) for dx in range(3)], 1)
@@ -36,3 +42,18 @@ def test_several_sums(gpu, b, h, w, cin, cout):
     longest = -(-tiles // parts)
     tol = 8 * longest / 2 * 2.0 ** -22 + -(-tiles // longest) * 2 * 2.0 ** -24
     assert np.all(np.abs(dw - ref) <= tol * ref)
+
+
+def test_gradient_at_any_float_address(gpu):
+    """The 16-byte atomics are for gradients at a multiple of 16 bytes; others take 4-byte ones."""
+    rng = np.random.default_rng(2)
+    b, h, w, cin, cout = 1, 16, 32, 48, 80
+    x = rng.random((b, h, w, cin)).astype(np.float32)
+    g = rng.random((b, h, w, cout)).astype(np.float32)
+    dx, dg = (torch.tensor(a, device="cuda").to(torch.bfloat16) for a in (x, g))
+    buf = torch.zeros(cout * 9 * cin + 2, device="cuda")
+    torch.cuda.synchronize()
+    assert gpu.lib().wrk_conv3x3_wgrad(dg.data_ptr(), dx.data_ptr(), b, h, w, cin, cout, buf.data_ptr() + 4) == 0
+    out = buf.cpu().numpy()
+    assert out[0] == 0.0 and out[-1] == 0.0
+    _check(out[1:-1].reshape(cout, 3, 3, cin), x, g)
