@@ -12,7 +12,8 @@
 //                2x2 average pool, the nearest 2x upsample (four stores) or the network's
 //                output image, so those take no passes of their own.
 // k_conv_wgrad -- weight gradient dW[co][tap][ci] = sum_p G[p][co] X[p+tap][ci]:
-//                M = 3 taps x input channels (128 rows), N = output channels, K = pixels;
+//                M = 3 taps x input channels (128 rows; or 128 input channels of one tap),
+//                N = output channels, K = pixels;
 //                both operands channel-contiguous (MN-major), the taps are descriptors into
 //                one halo.  Split over pixel ranges, f32 atomics into dW.
 #include <cuda.h>
@@ -597,11 +598,16 @@ __global__ void __launch_bounds__(fwd_threads(kResident), kResident && BLOCKS !=
 // number of tiles are added in registers; then f32 atomics into dW, a warp's lanes along
 // its input channels.
 //
+// kWide (CA = CB = 128): M is 128 input channels instead and a row's three taps are three
+// accumulators, so M is full and N = 128 takes 94 cycles where two of 64 take 110-120; for wide
+// layers over many pixels, which the MMAs bound (plan_wgrad): 512 -> 512 channels over 240 x 136
+// pixels 196 us in blocks of 32 x 64 channels, 120 so; 161 with a block per tap.
+//
 // What bounds it: a block per tap loaded both operands nine times and padded M from the 16
 // to 64 output channels of the wide layers to 128 (32 x 32 channels over 16 x 128 x 128
-// pixels 63 us, 31 of them MMAs; L2 at 4.8 TB/s).  Now 16 us, 10 of them MMAs, the rest
-// its start and its atomics; 192 -> 64 channels at half the width 37 -> 28 us, 256 -> 256 at
-// an eighth 25 -> 17 us; a training pass at 16 x 128 x 128 1106 -> 850 us.
+// pixels 63 us, 31 of them MMAs; L2 at 4.8 TB/s).  Now 14 us, 10 of them MMAs, the rest
+// its start and its atomics; 192 -> 64 channels at half the width 37 -> 25 us, 256 -> 256 at
+// an eighth 25 -> 15 us; a training pass at 16 x 128 x 128 1106 -> 846 us.
 
 // The 4 x 4 transpose of four lanes' (lane & ~3 on) four values each.
 __device__ __forceinline__ void transpose4(float* v, uint32_t lane) {
@@ -624,10 +630,13 @@ __global__ void __launch_bounds__(128, 1)
                   float* dW, uint32_t* err) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    constexpr uint32_t kRowA = CA * 2, kRowB = CB * 2;
-    constexpr uint32_t kHalo = wgrad_halo_rows(ROWS) * kHaloW, kHaloBytes = round_up(kHalo * kRowB, 1024), kStage = kHaloBytes + kTileP * kRowA;
-    constexpr uint32_t kCols = wgrad_cols(CA);
-    static_assert(ROWS * kCols <= (ROWS == 1 ? 128 : 256), "the plan's TMEM columns");
+    constexpr bool kWide = CB == 128;
+    // channels are loaded in groups of at most 64, one after the other
+    constexpr uint32_t kGroupsA = (CA + 63) / 64, kGroupsB = (CB + 63) / 64, kRowA = CA / kGroupsA * 2, kRowB = CB / kGroupsB * 2;
+    constexpr uint32_t kHalo = wgrad_halo_rows(ROWS) * kHaloW, kHaloBytes = round_up(kHalo * kRowB, 1024), kGBytes = kTileP * kRowA;
+    constexpr uint32_t kStage = kGroupsB * kHaloBytes + kGroupsA * kGBytes;
+    constexpr uint32_t kCols = wgrad_cols(CA), kAccs = kWide ? 3 : ROWS;
+    static_assert(kAccs * kCols <= (kWide ? 512 : ROWS == 1 ? 128 : 256), "the plan's TMEM columns");
     const uint32_t S = sh.stages;
     uint64_t* bars = (uint64_t*)(smem + S * kStage);
     uint32_t* tmemSlot = (uint32_t*)(bars + 2 * S + 1);
@@ -672,7 +681,7 @@ __global__ void __launch_bounds__(128, 1)
     // The block's tiles in sums of at most sh.sumTiles in TMEM (see plan_wgrad), which meet in
     // registers: row (warp, lane), columns dy * CA + co.
     const uint32_t rows = tmem + ((warp * 32u) << 16);  // this warp's rows of the accumulators
-    float total[ROWS * CA] = {};
+    float total[kWide ? 1 : ROWS * CA] = {};
     bool ok = true;
     for (uint32_t k0 = 0, sum = 0; ok && k0 < kSteps; k0 += sh.sumTiles, ++sum) {
         const uint32_t k1 = min(kSteps, k0 + sh.sumTiles);
@@ -687,10 +696,14 @@ __global__ void __launch_bounds__(128, 1)
                     const uint32_t t = t0 + issued;
                     const uint32_t b = t / perImg, rem = t % perImg;
                     const int h0 = (int)((rem / sh.tilesX) * kHTileH), w0 = (int)((rem % sh.tilesX) * kHTileW);
-                    mbar_expect_tx(full(s), kHalo * kRowB + kTileP * kRowA);
+                    mbar_expect_tx(full(s), kGroupsB * kHalo * kRowB + kGroupsA * kGBytes);
                     const uint32_t sa = base + s * kStage;
-                    tma_load_4d(sa, &mx, full(s), (int)ci0, w0 - 1, h0 - 1 + (int)dy0, (int)b);
-                    tma_load_4d(sa + kHaloBytes, &mg, full(s), (int)co0, w0, h0, (int)b);
+#pragma unroll
+                    for (uint32_t g = 0; g < kGroupsB; ++g)
+                        tma_load_4d(sa + g * kHaloBytes, &mx, full(s), (int)(ci0 + 64 * g), w0 - 1, h0 - 1 + (int)dy0, (int)b);
+#pragma unroll
+                    for (uint32_t g = 0; g < kGroupsA; ++g)
+                        tma_load_4d(sa + kGroupsB * kHaloBytes + g * kGBytes, &mg, full(s), (int)(co0 + 64 * g), w0, h0, (int)b);
                     if (++s == S) {
                         s = 0;
                         ph ^= 1u;
@@ -704,14 +717,16 @@ __global__ void __launch_bounds__(128, 1)
                     break;
                 }
                 const uint32_t b0 = base + s * kStage;
-                const uint64_t xd = sdesc(b0, kRowB, kHaloW * kRowB, layX), gd = sdesc(b0 + kHaloBytes, 0, 8 * kRowA, layG);
+                const uint64_t xd = sdesc(b0, kWide ? kHaloBytes : kRowB, kHaloW * kRowB, layX);
+                const uint64_t gd = sdesc(b0 + kGroupsB * kHaloBytes, kGroupsA > 1 ? kGBytes : 0, 8 * kRowA, layG);
                 if (leader) {
 #pragma unroll
                     for (uint32_t kk = 0; kk < kTileP / 16; ++kk)
 #pragma unroll
-                        for (uint32_t dy = 0; dy < ROWS; ++dy)  // 16 pixels: two rows of the tile
-                            umma_bf16(tmem + dy * kCols, xd + (2 * kk + dy) * (kHaloW * kRowB / 16), gd + kk * kRowA, idesc,
-                                      (k - k0 | kk) ? 1u : 0u);
+                        for (uint32_t a = 0; a < kAccs; ++a)  // 16 pixels: two rows of the tile; a: dy, or dx of kWide
+                            umma_bf16(tmem + a * kCols,
+                                      xd + ((2 * kk + (kWide ? 0 : a)) * kHaloW + (kWide ? a : 0)) * (kRowB / 16),
+                                      gd + kk * kRowA, idesc, (k - k0 | kk) ? 1u : 0u);
                     umma_commit(empty(s));
                 }
                 __syncwarp();
@@ -728,20 +743,22 @@ __global__ void __launch_bounds__(128, 1)
         tc_fence_after();
         if (!ready) {
             if (lane == 0) atomicOr(err, 1u);
-        } else if (warp * 32 < 3 * CB && sh.sumTiles < sh.tilesPerCta) {
+        } else if constexpr (!kWide) {
             // one of several sums: added to the others, which the last one leaves in its columns
+            if (warp * 32 < 3 * CB && sh.sumTiles < sh.tilesPerCta) {
 #pragma unroll
-            for (uint32_t j = 0; j < ROWS * CA / 16; ++j) {
-                float v[16];
-                tmem_ld16(rows + j / (CA / 16) * kCols + j % (CA / 16) * 16, v);
+                for (uint32_t j = 0; j < ROWS * CA / 16; ++j) {
+                    float v[16];
+                    tmem_ld16(rows + j / (CA / 16) * kCols + j % (CA / 16) * 16, v);
 #pragma unroll
-                for (uint32_t i = 0; i < 16; ++i) total[16 * j + i] += v[i];
-            }
-            if (k1 == kSteps) {
+                    for (uint32_t i = 0; i < 16; ++i) total[16 * j + i] += v[i];
+                }
+                if (k1 == kSteps) {
 #pragma unroll
-                for (uint32_t j = 0; j < ROWS * CA / 16; ++j)
-                    tmem_st16(rows + j / (CA / 16) * kCols + j % (CA / 16) * 16, total + 16 * j);
-                tmem_st_wait();
+                    for (uint32_t j = 0; j < ROWS * CA / 16; ++j)
+                        tmem_st16(rows + j / (CA / 16) * kCols + j % (CA / 16) * 16, total + 16 * j);
+                    tmem_st_wait();
+                }
             }
         }
         tc_fence_before();
@@ -749,15 +766,16 @@ __global__ void __launch_bounds__(128, 1)
         tc_fence_after();
     }
     if (ok && kSteps > 0 && warp * 32 < 3 * CB) {
-        // row dx * CB + ci, column co (a short loop: unrolled over registers it ran from cold
-        // instruction memory, 2.4 us)
-        const uint32_t row = warp * 32 + lane, dx = row / CB, ci = ci0 + row % CB;
-        const bool vec = ((uintptr_t)dW & 15u) == 0, mine = dx < 3 && ci < sh.Cin;
+        // row dx * CB + ci, column co, of accumulator dy (kWide: row ci of accumulator dx); a
+        // short loop: unrolled over registers it ran from cold instruction memory, 2.4 us
+        const uint32_t row = warp * 32 + lane, rowDx = row / CB, ci = ci0 + row % CB;
+        const bool vec = ((uintptr_t)dW & 15u) == 0, mine = rowDx < 3 && ci < sh.Cin;
 #pragma unroll 1
-        for (uint32_t j = 0; j < ROWS * CA / 16; ++j) {
-            const uint32_t dy = j / (CA / 16), c0 = j % (CA / 16) * 16, co = co0 + c0;
+        for (uint32_t j = 0; j < kAccs * CA / 16; ++j) {
+            const uint32_t acc = j / (CA / 16), c0 = j % (CA / 16) * 16, co = co0 + c0;
+            const uint32_t tap = kWide ? dy0 * 3 + acc : (dy0 + acc) * 3 + rowDx;
             float v[16];
-            tmem_ld16(rows + dy * kCols + c0, v);
+            tmem_ld16(rows + acc * kCols + c0, v);
             if (vec) {
                 // four lanes' inputs of one output channel meet in a lane, an atomic per 16 bytes:
                 // 64 -> 64 channels over 16 x 8 pixels 10.1 -> 8.3 us, a training pass of
@@ -767,11 +785,11 @@ __global__ void __launch_bounds__(128, 1)
                     transpose4(v + i, lane);
                     const uint32_t c = co + i + (lane & 3u);
                     if (mine && c < sh.coutStore)
-                        atomicAdd((float4*)(dW + ((size_t)c * 9 + (dy0 + dy) * 3 + dx) * sh.Cin + (ci & ~3u)),
+                        atomicAdd((float4*)(dW + ((size_t)c * 9 + tap) * sh.Cin + (ci & ~3u)),
                                   make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]));
                 }
             } else if (mine) {
-                float* o = dW + ((size_t)co * 9 + (dy0 + dy) * 3 + dx) * sh.Cin + ci;
+                float* o = dW + ((size_t)co * 9 + tap) * sh.Cin + ci;
 #pragma unroll
                 for (uint32_t i = 0; i < 16; ++i)
                     if (co + i < sh.coutStore) atomicAdd(o + (size_t)i * 9 * sh.Cin, v[i]);
@@ -969,8 +987,8 @@ int make_wgrad_maps(const WgradPlan& p, const void* g, const void* x, uint32_t B
                        {(cuuint64_t)C * 2, (cuuint64_t)W * C * 2, (cuuint64_t)H * W * C * 2}, {boxC, boxW, boxH, 1},
                        boxC * 2);
     };
-    const int rc = nhwc(mg, g, Cout, p.ca, kHTileW, kHTileH);
-    return rc ? rc : nhwc(mx, x, Cin, p.cb, kHaloW, wgrad_halo_rows(p.rows));
+    const int rc = nhwc(mg, g, Cout, std::min(64u, p.ca), kHTileW, kHTileH);
+    return rc ? rc : nhwc(mx, x, Cin, std::min(64u, p.cb), kHaloW, wgrad_halo_rows(p.rows));
 }
 
 int plan_wgrad(uint32_t B, uint32_t H, uint32_t W, uint32_t Cin, uint32_t Cout, uint32_t numSMs, WgradPlan* p) {
@@ -987,6 +1005,13 @@ int plan_wgrad(uint32_t B, uint32_t H, uint32_t W, uint32_t Cin, uint32_t Cout, 
     // as zeros and not stored (240 -> 240 over 4 x 64 x 64 in blocks of 16 x 16 171 us, here 34).
     p->ca = Cout <= 16 ? 16 : Cout <= 32 ? 32 : 64;
     p->cb = Cin <= 16 ? 16 : 32;
+    // The longest sum in TMEM, where every step is cut to f32, so that the error grows with the
+    // length: the tiles that two blocks an SM, of one tap, 128 output and 256 input channels
+    // each, would have (256 -> 256 channels over 16 x 16 x 16 pixels: 4.5e-7 from 64-bit sums
+    // with 4 tiles in one sum, 2.3e-7 with 2).
+    const uint32_t cells = 9 * ((Cin + 255) / 256) * ((Cout + 127) / 128);
+    const uint32_t parts = std::min((2 * numSMs + cells - 1) / cells, sh.tilesTotal);
+    const uint32_t longest = (sh.tilesTotal + parts - 1) / parts;
     // One wave of blocks, two an SM: one covers the other's start and atomics (one an SM:
     // 36 us for 96 -> 32 channels at full width, 32 with two), and a second wave would cost
     // a start (256 -> 256 channels at an eighth: 17 us, 24 with twice the blocks).  The
@@ -1009,17 +1034,37 @@ int plan_wgrad(uint32_t B, uint32_t H, uint32_t W, uint32_t Cin, uint32_t Cout, 
     sh.tilesPerCta = (sh.tilesTotal + splits - 1) / splits;
     splits = (sh.tilesTotal + sh.tilesPerCta - 1) / sh.tilesPerCta;
     p->grid = dim3(splits, ciBlocks, coBlocks);
-    // A sum in TMEM is cut to f32 at every step, so its error grows with its length: a sum
-    // takes at most the tiles that two blocks an SM, of one tap, 128 output and 256 input
-    // channels each, would have (256 -> 256 channels over 16 x 16 x 16 pixels: 4.5e-7 from
-    // 64-bit sums with all 4 tiles of a block in one sum, 2.3e-7 with 2).  A block of more
-    // reads several sums and adds them in registers: more blocks would each add all their
-    // weights to memory (a training pass of 16 x 128 x 128 858 us without the limit, 862 with
-    // it, 874 with blocks of that length).
-    const uint32_t cells = 9 * ((Cin + 255) / 256) * ((Cout + 127) / 128);
-    const uint32_t parts = std::min((2 * numSMs + cells - 1) / cells, sh.tilesTotal);
-    const uint32_t most = (sh.tilesTotal + parts - 1) / parts, sums = (sh.tilesPerCta + most - 1) / most;
+    // A block of more tiles than the longest sum reads several and adds them in registers: more
+    // blocks would each add all their weights to memory (a training pass of 16 x 128 x 128 858 us
+    // without the limit, 862 with it, 874 with blocks of that length).
+    const uint32_t sums = (sh.tilesPerCta + longest - 1) / longest;
     sh.sumTiles = (sh.tilesPerCta + sums - 1) / sums;
+    if (Cin <= 64 || Cout <= 64) return 0;
+
+    // kWide, one block an SM, with the splits (no longer sums) that take the least time in whole
+    // waves, where that beats the blocks above.  Measured on 148 SMs: a tile 1.17 us, a block's
+    // start and atomics as much as seven tiles, and 5 us; above 1.4 us a tile (of two blocks an SM) and
+    // 9 us.  512 -> 512 over 240 x 136 pixels 196 us above, 120 kWide, over 64 x 64 34 and 36;
+    // 256 -> 256 over 480 x 272 167 and 117, over 64 x 64 15 and 27.
+    const uint32_t ciWide = (Cin + 127) / 128, coWide = (Cout + 127) / 128 * 3;
+    uint32_t waves = ~0u, each = 0;
+    for (uint32_t n = parts; n <= std::min(sh.tilesTotal, 8 * parts); ++n) {
+        const uint32_t tiles = (sh.tilesTotal + n - 1) / n, time = (n * ciWide * coWide + numSMs - 1) / numSMs * (tiles + 7);
+        if (time < waves) {
+            waves = time;
+            each = tiles;
+        }
+    }
+    if (1.17f * waves + 5.0f < 1.4f * sh.tilesPerCta + 9.0f) {
+        p->ca = p->cb = 128;
+        p->rows = 1;
+        sh.tilesPerCta = sh.sumTiles = each;
+        p->grid = dim3((sh.tilesTotal + each - 1) / each, ciWide, coWide);
+        sh.tmemCols = 512;
+        sh.stages = 3;
+        const uint32_t wide = 2 * (round_up(wgrad_halo_rows(1) * kHaloW * 128, 1024) + kTileP * 128);
+        p->smem = smem_for(sh.stages * wide + (2 * sh.stages + 1) * 8 + 16 + 1024, sh.tmemCols);
+    }
     return 0;
 }
 
@@ -1088,6 +1133,7 @@ cudaError_t launch_wgrad(const WgradPlan& p, const CUtensorMap& mg, const CUtens
             e = cudaLaunchKernelEx(&lc, k_conv_wgrad<A, B, ROWS>, mg, mx, p.shape, dW, err); \
         return e != cudaSuccess ? e : cudaGetLastError();                                    \
     }
+    WRK_WGRAD_CASE(128, 128, 1)
     WRK_WGRAD_CASE(64, 32, 3)
     WRK_WGRAD_CASE(64, 16, 3)
     WRK_WGRAD_CASE(64, 32, 1)

@@ -11,7 +11,7 @@ using namespace wrk::conv;
 
 int main() {
     const uint32_t sizes[][3] = {{1, 8, 16}, {1, 64, 128}, {1, 1088, 1920}, {16, 128, 128}};
-    long plans = 0, byChunk = 0;
+    long plans = 0, byChunk = 0, wide = 0;
     for (uint32_t cin = 16; cin <= 2048; cin += 16)
         for (uint32_t n = 16; n <= 256; n += 16)
             for (int f32 = 0; f32 < 2; ++f32)
@@ -47,14 +47,19 @@ int main() {
                 const bool ok = rc == 0 && s.tilesTotal == tiles && p.grid.x * s.tilesPerCta >= tiles &&
                                 (p.grid.x - 1) * s.tilesPerCta < tiles && p.grid.y * p.cb >= cin &&
                                 p.grid.z * p.rows / 3 * p.ca >= cout && p.smem <= 227 * 1024 && s.stages >= 2 &&
-                                p.rows * ((p.ca + 31) / 32 * 32) <= s.tmemCols && s.sumTiles > 0 &&
+                                (p.ca == 128 ? 3 : p.rows) * ((p.ca + 31) / 32 * 32) <= s.tmemCols && s.sumTiles > 0 &&
                                 s.sumTiles <= (tiles + parts - 1) / parts &&
-                                // a row of taps a block where whole blocks would leave SMs idle
-                                (p.ca == 64 && ((cin + 31) / 32) * ((cout + 63) / 64) * tiles >= 148 ? p.rows == 3 : p.rows == 1) &&
-                                // no more blocks of channels than an MMA's rows and columns call for
-                                p.grid.y == (cin + 31) / 32 && p.grid.z * p.rows / 3 == (cout <= 32 ? 1 : (cout + 63) / 64);
+                                (p.ca == 128 ? p.cb == 128 && p.rows == 1 && s.sumTiles == s.tilesPerCta && cin > 64 && cout > 64
+                                             // no more blocks of channels than an MMA's rows and columns call for
+                                             : p.grid.y == (cin + 31) / 32 &&
+                                                   p.grid.z * p.rows / 3 == (cout <= 32 ? 1 : (cout + 63) / 64) &&
+                                                   // a row of taps a block where whole blocks would leave SMs idle
+                                                   (p.ca == 64 && ((cin + 31) / 32) * ((cout + 63) / 64) * tiles >= 148
+                                                        ? p.rows == 3
+                                                        : p.rows == 1));
                 ++plans;
+                wide += p.ca == 128;
                 if (!ok) std::printf("%u %u 2 %u %u %u %d\n", cin, cout, z[1], z[2], z[0], rc);
             }
-    std::printf("plans %ld by chunk %ld\n", plans, byChunk);
+    std::printf("plans %ld by chunk %ld wide %ld\n", plans, byChunk, wide);
 }

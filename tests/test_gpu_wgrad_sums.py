@@ -21,6 +21,9 @@ pytestmark = pytest.mark.gpu
     (1, 256, 256, 256, 16),
     (4, 64, 128, 16, 64),     # 16 input channels, all taps a block
     (1, 24, 48, 16, 64),      # and a row of taps a block
+    (1, 128, 128, 512, 512),  # blocks of 128 x 128 channels
+    (1, 136, 480, 224, 368),  # their last channels past the end, and an overhanging tile row
+    (1, 200, 320, 128, 128),
 ])
 def test_several_sums(gpu, b, h, w, cin, cout):
     rng = np.random.default_rng(cin * 5 + cout + h)
