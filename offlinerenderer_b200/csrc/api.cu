@@ -818,12 +818,24 @@ static void fill_stats(wrk_renderer* r, uint32_t iters, const float* stageMs, co
     }
 }
 
-// Resolves the sums, copies the images out when `host` buffers are given, and waits.
+// Resolves the sums, copies the images out when `host` buffers are given, and waits.  A
+// render that failed leaves the caller's images as they were: with `unchecked`, the counters
+// are still on their way to the host, so the resolve looks at the error on the device and
+// the host looks before it enqueues a copy (while the resolve runs).
 static int finish_render(wrk_renderer* r, const Frame& f, const wrk_render_params* p, float* d_rgb, float* d_alb,
-                         float* d_nrm, float* const* host) {
+                         float* d_nrm, float* const* host, bool unchecked) {
     cudaStream_t st = r->eng.stream;
-    launch_resolve(f, p->flags & WRK_FLAG_RAW_GUIDES, d_rgb, d_alb, d_nrm, st);
+    if (unchecked) CK(cudaEventRecord(r->ev1, st));
+    launch_resolve(f, p->flags & WRK_FLAG_RAW_GUIDES, d_rgb, d_alb, d_nrm, st, unchecked ? f.err : nullptr);
     CK(cudaGetLastError());
+    if (unchecked) {
+        CK(cudaEventSynchronize(r->ev1));
+        const uint32_t e = r->eng.hCtr->error;
+        if (e) {
+            CK(cudaStreamSynchronize(st));
+            return fail(WRK_ERR_DEVICE, "device error flags 0x%x during render", e);
+        }
+    }
     CK(cudaEventRecord(r->ev1, st));
     if (host) {
         float* const dev[3] = {d_rgb, d_alb, d_nrm};
@@ -873,8 +885,7 @@ static int render_impl(wrk_renderer* r, wrk_scene* s, const wrk_camera* cam, con
         launch_render_small(s->view, f, E.q.ctr, work, E.numSMs, st);
         CK(cudaEventRecord(r->evLoop1, st));
         CK(cudaMemcpyAsync(E.hCtr, E.q.ctr, sizeof(Counters), cudaMemcpyDeviceToHost, st));
-        if ((rc = finish_render(r, f, p, d_rgb, d_alb, d_nrm, host))) return rc;
-        if (E.hCtr->error) return fail(WRK_ERR_DEVICE, "device error flags 0x%x during render", E.hCtr->error);
+        if ((rc = finish_render(r, f, p, d_rgb, d_alb, d_nrm, host, true))) return rc;
         // as the wavefront loop counts: whole chunks of iterations, from the first path's
         // first to the last one's last
         iters = (E.hCtr->iteration + E.cfg.chunk - 1) / E.cfg.chunk * E.cfg.chunk;
@@ -924,7 +935,7 @@ static int render_impl(wrk_renderer* r, wrk_scene* s, const wrk_camera* cam, con
         if (iters > maxIters) return fail(WRK_ERR_DEVICE, "render did not converge after %u iterations", iters);
     }
     CK(cudaEventRecord(r->evLoop1, st));
-    if ((rc = finish_render(r, f, p, d_rgb, d_alb, d_nrm, host))) return rc;
+    if ((rc = finish_render(r, f, p, d_rgb, d_alb, d_nrm, host, false))) return rc;
     fill_stats(r, iters, stageMs, stageN, stats);
     return WRK_OK;
 }

@@ -840,11 +840,12 @@ void launch_render_small(const DevScene& s, const Frame& f, Counters* c, unsigne
     k_render_small<<<(int)(blocks < most ? blocks : most), kTraceBlock, 0, st>>>(s, f, c, work, lanes);
 }
 
-// rgb = sum * (1/spp) as renderer.cpp:308-313; guides averaged unless raw.
-__global__ void k_resolve(Frame f, uint32_t raw, float* rgb, float* albedo, float* normal) {
+// rgb = sum * (1/spp) as renderer.cpp:308-313; guides averaged unless raw.  Nothing is
+// written when *error (may be null) is set.
+__global__ void k_resolve(Frame f, uint32_t raw, float* rgb, float* albedo, float* normal, const uint32_t* error) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     uint32_t n = f.width * f.height;
-    if (i >= n) return;
+    if (i >= n || (error && *error)) return;
     float inv = 1.0f / (float)f.spp;
     float4 a = f.accum[i];
     rgb[3 * i] = a.x * inv;
@@ -865,9 +866,10 @@ __global__ void k_resolve(Frame f, uint32_t raw, float* rgb, float* albedo, floa
     }
 }
 
-void launch_resolve(const Frame& f, uint32_t raw, float* rgb, float* albedo, float* normal, cudaStream_t st) {
+void launch_resolve(const Frame& f, uint32_t raw, float* rgb, float* albedo, float* normal, cudaStream_t st,
+                    const uint32_t* error) {
     uint32_t n = f.width * f.height;
-    k_resolve<<<(n + 255) / 256, 256, 0, st>>>(f, raw, rgb, albedo, normal);
+    k_resolve<<<(n + 255) / 256, 256, 0, st>>>(f, raw, rgb, albedo, normal, error);
 }
 
 }  // namespace wrk

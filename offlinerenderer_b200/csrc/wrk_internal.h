@@ -248,7 +248,8 @@ constexpr int kSmallBlocksPerSM = 4;
 // longest path would take.
 void launch_render_small(const DevScene& s, const Frame& f, Counters* c, unsigned long long work, int numSMs,
                          cudaStream_t st);
-void launch_resolve(const Frame& f, uint32_t rawGuides, float* rgb, float* albedo, float* normal, cudaStream_t st);
+void launch_resolve(const Frame& f, uint32_t rawGuides, float* rgb, float* albedo, float* normal, cudaStream_t st,
+                    const uint32_t* error = nullptr);
 // End of one chunk of the device-driven loop: keeps the enclosing conditional
 // WHILE graph node running while a request in the admission order has work left.
 void launch_loop_cond(cudaGraphConditionalHandle h, const Queues& q, cudaStream_t st);
