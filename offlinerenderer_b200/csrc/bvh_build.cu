@@ -1049,7 +1049,8 @@ int build_bvh8(const float* d_vtx, const uint32_t* d_idx, const uint32_t* d_triM
     WRK_BCHECK(scratch_alloc(&items, pool, st, sizeof(CItem) * numBinary));
     WRK_BCHECK(scratch_alloc(&items2, pool, st, sizeof(CItem) * numBinary));
     WRK_BCHECK(scratch_alloc(&cctr, pool, st, sizeof(CollapseCtr)));
-    WRK_BCHECK(cudaMalloc(&onodes, sizeof(uint4) * 5 * (size_t)numBinary));
+    // (a wide node is the root or stands for an inner node of the binary tree, which are half of it)
+    WRK_BCHECK(cudaMalloc(&onodes, sizeof(uint4) * 5 * ((size_t)numBinary / 2 + 1)));
     WRK_BCHECK(cudaMalloc(&otris, sizeof(float4) * 3 * (size_t)n));
     {
         CItem r{0, 0};
