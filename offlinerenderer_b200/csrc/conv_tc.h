@@ -21,14 +21,14 @@ struct FwdShape {
 // (+ bias[co]) -> (ReLU) -> (x 0 where mask <= 0) -> store.  nOut > 0: by TMA through the
 // launch's output maps (bf16 or f32; four maps = the 2x nearest upsample), and the 2x2
 // average of the stored bf16 values into `pool` when it is set.  nOut = 0: the cropped
-// output image when headDst is set, else element stores to
-// out[pixel*outStride + outOffset + co] for co < coutValid.
+// output image when headDst is set, else plain stores to out[pixel*outStride + co] for
+// co < coutValid.
 struct Epilogue {
     const float* bias;  // bias[co] added for co < nBias (f32, at most 256 channels)
     uint32_t nBias;
     uint32_t nOut;
     void* out;
-    uint32_t outStride, outOffset, coutValid;
+    uint32_t outStride, coutValid;
     uint32_t relu, outF32;
     const __nv_bfloat16* mask;
     uint32_t maskStride, maskOffset;
@@ -73,11 +73,11 @@ int make_wgrad_maps(const WgradPlan& p, const void* g, const void* x, uint32_t B
 int plan_fwd(uint32_t B, uint32_t H, uint32_t W, uint32_t Cin, uint32_t N, bool outF32, uint32_t numSMs, FwdPlan* p);
 int plan_wgrad(uint32_t B, uint32_t H, uint32_t W, uint32_t Cin, uint32_t Cout, uint32_t numSMs, WgradPlan* p);
 // Tensor maps of a forward plan: the input, the weights [N * nSplit][9 * Cin] bf16, and
-// the output (channel `offset` on of a buffer `stride` channels wide; up = the 2x nearest
-// upsample of the output, whose buffer is 2W x 2H).
+// the output (its first C channels, from channel `offset` on of a buffer `stride` channels
+// wide; up = the 2x nearest upsample of the output, whose buffer is 2W x 2H).
 int make_input_map(const FwdPlan& p, const void* x, CUtensorMap* mx);
 int make_weight_map(const FwdPlan& p, const void* w, CUtensorMap* mw);
-int make_out_maps(const FwdPlan& p, void* out, uint32_t stride, uint32_t offset, bool f32, bool up, OutMaps* mo);
+int make_out_maps(const FwdPlan& p, void* out, uint32_t C, uint32_t stride, uint32_t offset, bool f32, bool up, OutMaps* mo);
 // overlap: the launch may begin before the stream's previous kernel has ended; the weights
 // and the bias must then be older than that kernel.
 cudaError_t launch_fwd(const FwdPlan& p, const CUtensorMap& mx, const CUtensorMap& mw, const OutMaps& mo,

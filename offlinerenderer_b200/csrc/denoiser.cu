@@ -430,7 +430,7 @@ int set_shape(wrk_denoiser* d, uint32_t B, uint32_t H, uint32_t W, bool train) {
                 return dfail(WRK_ERR_INVALID, "no forward plan for layer %d", i);
             if (conv::make_input_map(d->fplan[i], io.in, &d->fin[i]) ||
                 conv::make_weight_map(d->fplan[i], d->wf[i].p, &d->fw[i]) ||
-                conv::make_out_maps(d->fplan[i], io.out, io.outStride, io.outOffset, head, io.up, &d->fout[i]))
+                conv::make_out_maps(d->fplan[i], io.out, pad16(L.cout), io.outStride, io.outOffset, head, io.up, &d->fout[i]))
                 return dfail(WRK_ERR_CUDA, "tensor map encoding failed (layer %d)", i);
         }
         d->shapeReady = true;
@@ -459,7 +459,7 @@ int set_shape(wrk_denoiser* d, uint32_t B, uint32_t H, uint32_t W, bool train) {
                 return dfail(WRK_ERR_INVALID, "no data-gradient plan for layer %d", i);
             if (conv::make_input_map(d->dplan[i], d->g[i].p, &d->din[i]) ||
                 conv::make_weight_map(d->dplan[i], d->wd[i].p, &d->dwmap[i]) ||
-                conv::make_out_maps(d->dplan[i], dst, L.cin, 0, f32, false, &d->dout[i]))
+                conv::make_out_maps(d->dplan[i], dst, L.cin, L.cin, 0, f32, false, &d->dout[i]))
                 return dfail(WRK_ERR_CUDA, "tensor map encoding failed (layer %d dgrad)", i);
         }
     }
@@ -662,8 +662,8 @@ int wrk_conv3x3_forward(const void* x, uint32_t B, uint32_t H, uint32_t W, uint3
     ep.coutValid = Cout;
     ep.relu = flags & 1u;
     ep.outF32 = f32;
-    // whole 16-byte rows leave by TMA; a padded Cout or an unaligned output by element stores
-    if (N == Cout && conv::make_out_maps(plan, out, Cout, 0, f32, false, &mo) == 0) ep.nOut = 1;
+    // rows of whole 16-byte units leave by TMA, which drops the padding channels
+    if (conv::make_out_maps(plan, out, Cout, Cout, 0, f32, false, &mo) == 0) ep.nOut = 1;
     DCK(conv::launch_fwd(plan, mx, mw, mo, ep, false, err.as<uint32_t>(), 0));
     uint32_t e = 0;
     DCK(cudaMemcpy(&e, err.p, 4, cudaMemcpyDeviceToHost));
