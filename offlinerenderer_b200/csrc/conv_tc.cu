@@ -933,13 +933,15 @@ int plan_fwd(uint32_t B, uint32_t H, uint32_t W, uint32_t Cin, uint32_t N, bool 
         while (sh.stagesA > G && need(sh.stagesA, 6) > limit) --sh.stagesA;
         sh.stagesB = 16;
         while (sh.stagesB > 2 && need(sh.stagesA, sh.stagesB) > limit) --sh.stagesB;
-        // Where the halos leave room for fewer than sixteen MMAs' weights (more than 384
-        // channels, or many 16- and 32-channel chunks), the item runs chunk by chunk with the
-        // room for weights: the MMAs waited for their slices otherwise (528 -> 64 channels at
-        // 960 x 544 1224 us with five slices, 846 by chunk; 288 -> 32 356, 195), and inputs
-        // whose chunks do not fit at all are held no other way (512 -> 128 at 1920 x 1088 1690 us).
+        // Chunk by chunk where the halos leave room for fewer than sixteen MMAs' weights (more
+        // than 384 channels): the MMAs waited for their slices otherwise (16 x 128 x 128
+        // 448 -> 192 260 us by chunk; with one slice beside seven chunks no plan at all), and
+        // inputs whose chunks do not fit are held no other way (512 -> 128 at 1920 x 1088 1690
+        // us).  And with 16- and 32-channel chunks, one or two MMAs a slice: the straight loop
+        // over nine taps steps twice as fast as the one over chunks (144 -> 32 at 960 x 544 361
+        // us tap by tap, 190 by chunk; 96 -> 96 150, 131).
         const uint32_t mmas = p->chunk / 16;
-        p->byChunk = need(sh.stagesA, sh.stagesB) > limit || sh.stagesB * mmas < 16;
+        p->byChunk = p->chunk < 64 || need(sh.stagesA, sh.stagesB) > limit || sh.stagesB * mmas < 16;
         if (p->byChunk) {
             sh.stagesA = std::min(G, 4u);
             while (sh.stagesA > 2 && need(sh.stagesA, 16 / mmas) > limit) --sh.stagesA;

@@ -28,7 +28,8 @@ int main() {
                         // (split further only where an image has few tiles)
                         (s.nSplit <= 4 || z[1] < 128) &&
                         (p.byChunk ? s.stagesA >= 2 || s.stagesA == chunks : s.stagesA >= chunks) &&
-                        (p.resident ? !p.byChunk : s.stagesB >= 2);
+                        // (a slice of fewer than four MMAs is worth its wait only in the loop by chunk)
+                        (p.resident ? !p.byChunk : s.stagesB >= 2 && (p.chunk == 64 || p.byChunk));
                     ++plans;
                     byChunk += p.byChunk;
                     if (!ok) std::printf("%u %u %d %u %u %u %d\n", cin, n, f32, z[1], z[2], z[0], rc);
