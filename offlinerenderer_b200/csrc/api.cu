@@ -8,6 +8,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -127,7 +128,8 @@ struct wrk_scene {
     // one device allocation holds everything but the tree (a dozen of them, 0.1-0.3 ms each
     // to make and to free, were a quarter of a 676k-triangle scene's life)
     DevBuf arena;
-    uint32_t* dErr = nullptr;
+    uint32_t* dErr = nullptr;  // a query's error bits, and the word its kernels decide by
+    std::mutex queryLock;      // both are one query's at a time
     uint4* nodes = nullptr;
     float4* tris = nullptr;
     std::vector<uint32_t> emissive;
@@ -613,7 +615,7 @@ int wrk_scene_finalize(wrk_scene* s) {
                  oTexels = plan.place<uint8_t>(texelBytes), oTi = plan.place<TexInfo>(ti.size()),
                  oEmissive = plan.place<uint32_t>(s->emissive.size()), oCdf = plan.place<float>(s->cdf.size()),
                  oLights = plan.place<float4>(lights.size()), oEnv = plan.place<float>(s->envMap.size()),
-                 oErr = plan.place<uint32_t>(1), oPairs = plan.place<float4>(5 * (size_t)nt);
+                 oErr = plan.place<uint32_t>(2), oPairs = plan.place<float4>(5 * (size_t)nt);
     if ((rc = s->arena.alloc(plan.bytes))) return rc;
     uint8_t* const base = s->arena.as<uint8_t>();
     CK(copy_in(s->arena, oVtx, s->vtx));
@@ -975,8 +977,9 @@ int wrk_trace_closest(wrk_scene* s, const float* rays, uint32_t n, float* t, uin
     int rc = check_scene(s);
     if (rc) return rc;
     if (n && (!rays || !t || !prim)) return fail(WRK_ERR_INVALID, "null buffer");
-    CK(cudaMemset(s->dErr, 0, sizeof(uint32_t)));
-    launch_closest_query(s->view, rays, n, t, prim, s->dErr, 0);
+    if (!n) return WRK_OK;
+    std::lock_guard<std::mutex> lock(s->queryLock);
+    launch_closest_query(s->view, rays, n, t, prim, s->dErr, s->dErr + 1, 0);
     CK(cudaGetLastError());
     uint32_t e = 0;
     CK(cudaMemcpy(&e, s->dErr, sizeof(uint32_t), cudaMemcpyDeviceToHost));
@@ -987,8 +990,9 @@ int wrk_trace_occluded(wrk_scene* s, const float* rays, uint32_t n, uint32_t* oc
     int rc = check_scene(s);
     if (rc) return rc;
     if (n && (!rays || !occ)) return fail(WRK_ERR_INVALID, "null buffer");
-    CK(cudaMemset(s->dErr, 0, sizeof(uint32_t)));
-    launch_occluded_query(s->view, rays, n, occ, s->dErr, 0);
+    if (!n) return WRK_OK;
+    std::lock_guard<std::mutex> lock(s->queryLock);
+    launch_occluded_query(s->view, rays, n, occ, s->dErr, s->dErr + 1, 0);
     CK(cudaGetLastError());
     uint32_t e = 0;
     CK(cudaMemcpy(&e, s->dErr, sizeof(uint32_t), cudaMemcpyDeviceToHost));

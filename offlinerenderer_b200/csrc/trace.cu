@@ -33,10 +33,65 @@ __device__ __forceinline__ Ray load_ray8(const float* p) {
 // refilling idle lanes from its chunks (below kRefillQuery busy lanes), so a warp does not
 // wait for its slowest ray (one thread per ray ran at 8 of 32 lanes per instruction:
 // 1M closest + occlusion queries of a 676k-triangle scene 1022 us, 803 with the refill).
-// The chunks are assigned statically: no state is shared between calls.
+// The chunks are assigned statically.
+//
+// That suits rays that part ways.  Rays of neighbouring pixels end together, and a warp
+// that mixes chunks, or waits behind others in its share of a bright column of the image,
+// only loses by it: 2048 x 2048 camera rays of a 676k-triangle scene 885 us with a thread
+// per ray scheduled by the hardware, 1248 here (scattered rays: 2178 and 1287).  So a batch of
+// several chunks a warp is sampled first, and a coherent one is left to k_query_each, which
+// follows.
+constexpr uint32_t kQuerySamples = 8;
+
+// Programmatic dependent launch (as the convolutions').
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// Eight runs of 32 rays over the batch: are at least six of them bundles, whose origins lie
+// within 2 % of the scene's extent (the root's quantization frame) and whose directions
+// within an eighth of the first ray's?  (A kernel of its own: in k_query it cost the
+// traversal spills, 7 % of scattered batches.)  Clears the query's error word, too.
+__global__ void __launch_bounds__(kQuerySamples * 32)
+    k_query_sample(const uint4* __restrict__ nodes, const float* __restrict__ rays, uint32_t n, uint32_t* err,
+                   uint32_t* sampled) {
+    grid_launch_dependents();
+    if (threadIdx.x == 0) *err = 0;
+    if (!sampled) return;
+    const uint32_t lane = threadIdx.x & 31u, sample = threadIdx.x >> 5, e = __ldg(nodes).w;
+    const float extent = 256.0f * __uint_as_float(max(max(e & 0xffu, (e >> 8) & 0xffu), (e >> 16) & 0xffu) << 23);
+    const uint64_t at = (uint64_t)n * (2 * sample + 1) / (2 * kQuerySamples) & ~31ull;  // (n >= 512)
+    const Ray r = load_ray8(rays + 8 * (at + lane));
+    auto away = [](float v, float& of) {
+        const float first = __shfl_sync(0xffffffffu, v, 0);
+        of += fabsf(first);
+        return fabsf(v - first);
+    };
+    float d0 = 0.0f, o0 = 0.0f;
+    const float dd = away(r.dx, d0) + away(r.dy, d0) + away(r.dz, d0);
+    const float od = away(r.ox, o0) + away(r.oy, o0) + away(r.oz, o0);
+    const bool bundle = __all_sync(0xffffffffu, dd <= 0.125f * d0 && od <= 0.02f * extent);
+    const uint32_t bundles = __syncthreads_count(lane == 0 && bundle);
+    if (threadIdx.x == 0) *sampled = bundles >= kQuerySamples * 3 / 4 ? 1u : 0u;
+}
+
+template <bool kAnyHit>
+__device__ __forceinline__ void write_answer(const DevScene& s, const Trav& t, uint64_t idx, float* tOut, uint32_t* pOut) {
+    const bool hit = t.lBest != kNoHit;
+    if (kAnyHit) {
+        pOut[idx] = hit ? 1u : 0u;
+    } else {
+        tOut[idx] = hit ? t.tBest : __int_as_float(0x7f800000);
+        pOut[idx] = record_prim(s.tris, t.lBest);
+    }
+}
+
 template <bool kAnyHit>
 __global__ void __launch_bounds__(kTraceBlock, kBlocksQuery)
-    k_query(DevScene s, const float* __restrict__ rays, uint32_t n, float* tOut, uint32_t* pOut, uint32_t* err) {
+    k_query(DevScene s, const float* __restrict__ rays, uint32_t n, float* tOut, uint32_t* pOut, uint32_t* err,
+            const uint32_t* sampled) {
+    grid_wait();
+    grid_launch_dependents();
+    if (sampled && *sampled) return;
     __shared__ uint2 sstack[kStackSmem * kTraceBlock];
     __shared__ float4 sdir[kTraceBlock];  // the lanes' ray directions | tmin (read by triangle tests only)
     uint2 lstack[kStackLocal];
@@ -71,34 +126,68 @@ __global__ void __launch_bounds__(kTraceBlock, kBlocksQuery)
             if (active && !fin) fin = trav_step<kAnyHit, false>(geo, t, sdir, sstack, lstack, err);
         } while (__popc(__ballot_sync(0xffffffffu, active && !fin)) >= refillAt);
         if (active && fin) {
-            const bool hit = t.lBest != kNoHit;
-            if (kAnyHit) {
-                pOut[idx] = hit ? 1u : 0u;
-            } else {
-                tOut[idx] = hit ? t.tBest : __int_as_float(0x7f800000);
-                pOut[idx] = record_prim(s.tris, t.lBest);
-            }
+            write_answer<kAnyHit>(s, t, idx, tOut, pOut);
             active = false;
         }
     }
 }
 
-static int query_grid(uint32_t n) {
+// A thread per ray, for coherent batches.
+template <bool kAnyHit>
+__global__ void __launch_bounds__(kTraceBlock)
+    k_query_each(DevScene s, const float* __restrict__ rays, uint32_t n, float* tOut, uint32_t* pOut, uint32_t* err,
+                 const uint32_t* sampled) {
+    // launched while k_query drains, which hides the blocks that have nothing to do; one of
+    // them ends only after it, and so does this launch
+    if (blockIdx.x == 0) grid_wait();
+    if (!*sampled) return;
+    __shared__ uint2 sstack[kStackSmem * kTraceBlock];
+    __shared__ float4 sdir[kTraceBlock];
+    uint2 lstack[kStackLocal];
+    const uint64_t idx = (uint64_t)blockIdx.x * kTraceBlock + threadIdx.x;
+    if (idx >= n) return;
+    const TraceGeom geo{s.nodes, s.tris, s.pairs, s.numNodes, s.numTris};
+    Trav t;
+    trav_init(t, sdir, load_ray8(rays + 8 * idx));
+    while (!trav_step<kAnyHit, false>(geo, t, sdir, sstack, lstack, err)) {
+    }
+    write_answer<kAnyHit>(s, t, idx, tOut, pOut);
+}
+
+template <bool kAnyHit>
+static void launch_query(const DevScene& s, const float* rays, uint32_t n, float* t, uint32_t* out, uint32_t* err,
+                         uint32_t* sampled, cudaStream_t st) {
+    if (!n) return;
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    return (int)std::min<uint64_t>(((uint64_t)n + kTraceBlock - 1) / kTraceBlock, (uint64_t)sms * kBlocksQuery);
+    const uint32_t blocks = (n - 1) / kTraceBlock + 1, resident = (uint32_t)sms * kBlocksQuery;
+    // (one chunk a warp needs no choice, which takes 2 us; with two, 262,144 camera rays of a
+    // 676k-triangle scene in 8 x 4 tiles take 183 us in k_query and 152 chosen, of 36 triangles 37 and 37)
+    const bool choose = blocks > resident;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t lc{};
+    lc.gridDim = dim3(std::min(blocks, resident));
+    lc.blockDim = dim3(kTraceBlock);
+    lc.stream = st;
+    lc.attrs = &at;
+    lc.numAttrs = 1;
+    const uint32_t* flag = choose ? sampled : nullptr;
+    k_query_sample<<<1, kQuerySamples * 32, 0, st>>>(s.nodes, rays, n, err, choose ? sampled : nullptr);
+    cudaLaunchKernelEx(&lc, k_query<kAnyHit>, s, rays, n, t, out, err, flag);
+    lc.gridDim = dim3(blocks);
+    if (choose) cudaLaunchKernelEx(&lc, k_query_each<kAnyHit>, s, rays, n, t, out, err, flag);
 }
 
 void launch_closest_query(const DevScene& s, const float* rays, uint32_t n, float* t, uint32_t* prim, uint32_t* err,
-                          cudaStream_t st) {
-    if (!n) return;
-    k_query<false><<<query_grid(n), kTraceBlock, 0, st>>>(s, rays, n, t, prim, err);
+                          uint32_t* sampled, cudaStream_t st) {
+    launch_query<false>(s, rays, n, t, prim, err, sampled, st);
 }
 void launch_occluded_query(const DevScene& s, const float* rays, uint32_t n, uint32_t* occ, uint32_t* err,
-                           cudaStream_t st) {
-    if (!n) return;
-    k_query<true><<<query_grid(n), kTraceBlock, 0, st>>>(s, rays, n, nullptr, occ, err);
+                           uint32_t* sampled, cudaStream_t st) {
+    launch_query<true>(s, rays, n, nullptr, occ, err, sampled, st);
 }
 
 // ---------------------------------------------------------------------------

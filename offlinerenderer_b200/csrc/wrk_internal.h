@@ -276,10 +276,10 @@ int report_error(int code, const char* msg);
 void launch_leaf_records(float4* tris, uint32_t numTris, const wrk_material* mats, uint32_t numMats, float4* pairs,
                          cudaStream_t st);
 
-// standalone ray queries (trace.cu)
-void launch_closest_query(const DevScene& s, const float* rays, uint32_t n, float* t, uint32_t* prim,
-                          uint32_t* err, cudaStream_t st);
+// standalone ray queries (trace.cu); `sampled`: a device word of the query's own
+void launch_closest_query(const DevScene& s, const float* rays, uint32_t n, float* t, uint32_t* prim, uint32_t* err,
+                          uint32_t* sampled, cudaStream_t st);
 void launch_occluded_query(const DevScene& s, const float* rays, uint32_t n, uint32_t* occ, uint32_t* err,
-                           cudaStream_t st);
+                           uint32_t* sampled, cudaStream_t st);
 
 }  // namespace wrk
