@@ -72,7 +72,7 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 // memory and TMA stores (75 us); the layers whose weights do not fit waited on L2 ->
 // shared memory traffic, nine copies of the input among it (192 -> 64 202 -> 164 us,
 // 384 -> 128 125 -> 96 us) and now wait on their weight slices' MMA steps (315 cycles for
-// 200 of MMAs at 64 channels).  The whole frame: 1940 -> 1125 us.
+// 200 of MMAs at 64 channels).  The whole frame: 1940 -> 1100 us.
 constexpr uint32_t kHaloW = 10, kHaloH = 18, kHaloPix = kHaloW * kHaloH, kHTileW = 8, kHTileH = 16;
 // Epilogue warps: four per accumulator buffer for resident layers (one group of four
 // alternating between the buffers could not keep up with 9-36 MMAs a tile), four in all
@@ -129,7 +129,7 @@ __device__ __forceinline__ void finish16(const Epilogue& ep, const float* bias, 
         for (uint32_t j = 0; j < 16; ++j) v[j] = fmaxf(v[j], 0.0f);
     }
     if (ep.mask && inside) {
-        const __nv_bfloat16* m = ep.mask + pix * ep.maskStride + ep.maskOffset + c0;
+        const __nv_bfloat16* m = ep.mask + pix * ep.maskStride + c0;
         const uint4 a = *(const uint4*)m, b = *(const uint4*)(m + 8);
         const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
 #pragma unroll

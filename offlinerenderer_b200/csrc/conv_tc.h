@@ -31,7 +31,7 @@ struct Epilogue {
     uint32_t outStride, coutValid;
     uint32_t relu, outF32;
     const __nv_bfloat16* mask;
-    uint32_t maskStride, maskOffset;
+    uint32_t maskStride;
     __nv_bfloat16* pool;  // [B][H/2][W/2][poolStride]
     uint32_t poolStride;
     const float* headRgb;  // [B][headH][headW][3]

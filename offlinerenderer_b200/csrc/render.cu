@@ -29,8 +29,8 @@
 namespace wrk {
 
 constexpr int kShadeBlock = 256;
-// Range of a camera ray and of every later extension ray (whose tmin is 0).
 constexpr uint32_t kSmallCounters = 8;  // rays, shadow rays traced / answered, hits of four buckets, last iteration
+// Range of a camera ray and of every later extension ray (whose tmin is 0).
 constexpr float kCameraTmin = 0.0001f, kRayTmax = 1e20f;
 
 __device__ __forceinline__ uint32_t append_pos(uint32_t* counter, bool pred, uint32_t cap, uint32_t* err) {
