@@ -69,11 +69,11 @@ UNET_FLOP_PER_PX = sum(2 * 9 * ci * co / 4 ** lv for ci, co, lv in UNET_LAYERS)
 # 512x512 16-spp render of the same scene that ncu profiles (the plain-launch,
 # stage-timed one), divided by its 14,406,486 extension rays; traffic per launch of
 # the full workload = this x rays per launch (traffic grows with the rays traced).
-TRACE_EXT_TRAFFIC_BYTES_PER_RAY = 149.2
+TRACE_EXT_TRAFFIC_BYTES_PER_RAY = 150.4
 # SM issue-slot utilisation of the traversal and shading kernels (the roofline that
-# bounds them: SIMT integer / FP32 work, not HBM), smsp__issue_active from ncu --set
-# full on the 16-spp capture of the same scene.  CUDA events cannot measure it live.
-STAGE_ISSUE_ACTIVE = {"trace_extension": 0.710, "trace_shadow": 0.630, "shade_lambert": 0.566}
+# bounds them: SIMT integer / FP32 work, not HBM), smsp__issue_active from ncu on the
+# 16-spp capture of the same scene (profiles/).  CUDA events cannot measure it live.
+STAGE_ISSUE_ACTIVE = {"trace_extension": 0.637, "trace_shadow": 0.544, "shade_lambert": 0.457}
 STAGE_BYTES = {"trace_extension": 48, "trace_shadow": 80, "shade_lambert": 160, "shade_dielectric": 160,
                "shade_ggx": 160, "shade_emissive": 160}
 
