@@ -91,7 +91,7 @@ __global__ void __launch_bounds__(kTraceBlock, kBlocksQuery)
             const uint32_t* sampled) {
     grid_wait();
     grid_launch_dependents();
-    if (sampled && *sampled) return;
+    if (sampled && __ldcg(sampled)) return;
     __shared__ uint2 sstack[kStackSmem * kTraceBlock];
     __shared__ float4 sdir[kTraceBlock];  // the lanes' ray directions | tmin (read by triangle tests only)
     uint2 lstack[kStackLocal];
@@ -140,7 +140,7 @@ __global__ void __launch_bounds__(kTraceBlock)
     // launched while k_query drains, which hides the blocks that have nothing to do; one of
     // them ends only after it, and so does this launch
     if (blockIdx.x == 0) grid_wait();
-    if (!*sampled) return;
+    if (!__ldcg(sampled)) return;  // (written before k_query began, which is all that is known here: read from L2)
     __shared__ uint2 sstack[kStackSmem * kTraceBlock];
     __shared__ float4 sdir[kTraceBlock];
     uint2 lstack[kStackLocal];
